@@ -59,8 +59,8 @@ typedef struct {
   int32_t blocks_per_sm;         /* persistent grid = SMs * blocks_per_sm (0 = default) */
   int32_t sort_keys;             /* wavefront queue sorting, bit mask: 1 shading queue by material,
                                     2 extension rays by direction octant, 4 shadow rays by light (0 = off) */
-  int32_t trace_budget;          /* wavefront: traversal steps between refills of idle lanes (0 = 32) */
-  int32_t traversal;             /* TS_TRAVERSAL_DEFAULT or TS_TRAVERSAL_SPECULATIVE (two-child nodes) */
+  int32_t trace_budget;          /* wavefront: accepted, without effect (idle lanes are refilled as they gather) */
+  int32_t traversal;             /* TS_TRAVERSAL_DEFAULT or TS_TRAVERSAL_SPECULATIVE; both run the same loop */
   int32_t occupancy;             /* megakernel register budget: 0 = 5 resident blocks of 128 per SM (96 registers),
                                     8 = 8 blocks (64 registers, spills; more latency hiding on large frames) */
   int32_t queue_capacity;        /* wavefront path slots (0 = one per pixel; at most 2^25).  With sort_keys == 0,
@@ -298,7 +298,7 @@ typedef struct {
                              CUDA graph with use_graph */
   int32_t queue_capacity; /* wavefront: path slots shared by all scenes (0 = min(paths per step, 2^24); at most
                              2^25; 160 B of device memory per slot) */
-  int32_t trace_budget;   /* wavefront: traversal steps between refills of idle lanes (0 = 16) */
+  int32_t trace_budget;   /* wavefront: accepted, without effect */
 } ts_batch_config;
 
 ts_status ts_batch_create(const ts_batch_config *cfg, ts_ctx *const *ctxs, int32_t num_scenes, ts_batch **out);

@@ -206,7 +206,7 @@ __device__ void grad_surface(const DevScene &s, const DevConfig &c, int pmat, co
 namespace {
 
 template <int W, int kPhase>
-__global__ void __launch_bounds__(128, kPhase ? 4 : 5) k_adjoint(DevScene s, DevConfig c, uint32_t pass0, int npass, int band0,
+__global__ void __launch_bounds__(128, kPhase ? 4 : 5) k_adjoint(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass0, int npass, int band0,
                                                  const double *__restrict__ adj, double *__restrict__ grad,
                                                  float *__restrict__ weight, int pm_shared, int pmat,
                                                  int *__restrict__ counter, uint32_t *__restrict__ err,
@@ -430,8 +430,6 @@ cudaError_t launch_adjoint(const DevScene &s, const DevConfig &c, uint32_t pass,
     launch_pair<8>(s, c, pass, npass, band, adj, grad, weight, psh, pmat, counter, err, grid, st, rec);
   else if (s.node_width == 4)
     launch_pair<4>(s, c, pass, npass, band, adj, grad, weight, psh, pmat, counter, err, grid, st, rec);
-  else if (c.speculative)
-    launch_pair<3>(s, c, pass, npass, band, adj, grad, weight, psh, pmat, counter, err, grid, st, rec);
   else launch_pair<2>(s, c, pass, npass, band, adj, grad, weight, psh, pmat, counter, err, grid, st, rec);
   return cudaGetLastError();
 }

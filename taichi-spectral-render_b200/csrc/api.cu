@@ -178,7 +178,6 @@ ts_status ts_create(const ts_config *cfg, ts_ctx **out) {
   d.fov = k.fov_scale;
   d.seed = k.seed;
   d.scene_id = k.scene_id;
-  d.speculative = k.traversal == TS_TRAVERSAL_SPECULATIVE ? 1 : 0;
   const size_t cells = (size_t)k.width * k.height * k.bands;
   for (int i = 0; i < 3; ++i) {
     e = cudaMalloc((void **)&c->d_film[i], cells * sizeof(double));
@@ -224,7 +223,6 @@ ts_status ts_set_launch_config(ts_ctx *c, const ts_config *k) {
     return fail(c, TS_ERR_INVALID_ARG, "ts_set_launch_config: queue_capacity above 2^25 path slots");
   c->cfg.queue_capacity = k->queue_capacity;
   c->cfg.loop_host = k->loop_host;
-  c->dc.speculative = k->traversal == TS_TRAVERSAL_SPECULATIVE ? 1 : 0;
   return TS_OK;
 }
 
@@ -302,23 +300,25 @@ ts_status ts_upload_scene(ts_ctx *c, const ts_scene_desc *sd) {
   // ---- triangles in slot order
   std::vector<float4> tri((size_t)3 * T), shade((size_t)3 * T);
   std::vector<int32_t> slot_mat(T);
-  for (int s = 0; s < T; ++s) {
-    const int o = bvh.perm[s];
-    const float *a = sd->v0 + 3 * (size_t)o, *b = sd->v1 + 3 * (size_t)o, *q = sd->v2 + 3 * (size_t)o;
-    int32_t oid = o, mid = sd->mat_id[o];
-    float fo, fm;
-    std::memcpy(&fo, &oid, 4);
-    std::memcpy(&fm, &mid, 4);
-    tri[3 * s + 0] = make_float4(a[0], a[1], a[2], fo);
-    tri[3 * s + 1] = make_float4(b[0] - a[0], b[1] - a[1], b[2] - a[2], fm);
-    tri[3 * s + 2] = make_float4(q[0] - a[0], q[1] - a[1], q[2] - a[2], 0.f);
-    const float *g = sd->normal + 3 * (size_t)o;
-    const float *n0 = sd->n0 + 3 * (size_t)o, *n1 = sd->n1 + 3 * (size_t)o, *n2 = sd->n2 + 3 * (size_t)o;
-    shade[3 * s + 0] = make_float4(n0[0], n0[1], n0[2], g[0]);
-    shade[3 * s + 1] = make_float4(n1[0], n1[1], n1[2], g[1]);
-    shade[3 * s + 2] = make_float4(n2[0], n2[1], n2[2], g[2]);
-    slot_mat[s] = mid;
-  }
+  ts::parallel_chunks(T, [&](int begin, int end) {
+    for (int s = begin; s < end; ++s) {
+      const int o = bvh.perm[s];
+      const float *a = sd->v0 + 3 * (size_t)o, *b = sd->v1 + 3 * (size_t)o, *q = sd->v2 + 3 * (size_t)o;
+      int32_t oid = o, mid = sd->mat_id[o];
+      float fo, fm;
+      std::memcpy(&fo, &oid, 4);
+      std::memcpy(&fm, &mid, 4);
+      tri[3 * (size_t)s + 0] = make_float4(a[0], a[1], a[2], fo);
+      tri[3 * (size_t)s + 1] = make_float4(b[0] - a[0], b[1] - a[1], b[2] - a[2], fm);
+      tri[3 * (size_t)s + 2] = make_float4(q[0] - a[0], q[1] - a[1], q[2] - a[2], 0.f);
+      const float *g = sd->normal + 3 * (size_t)o;
+      const float *n0 = sd->n0 + 3 * (size_t)o, *n1 = sd->n1 + 3 * (size_t)o, *n2 = sd->n2 + 3 * (size_t)o;
+      shade[3 * (size_t)s + 0] = make_float4(n0[0], n0[1], n0[2], g[0]);
+      shade[3 * (size_t)s + 1] = make_float4(n1[0], n1[1], n1[2], g[1]);
+      shade[3 * (size_t)s + 2] = make_float4(n2[0], n2[1], n2[2], g[2]);
+      slot_mat[s] = mid;
+    }
+  });
   // ---- materials, main.py:545-561
   std::vector<float4> mat((size_t)M * B * 2);
   for (int m = 0; m < M; ++m)
@@ -353,8 +353,11 @@ ts_status ts_upload_scene(ts_ctx *c, const ts_scene_desc *sd) {
     }
   // ---- lights per band over slots, main.py:590-627 (float32 sums, CDF left unclamped)
   std::vector<std::vector<int>> lights(B);
+  std::vector<char> emits(M, 0);  // in any band
+  for (int m = 0; m < M; ++m)
+    for (int b = 0; b < B; ++b) emits[m] |= sd->mat_i32[(size_t)m * 2 * B + 1 * B + b] != 0;
   for (int s = 0; s < T; ++s)
-    for (int b = 0; b < B; ++b)
+    for (int b = 0; emits[slot_mat[s]] && b < B; ++b)
       if (sd->mat_i32[(size_t)slot_mat[s] * 2 * B + 1 * B + b]) lights[b].push_back(s);
   int L = 1;
   for (int b = 0; b < B; ++b) L = std::max<int>(L, (int)lights[b].size());
@@ -431,7 +434,7 @@ ts_status ts_upload_scene(ts_ctx *c, const ts_scene_desc *sd) {
   c->d_cmf = d_cmf;
   c->perm = bvh.perm;
   c->info.num_tris = T;
-  c->info.num_nodes = ds.num_nodes;
+  c->info.num_nodes = bvh.width == 2 ? bvh.two_child_nodes : ds.num_nodes;
   c->info.num_ref_nodes = ds.num_ref_nodes;
   c->info.max_depth = bvh.max_depth;
   c->info.leaves = bvh.leaves;
@@ -547,7 +550,7 @@ static ts_status render_wave_loop(ts_ctx *c, uint32_t pass0, int npass, int band
   int per_sm = c->cfg.blocks_per_sm;
   if (per_sm <= 0) per_sm = std::max(1, 2048 / bs);
   TS_CUDA(c, ts::launch_wave_loop(c->ds, c->dc, pass0, band0, npass, film_of(c), c->wave, c->d_err,
-                                  c->num_sms * per_sm, bs, st, c->cfg.trace_budget, cap, &c->wave_loop,
+                                  c->num_sms * per_sm, bs, st, cap, &c->wave_loop,
                                   c->cfg.loop_host != 0, c->loop_limit),
           what);
   return TS_OK;
@@ -637,7 +640,7 @@ ts_status ts_render_pass(ts_ctx *c, uint32_t pass_idx, int32_t band, void *strea
     if (c->cfg.queue_capacity > 0 && c->cfg.sort_keys == 0)
       return render_wave_loop(c, pass_idx, 1, band, st, "render pass");
     TS_CUDA(c, ts::launch_wave_pass(c->ds, c->dc, pass_idx, band, film_of(c), c->wave, c->d_err, grid, bs,
-                                    c->cfg.sort_keys, st, c->cfg.trace_budget, c->cfg.queue_capacity),
+                                    c->cfg.sort_keys, st, c->cfg.queue_capacity),
             "render pass");
   }
   return TS_OK;
@@ -743,7 +746,7 @@ ts_status ts_render_tile_noalloc(ts_ctx *c, uint32_t pass_idx, int32_t band, int
   int per_sm = c->cfg.blocks_per_sm;
   if (per_sm <= 0) per_sm = std::max(1, 2048 / bs);
   TS_CUDA(c, ts::launch_wave_tile_noalloc(c->ds, c->dc, pass_idx, band, f, scratch, x0, y0, tile_w, tile_h, c->d_err,
-                                          c->num_sms * per_sm, bs, as_stream(stream), c->cfg.trace_budget),
+                                          c->num_sms * per_sm, bs, as_stream(stream)),
           "ts_render_tile_noalloc");
   return TS_OK;
 }
@@ -973,7 +976,10 @@ void batch_free(ts_batch *b) {
   cudaFree(b->d_err);
 }
 
-int batch_width(const ts_ctx *c) { return c->ds.node_width == 2 && c->dc.speculative ? 3 : c->ds.node_width; }
+// layout and traversal variant, which the scenes of a batch share
+int batch_width(const ts_ctx *c) {
+  return c->ds.node_width == 2 && c->cfg.traversal == TS_TRAVERSAL_SPECULATIVE ? 3 : c->ds.node_width;
+}
 }  // namespace
 
 extern "C" {
@@ -1117,7 +1123,7 @@ ts_status ts_batch_step(ts_batch *b, void *stream) {
     // one regenerating wavefront loop over every active scene's block; with
     // use_graph the whole step (prepare, init, while-loop, averages) is one graph
     TS_BCUDA(b, ts::launch_batch_loop_step(b->d_slots, b->n, b->d_hdr, b->d_active, b->d_err, b->wave, b->width,
-                                           b->num_sms * 8, ts::kMaxBlock, b->cfg.trace_budget, b->loop_cap,
+                                           b->num_sms * 8, ts::kMaxBlock, b->loop_cap,
                                            b->loop_limit, acc_blocks, as_stream(stream), &b->loop,
                                            b->cfg.use_graph != 0),
              "ts_batch_step");

@@ -53,7 +53,7 @@ cudaError_t launch_batch_finish(BatchSlot *slots, int n, int acc_blocks, cudaStr
 // limit bounds the loop's iterations (kErrIterationCap past it).
 struct BatchLoopGraph;
 cudaError_t launch_batch_loop_step(BatchSlot *slots, int n, BatchHeader *h, const int *active, uint32_t *err,
-                                   const WaveBuffers &w, int width, int grid, int block, int budget, int capacity,
+                                   const WaveBuffers &w, int width, int grid, int block, int capacity,
                                    int limit, int acc_blocks, cudaStream_t st, BatchLoopGraph **graph, bool use_graph);
 void free_batch_loop(BatchLoopGraph *g);
 cudaError_t batch_set_smem_limit(int n);

@@ -240,9 +240,8 @@ void expand_big_leaves(std::vector<BNode> &tree, const std::vector<Prim> &prims,
 
 // Wide layout: collapse the binary tree greedily (an inner child with the
 // largest surface area is replaced by its two children until a node has
-// `width` children) and store each node's child boxes as SoA float4 rows:
-//   width 4: lo.x hi.x lo.y hi.y lo.z hi.z refs pad         (8 float4, 128 B)
-//   width 8: each of the six rows and the refs as two float4 (16 float4, 256 B)
+// `width` children) and store a 32-byte record per child:
+//   (lo.x, hi.x, lo.y, hi.y), (lo.z, hi.z, link, -)       128 / 256 B per node
 // Empty child slots have NaN boxes, which no slab test accepts.  Returns false
 // (out untouched) if the traversal stack bound would be exceeded.
 // Quantized wide node (layout ids 5 and 9): the node's origin (the low corner
@@ -311,6 +310,7 @@ bool flatten_wide(const std::vector<BNode> &tree, int W, BvhOut &out, bool quant
     int n;
   };
   std::vector<WN> wn;
+  wn.reserve(tree.size() / 4 + 1);
   std::vector<int> wmap(tree.size(), -1);
   int max_stack = 0;
   // iterative DFS over binary inner nodes that start a wide node
@@ -327,7 +327,6 @@ bool flatten_wide(const std::vector<BNode> &tree, int W, BvhOut &out, bool quant
   } else {
     todo.push_back({0, 0});
   }
-  std::vector<std::pair<int, int>> order;  // (binary node, wide index) in creation order
   while (!todo.empty()) {
     const Item it = todo.back();
     todo.pop_back();
@@ -379,38 +378,34 @@ bool flatten_wide(const std::vector<BNode> &tree, int W, BvhOut &out, bool quant
   const int F = node_float4s(W);
   std::vector<float4> nodes((size_t)F * wn.size());
   const float qnan = std::nanf("");
-  for (size_t i = 0; i < wn.size(); ++i) {
-    float row[6][8];
-    int ref[8];
-    for (int k = 0; k < 8; ++k) {
-      for (int r = 0; r < 6; ++r) row[r][k] = qnan;
-      ref[k] = leaf_code(0, 1);
+  parallel_chunks((int)wn.size(), [&](int b, int e) {
+    for (int i = b; i < e; ++i) {
+      float4 *dst = nodes.data() + (size_t)F * i;
+      for (int k = 0; k < W; ++k) {
+        float4 &xy = dst[2 * k], &zr = dst[2 * k + 1];
+        int ref = leaf_code(0, 1);
+        if (k < wn[i].n) {
+          const BNode &c = tree[wn[i].ch[k]];
+          xy = make_float4(c.lo[0], c.hi[0], c.lo[1], c.hi[1]);
+          zr = make_float4(c.lo[2], c.hi[2], 0.f, 0.f);
+          ref = c.left >= 0 ? wmap[wn[i].ch[k]] : leaf_code(c.first, c.count);
+        } else {
+          xy = make_float4(qnan, qnan, qnan, qnan);
+          zr = make_float4(qnan, qnan, 0.f, 0.f);
+        }
+        std::memcpy(&zr.z, &ref, sizeof ref);
+      }
     }
-    for (int k = 0; k < wn[i].n; ++k) {
-      const BNode &c = tree[wn[i].ch[k]];
-      row[0][k] = c.lo[0]; row[1][k] = c.hi[0];
-      row[2][k] = c.lo[1]; row[3][k] = c.hi[1];
-      row[4][k] = c.lo[2]; row[5][k] = c.hi[2];
-      ref[k] = c.left >= 0 ? wmap[wn[i].ch[k]] : leaf_code(c.first, c.count);
-    }
-    float4 *dst = nodes.data() + (size_t)F * i;
-    const int per = W / 4;  // float4s per row
-    for (int r = 0; r < 6; ++r)
-      for (int q = 0; q < per; ++q) dst[r * per + q] = make_float4(row[r][4 * q], row[r][4 * q + 1], row[r][4 * q + 2], row[r][4 * q + 3]);
-    for (int q = 0; q < per; ++q) {
-      int4 l = make_int4(ref[4 * q], ref[4 * q + 1], ref[4 * q + 2], ref[4 * q + 3]);
-      std::memcpy(&dst[6 * per + q], &l, sizeof(int4));
-    }
-  }
+  });
   out.node2.swap(nodes);
   out.width = W;
   out.stack_need = max_stack;
   return true;
 }
 
-// Flatten a preorder BNode tree into the device layout (two-child, or wide
-// with `width` 4 or 8).  Returns false on a malformed tree.
-bool flatten_two_child(std::vector<BNode> tree, const std::vector<Prim> &prims, const std::vector<int32_t> &perm,
+// Flatten a preorder BNode tree into the device nodes of a layout (`width` 2,
+// 4 or 8).  Returns false on a malformed tree.
+bool flatten_tree(std::vector<BNode> &&tree, const std::vector<Prim> &prims, const std::vector<int32_t> &perm,
                        BvhOut &out, std::string &err, int width = 2, bool quantize = false) {
   expand_big_leaves(tree, prims, perm);
   const int N = (int)tree.size();
@@ -418,8 +413,7 @@ bool flatten_two_child(std::vector<BNode> tree, const std::vector<Prim> &prims, 
     out.node2.clear();
     return true;
   }
-  // number the inner nodes (depth-first, children in left/right order)
-  std::vector<int> map(N, -1), depth(N, 0);
+  std::vector<int> depth(N, 0);
   std::vector<int> stack = {0};
   int inner = 0, leaves = 0, maxd = 0;
   std::vector<char> seen(N, 0);
@@ -433,7 +427,7 @@ bool flatten_two_child(std::vector<BNode> tree, const std::vector<Prim> &prims, 
     seen[i] = 1;
     maxd = std::max(maxd, depth[i]);
     if (tree[i].left >= 0) {
-      map[i] = inner++;
+      ++inner;
       const int l = tree[i].left, r = tree[i].right;
       if (l < 0 || l >= N || r < 0 || r >= N) {
         err = "BVH: child index out of range";
@@ -450,53 +444,35 @@ bool flatten_two_child(std::vector<BNode> tree, const std::vector<Prim> &prims, 
     err = "BVH: tree depth " + std::to_string(maxd) + " exceeds the traversal stack";
     return false;
   }
-  const bool root_leaf = tree[0].left < 0;
-  const int nodes = root_leaf ? 1 : inner;
-  out.node2.assign((size_t)4 * nodes, make_float4(0.f, 0.f, 0.f, 0.f));
-  auto child_ref = [&](int c) { return tree[c].left >= 0 ? map[c] : leaf_code(tree[c].first, tree[c].count); };
-  auto put = [&](int slot, int c0, int c1, bool c1_empty) {
-    const BNode &A = tree[c0];
-    const float nanf_ = std::nanf("");
-    float b1[6];
-    if (c1_empty) {
-      for (float &x : b1) x = nanf_;
-    } else {
-      const BNode &Bn = tree[c1];
-      b1[0] = Bn.lo[0]; b1[1] = Bn.hi[0]; b1[2] = Bn.lo[1]; b1[3] = Bn.hi[1]; b1[4] = Bn.lo[2]; b1[5] = Bn.hi[2];
-    }
-    out.node2[4 * slot + 0] = make_float4(A.lo[0], A.hi[0], A.lo[1], A.hi[1]);
-    out.node2[4 * slot + 1] = make_float4(b1[0], b1[1], b1[2], b1[3]);
-    out.node2[4 * slot + 2] = make_float4(A.lo[2], A.hi[2], b1[4], b1[5]);
-    int4 link = make_int4(child_ref(c0), c1_empty ? child_ref(c0) : child_ref(c1), 0, 0);
-    std::memcpy(&out.node2[4 * slot + 3], &link, sizeof(int4));
-  };
-  if (root_leaf) {
-    put(0, 0, 0, true);
-  } else {
-    for (int i = 0; i < N; ++i)
-      if (tree[i].left >= 0) put(map[i], tree[i].left, tree[i].right, false);
-  }
+  out.two_child_nodes = tree[0].left < 0 ? 1 : inner;
   out.max_depth = maxd;
   out.leaves = leaves;
-  out.width = 2;
   out.stack_need = maxd;
-  // keeps the two-child layout if the wide one cannot be built
-  if (width == 4 || width == 8)
-    if (!flatten_wide(tree, width, out, quantize) && quantize) flatten_wide(tree, width, out, false);
+  if (width == 4 || width == 8) {
+    if (flatten_wide(tree, width, out, quantize)) return true;
+    if (quantize && flatten_wide(tree, width, out, false)) return true;
+  }
+  // the two-child layout (asked for, or because the wide one cannot be built):
+  // its device nodes are the same tree collapsed to four children, or none
+  // where the wide traversal stack could overflow
+  if (!flatten_wide(tree, 4, out)) out.node2.clear();
+  out.width = 2;
   return true;
 }
 
 std::vector<Prim> make_prims(int T, const float *v0, const float *v1, const float *v2) {
   std::vector<Prim> prims(T);
-  for (int t = 0; t < T; ++t) {
-    Prim &q = prims[t];
-    for (int a = 0; a < 3; ++a) {
-      const float x = v0[3 * t + a], y = v1[3 * t + a], z = v2[3 * t + a];
-      q.lo[a] = std::min(std::min(x, y), z);
-      q.hi[a] = std::max(std::max(x, y), z);
-      q.c[a] = ((x + y) + z) / 3.0f;
+  parallel_chunks(T, [&](int b, int e) {
+    for (int t = b; t < e; ++t) {
+      Prim &q = prims[t];
+      for (int a = 0; a < 3; ++a) {
+        const float x = v0[3 * (size_t)t + a], y = v1[3 * (size_t)t + a], z = v2[3 * (size_t)t + a];
+        q.lo[a] = std::min(std::min(x, y), z);
+        q.hi[a] = std::max(std::max(x, y), z);
+        q.c[a] = ((x + y) + z) / 3.0f;
+      }
     }
-  }
+  });
   return prims;
 }
 
@@ -541,7 +517,7 @@ bool build_bvh_binned(int T, const float *v0, const float *v1, const float *v2, 
     }
   }
   out.sah_cost = cost;
-  return flatten_two_child(std::move(tree), prims, out.perm, out, err, p.width, p.quantize);
+  return flatten_tree(std::move(tree), prims, out.perm, out, err, p.width, p.quantize);
 }
 
 bool bvh_from_reference(int T, const float *v0, const float *v1, const float *v2, int N, const float *nmin,
@@ -596,7 +572,7 @@ bool bvh_from_reference(int T, const float *v0, const float *v1, const float *v2
       out.ref_link[i] = make_int4(left[i], right[i], 0, 0);
     }
   }
-  return flatten_two_child(std::move(tree), prims, out.perm, out, err, width, quantize);
+  return flatten_tree(std::move(tree), prims, out.perm, out, err, width, quantize);
 }
 
 }  // namespace ts

@@ -3,10 +3,34 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
+#include <thread>
 #include <vector>
 
 namespace ts {
+
+// f(begin, end) over [0, n) in chunks, on up to 8 threads where there is enough to share
+template <class F>
+void parallel_chunks(int n, F f) {
+  const int nt = std::min({8, (int)std::max(1u, std::thread::hardware_concurrency()), n / 16384});
+  if (nt <= 1) {
+    f(0, n);
+    return;
+  }
+  std::vector<std::thread> th;
+  th.reserve(nt);
+  for (int k = 1; k < nt; ++k) {
+    const int b = (int)((int64_t)n * k / nt), e = (int)((int64_t)n * (k + 1) / nt);
+    try {
+      th.emplace_back(f, b, e);
+    } catch (...) {  // no thread to be had
+      f(b, e);
+    }
+  }
+  f(0, (int)((int64_t)n / nt));
+  for (std::thread &x : th) x.join();
+}
 
 struct BvhParams {
   int bins = 32;          // SAH bins per axis
@@ -21,8 +45,9 @@ struct BvhParams {
 
 struct BvhOut {
   std::vector<int32_t> perm;   // slot -> original triangle index
-  std::vector<float4> node2;   // device layout: width 2 -> 4 float4 per node, 4 -> 8, 8 -> 16
-  int width = 2;               // node width of node2 (a wide layout falls back to 2 if its stack bound is exceeded)
+  std::vector<float4> node2;   // device nodes: 8 float4 each for the layouts of width 2 and 4, 16 for 8
+  int width = 2;               // node width of the layout (a wide layout falls back to 2 if its stack bound is exceeded)
+  int two_child_nodes = 0;     // inner nodes of the binary tree (1 for a lone leaf)
   bool quantized = false;      // node2 holds quantized wide nodes
   int stack_need = 0;          // deepest traversal stack the device layout can require
   std::vector<float> ref_min, ref_max;  // reference layout, [N][3]
@@ -40,7 +65,7 @@ bool build_bvh_binned(int T, const float *v0, const float *v1, const float *v2, 
 // boxes as bytes relative to the node's origin -- 4 float4 for 4-wide, 6 for 8-wide).
 inline int node_float4s(int width, bool quantized = false) {
   if (quantized) return width == 8 ? 6 : 4;
-  return width == 8 ? 16 : (width == 4 ? 8 : 4);
+  return width == 8 ? 16 : 8;  // width 2: the binary tree collapsed to four children
 }
 // the device layout id: the node width, plus one for quantized child boxes (5, 9)
 inline int layout_id(int width, bool quantized) { return quantized && width >= 4 ? width + 1 : width; }

@@ -31,7 +31,6 @@ struct DevConfig {
   int32_t max_depth, scatter_bounces;
   float aspect, fov;
   uint32_t seed, scene_id;
-  int32_t speculative;  // two-child layout: speculative while-while traversal
 };
 
 // Device scene.  Triangles are in BVH leaf order ("slot" order).
@@ -39,18 +38,15 @@ struct DevConfig {
 //   tri[3*s+1] = (e1.xyz, material bits)     e1 = v1 - v0 (float32)
 //   tri[3*s+2] = (e2.xyz, 0)                 e2 = v2 - v0 (float32)
 //   shade[3*s+k] = (n_k.xyz, geometric_normal[k])
-// Wide nodes (width 4 / 8): six rows of child-box bounds (lo.x hi.x lo.y hi.y
-// lo.z hi.z, one float per child) followed by the child links, 128 / 256 B.
-// Two-child BVH nodes, 64 B each:
-//   node[4*i+0] = (c0.lo.x, c0.hi.x, c0.lo.y, c0.hi.y)
-//   node[4*i+1] = (c1.lo.x, c1.hi.x, c1.lo.y, c1.hi.y)
-//   node[4*i+2] = (c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z)
-//   node[4*i+3] = (child0, child1, -, -) as int; child >= 0 is an inner node,
-//                 child < 0 is a leaf: ~child = (first_slot << 4) | (count - 1)
+// Wide nodes (width 4 / 8): one 32-byte record per child,
+//   (lo.x, hi.x, lo.y, hi.y), (lo.z, hi.z, link, -)
+// A child >= 0 is an inner node, < 0 a leaf: ~child = (first_slot << 4) |
+// (count - 1).  The two-child layout's device nodes are its tree collapsed to
+// four children.
 // Reference-layout nodes (main.py:267-275) are kept for the exact-order
-// traversal used by parity checks.
+// traversal used by parity checks and for the two-child order.
 struct DevScene {
-  const float4 *__restrict__ node;    // device BVH layout (node_width children per node)
+  const float4 *__restrict__ node;    // device BVH layout
   const float4 *__restrict__ tri;
   const float4 *__restrict__ shade;
   int32_t num_nodes, num_tris;

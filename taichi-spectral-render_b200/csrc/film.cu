@@ -87,7 +87,7 @@ __global__ void k_resolve_rgb(Film f, const float *__restrict__ cmf, double scal
 
 // visualize_normals, main.py:1631-1659 (render-resolution part)
 template <int W>
-__global__ void k_normals(DevScene s, DevConfig c, float *__restrict__ out, uint32_t *err) {
+__global__ void k_normals(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, float *__restrict__ out, uint32_t *err) {
   const int npix = c.W * c.H;
   uint32_t eb = 0;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
@@ -107,7 +107,7 @@ __global__ void k_normals(DevScene s, DevConfig c, float *__restrict__ out, uint
 }
 
 template <int kMode, int W>
-__global__ void k_trace_batch(DevScene s, float eps, const float *__restrict__ rays, int n,
+__global__ void k_trace_batch(const __grid_constant__ DevScene s, float eps, const float *__restrict__ rays, int n,
                               int32_t *__restrict__ tri_orig, float *__restrict__ t, float *__restrict__ u,
                               float *__restrict__ v, uint32_t *err) {
   uint32_t eb = 0;

@@ -84,7 +84,7 @@ constexpr int kMaxKeys = 256;
 // capacity: paths per chunk of the frame (0 = the whole frame); w holds at least that many slots
 cudaError_t launch_wave_pass(const DevScene &s, const DevConfig &c, uint32_t pass, int band, Film f,
                              const WaveBuffers &w, uint32_t *err, int grid, int block, int sort_keys,
-                             cudaStream_t st, int trace_budget, int capacity = 0);
+                             cudaStream_t st, int capacity = 0);
 
 // npass passes from pass0 / band0 (band wrapping mod B) over `capacity` path
 // slots (<= w.capacity) with path regeneration, as a CUDA-graph while-loop.
@@ -92,8 +92,7 @@ cudaError_t launch_wave_pass(const DevScene &s, const DevConfig &c, uint32_t pas
 struct WaveLoopGraph;
 // host_driven: launch the iterations from the host instead (one stream sync each)
 cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pass0, int band0, int npass, Film f,
-                             const WaveBuffers &w, uint32_t *err, int grid, int block, cudaStream_t st,
-                             int trace_budget, int capacity, WaveLoopGraph **graph, bool host_driven = false,
+                             const WaveBuffers &w, uint32_t *err, int grid, int block, cudaStream_t st, int capacity, WaveLoopGraph **graph, bool host_driven = false,
                              int limit_override = 0);
 void free_wave_loop(WaveLoopGraph *graph);
 
@@ -116,6 +115,6 @@ size_t noalloc_scratch_bytes();
 cudaError_t noalloc_setup(int device, void **ptr);
 cudaError_t launch_wave_tile_noalloc(const DevScene &s, const DevConfig &c, uint32_t pass, int band, Film f,
                                      void *scratch, int x0, int y0, int tw, int th, uint32_t *err, int grid,
-                                     int block, cudaStream_t st, int trace_budget);
+                                     int block, cudaStream_t st);
 
 }  // namespace ts

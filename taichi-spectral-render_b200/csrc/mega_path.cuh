@@ -55,14 +55,14 @@ __device__ __forceinline__ void mega_start(const DevScene &s, const DevConfig &c
 }
 
 // Returns true when the path has ended (its deposit flushed).
-template <int W, bool kCount>
+template <int W, bool kCount, bool kTogether = true>
 __device__ __forceinline__ bool mega_vertex(const DevScene &s, const DevConfig &c, const Film &f, MegaLane &L,
                                             uint32_t &errbits, MegaCounts &cnt, bool shared) {
   PathState &p = L.p;
   const int band = L.band;
   bool done = false;
   // hits beyond ESCAPE count as escapes (main.py:1209-1214): traverse no further
-  const Hit h = trace_closest<W, kCount>(s, p.pos, p.dir, c.eps, errbits, &cnt.tc, c.escape);
+  const Hit h = trace_closest<W, kCount, kTogether>(s, p.pos, p.dir, c.eps, errbits, &cnt.tc, c.escape);
   const VolEvent ev = volume_event(s, c, p, h, L.rng);
   if (kCount) {
     cnt.trace++;
@@ -97,7 +97,7 @@ __device__ __forceinline__ bool mega_vertex(const DevScene &s, const DevConfig &
       ss.seg = 0;
       for (;;) {
         const Hit sh =
-            trace_closest<W, kCount>(s, ss.pos, q.dir, c.eps, errbits, &cnt.tc, shadow_bound(s, c, q, ss, p.active));
+            trace_closest<W, kCount, kTogether>(s, ss.pos, q.dir, c.eps, errbits, &cnt.tc, shadow_bound(s, c, q, ss, p.active));
         if (kCount) {
           cnt.trace++;
           cnt.hit += sh.slot >= 0 && sh.slot != q.light_slot;

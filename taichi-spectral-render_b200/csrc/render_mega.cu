@@ -22,7 +22,7 @@ namespace {
 // (5: 96 registers, no spills; 8: 64 registers with local-memory spills --
 // more warps to hide the node-fetch latency, faster on large frames).
 template <int W, bool kCount, int kMinBlocks = 5>
-__global__ void __launch_bounds__(128, kMinBlocks) k_render_mega(DevScene s, DevConfig c, uint32_t pass0, int npass, int band0,
+__global__ void __launch_bounds__(128, kMinBlocks) k_render_mega(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass0, int npass, int band0,
                                                      Film f, int *__restrict__ counter, uint32_t *__restrict__ err,
                                                      unsigned long long *__restrict__ work) {
   const int lane = threadIdx.x & 31;
@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(128, kMinBlocks) k_render_mega(DevScene s, Dev
     }
     if (__ballot_sync(0xffffffffu, L.pix >= 0) == 0) break;
     if (L.pix < 0) continue;
-    mega_vertex<W, kCount>(s, c, f, L, errbits, cnt, npass > 1);
+    mega_vertex<W, kCount, false>(s, c, f, L, errbits, cnt, npass > 1);
   }
   if (errbits) atomicOr(err, errbits);
   if (kCount) {
@@ -91,7 +91,6 @@ cudaError_t launch_render_mega(const DevScene &s, const DevConfig &c, uint32_t p
   else if (s.node_width == 5) launch_w<5>(s, c, pass, npass, band, f, counter, err, grid, block, st, work, occupancy);
   else if (s.node_width == 8) launch_w<8>(s, c, pass, npass, band, f, counter, err, grid, block, st, work, occupancy);
   else if (s.node_width == 4) launch_w<4>(s, c, pass, npass, band, f, counter, err, grid, block, st, work, occupancy);
-  else if (c.speculative) launch_w<3>(s, c, pass, npass, band, f, counter, err, grid, block, st, work, occupancy);
   else launch_w<2>(s, c, pass, npass, band, f, counter, err, grid, block, st, work, occupancy);
   return cudaGetLastError();
 }

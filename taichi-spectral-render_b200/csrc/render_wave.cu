@@ -78,7 +78,7 @@ __device__ __forceinline__ void start_path(float3 o, float3 cu, float3 cv, float
 }
 
 // camera rays of pixels [p0, p0 + n): path slot q <-> pixel p0 + q
-__global__ void k_generate(DevScene s, DevConfig c, uint32_t pass, int band, WaveBuffers w, int p0, int n) {
+__global__ void k_generate(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass, int band, WaveBuffers w, int p0, int n) {
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
     start_path(s.cam_o, s.cam_u, s.cam_v, s.cam_w, c, pass, band, p0 + q, w, q);
     w.queue[0][q] = q;
@@ -86,145 +86,333 @@ __global__ void k_generate(DevScene s, DevConfig c, uint32_t pass, int band, Wav
   if (blockIdx.x == 0 && threadIdx.x == 0) w.counts[kCntExt + 0] = n;
 }
 
+// ---- the trace stage ---------------------------------------------------------
+// Work items are shadow queries (a query's whole chain of segments) and extension
+// rays.  Two ways to run them, for the same results: a ray per lane, the lanes of
+// a warp stepping together (trace_lanes), and a group of lanes per ray
+// (trace_groups).  launch_trace() says which when.
+struct TraceItems {
+  int nsh, total;           // shadow queries [0, nsh), then extension rays
+  const int *q;             // path slots of the extension rays
+  const int *shadow_order;  // nullptr: queries in order
+  int *fetch;
+};
+
+// what a work item renders: one scene, or a view of a batch
+struct OneScene {
+  const DevScene &s;
+  const DevConfig &c;
+  const Film &f;
+  bool shared_film;
+  __device__ __forceinline__ int view_of_query(const WaveBuffers &, int) const { return 0; }
+  __device__ __forceinline__ int view_of_path(const WaveBuffers &, int) const { return 0; }
+  __device__ __forceinline__ const DevScene &scene(int) const { return s; }
+  __device__ __forceinline__ const DevConfig &config(int) const { return c; }
+  __device__ __forceinline__ const Film &film(int) const { return f; }
+  __device__ __forceinline__ bool shared(int) const { return shared_film; }
+};
+
+// the next work item for each lane that wants one (one atomic per warp; G lanes
+// of a group share one), -1 for the others
+template <int G>
+__device__ __forceinline__ int fetch_items(int *fetch, bool want) {
+  const unsigned m = __ballot_sync(0xffffffffu, want);
+  if (!m) return -1;
+  const int lane = threadIdx.x & 31;
+  const int leader = __ffs(m) - 1;
+  int base = 0;
+  if (lane == leader) base = atomicAdd(fetch, __popc(m) / G);
+  base = __shfl_sync(0xffffffffu, base, leader);
+  return want ? base + __popc(m & ((1u << (lane & ~(G - 1))) - 1u)) / G : -1;
+}
+
+__device__ __forceinline__ ShadowQuery load_query(const WaveBuffers &w, int qi, int &pixel, int &band, int &dep_band) {
+  const float4 o = w.sq_origin[qi], d = w.sq_dir[qi];
+  const int4 m = w.sq_meta[qi];
+  ShadowQuery q;
+  q.origin = xyz(o);
+  q.max_dist = o.w;
+  q.dir = xyz(d);
+  q.contrib = d.w;
+  q.light_slot = m.y;
+  q.vol = m.z;
+  pixel = m.x;
+  band = m.w & 0xff;
+  dep_band = m.w >> 8;
+  return q;
+}
+
+// A work item under way.  Only what changes from one traversal to the next is
+// held in registers; a query's constants are read again when a segment ends.
+struct TraceItem {
+  int id = -1;        // shadow query or path slot, -1: none
+  int view = 0;
+  bool shadow = false;
+  bool plain = false;  // waits for item_plain()
+  float total = 0.f, traveled = 0.f;  // of the shadow chain
+  int vol_seg = 0;                    // medium | segment << 24
+};
+
+// begin(scene, origin, direction, bound) starts the ray, once in each branch: a
+// ray carried from the branches to one common start costs the hot loop its
+// registers (10 % of the launch).
+template <class Src, class Begin>
+__device__ __forceinline__ void item_start(const Src &src, const WaveBuffers &w, const TraceItems &it, int idx,
+                                           TraceItem &im, Begin begin) {
+  im.plain = false;
+  im.shadow = idx < it.nsh;
+  if (im.shadow) {
+    im.id = it.shadow_order ? it.shadow_order[idx] : idx;
+    im.view = src.view_of_query(w, im.id);
+    int pixel, band, dep_band;
+    const ShadowQuery q = load_query(w, im.id, pixel, band, dep_band);
+    im.total = 1.f;
+    im.traveled = 0.f;
+    im.vol_seg = q.vol;
+    const ShadowState ss{q.origin, 1.f, 0.f, q.vol, 0};
+    const DevScene &s = src.scene(im.view);
+    begin(s, q.origin, q.dir, shadow_bound(s, src.config(im.view), q, ss, band));
+  } else {
+    im.id = it.q[idx - it.nsh];
+    im.view = src.view_of_path(w, im.id);
+    begin(src.scene(im.view), xyz(w.pos_thr[im.id]), xyz(w.dir_spdf[im.id]), src.config(im.view).escape);
+  }
+}
+
+// The item's ray has hit h (or missed).  An extension ray's hit is stored; a
+// shadow segment goes on to the next, or the chain deposits and ends.
+// writer: this lane stores.
+template <class Src, class Begin>
+__device__ __forceinline__ void item_hit(const Src &src, const WaveBuffers &w, TraceItem &im, const Hit &h, bool writer,
+                                         Begin begin) {
+  const int id = im.id;
+  if (!im.shadow) {
+    if (writer) w.hit[id] = make_float4(h.t, h.u, h.v, __int_as_float(h.slot));
+    im.id = -1;
+    return;
+  }
+  const DevScene &s = src.scene(im.view);
+  const DevConfig &c = src.config(im.view);
+  int pixel, band, dep_band;
+  const ShadowQuery q = load_query(w, id, pixel, band, dep_band);
+  ShadowState ss{q.origin, im.total, im.traveled, im.vol_seg & 0xffffff, im.vol_seg >> 24};
+  if (shadow_segment(s, c, q, h, band, ss)) {
+    if (writer && ss.total > 1e-6f) deposit(src.film(im.view), pixel, dep_band, q.contrib * ss.total, src.shared(im.view));
+    im.id = -1;
+  } else {
+    im.total = ss.total;
+    im.traveled = ss.traveled;
+    im.vol_seg = ss.vol | ss.seg << 24;
+    begin(s, ss.pos, q.dir, shadow_bound(s, c, q, ss, band));
+  }
+}
+
+// The whole work item through trace_plain(), outside the hot loop, whose
+// registers a call would spill; a shadow chain starts over, with the same hits.
+template <int W>
+__device__ __noinline__ void item_plain(const DevScene &s, const DevConfig &c, const Film &f, const WaveBuffers &w,
+                                        int id, bool shadow, bool shared, uint32_t &eb) {
+  if (!shadow) {
+    const Hit h = trace_plain<W>(s, xyz(w.pos_thr[id]), xyz(w.dir_spdf[id]), c.eps, eb, c.escape);
+    w.hit[id] = make_float4(h.t, h.u, h.v, __int_as_float(h.slot));
+    return;
+  }
+  int pixel, band, dep_band;
+  const ShadowQuery q = load_query(w, id, pixel, band, dep_band);
+  ShadowState ss{q.origin, 1.f, 0.f, q.vol, 0};
+  for (;;) {
+    const Hit h = trace_plain<W>(s, ss.pos, q.dir, c.eps, eb, shadow_bound(s, c, q, ss, band));
+    if (shadow_segment(s, c, q, h, band, ss)) break;
+  }
+  if (ss.total > 1e-6f) deposit(f, pixel, dep_band, q.contrib * ss.total, shared);
+}
+
+// Items whose result a tie left open, once no lane of the warp has a ray; returns
+// false when the warp is out of work.
+template <int W, class Src>
+__device__ __forceinline__ bool run_plain(const Src &src, const WaveBuffers &w, TraceItem &im, bool writer,
+                                          bool exhausted, uint32_t &eb) {
+  if (im.id >= 0 && im.plain) {
+    if (writer)
+      item_plain<W>(src.scene(im.view), src.config(im.view), src.film(im.view), w, im.id, im.shadow,
+                    src.shared(im.view), eb);
+    im.id = -1;
+  }
+  im.plain = false;
+  return __ballot_sync(0xffffffffu, im.id >= 0 || !exhausted) != 0;
+}
+
+// A ray per lane.  A warp looks every kPhases phases for lanes that have
+// finished, and ends their items and starts others once kIdleLanes of them wait:
+// the end of a shadow segment is as long as three node tests, and when every
+// finished lane had its own, it ran with two lanes of 32.
+constexpr int kPhases = 4;      // 1: 5 % slower, 8: the same
+constexpr int kIdleLanes = 16;  // 4 / 8 / 12: 11 / 5 / 1 % slower, 20: 3 % slower on the volume
+
+template <int W, class Src>
+__device__ __forceinline__ void trace_lanes(const Src &src, const WaveBuffers &w, const TraceItems &it,
+                                            uint32_t &eb) {
+  constexpr unsigned kFull = 0xffffffffu;
+  TraceItem im;
+  Traversal t;
+  t.node = kTravDone;
+  t.tie = 0;
+  int2 stack[kWideStack];
+  bool exhausted = false;
+  for (;;) {
+    const bool done = t.node == kTravDone && !im.plain;
+    const unsigned idle = __ballot_sync(kFull, done && !(exhausted && im.id < 0));
+    if (__popc(idle) >= kIdleLanes || __ballot_sync(kFull, t.node != kTravDone) == 0) {
+      const auto begin = [&](const DevScene &s, float3 o, float3 d, float bound) { trav_begin<W>(s, t, o, d, bound); };
+      if (done && im.id >= 0) {
+        im.plain = trav_tied<W>(t);
+        if (!im.plain) item_hit(src, w, im, t.h, true, begin);
+      }
+      __syncwarp();
+      const int idx = fetch_items<1>(it.fetch, im.id < 0 && !exhausted);
+      if (idx >= 0) {
+        exhausted = idx >= it.total;
+        if (!exhausted) item_start(src, w, it, idx, im, begin);
+      }
+      if (__ballot_sync(kFull, t.node != kTravDone) == 0) {
+        if (!run_plain<W>(src, w, im, true, exhausted, eb)) break;
+        continue;
+      }
+    }
+    const DevScene &s = src.scene(im.view);
+    const float eps = src.config(im.view).eps;
+#pragma unroll 1
+    for (int i = 0; i < kPhases; ++i)
+      if (!warp_phase<Nodes<W>::value>(s, t, stack, eps, eb)) break;
+  }
+}
+
+// A group of lanes per ray (full-precision nodes), looking for finished groups
+// every kGroupSteps steps and stopping for kGroupIdle of them.
+constexpr int kGroupSteps = 2, kGroupIdle = 2;
+
+template <int W, class Src>
+__device__ __forceinline__ void trace_groups(const Src &src, const WaveBuffers &w, const TraceItems &it, int2 *stacks,
+                                             uint32_t &eb) {
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int G = W == 8 ? 8 : 4;
+  const int lane = threadIdx.x & 31, sub = lane & (G - 1), shift = lane & ~(G - 1);
+  const int stride = blockDim.x / G;
+  int2 *stack = stacks + threadIdx.x / G;
+  TraceItem im;
+  GroupRay<G> t;
+  t.node = kTravDone;
+  t.sp = 0;
+  t.over = false;
+  t.h.t = 1e9f;
+  t.h.u = t.h.v = 0.f;
+  t.h.slot = -1;
+  t.tie = false;
+  bool exhausted = false;
+  for (;;) {
+    const bool done = t.node == kTravDone && !im.plain;
+    const unsigned idle = __ballot_sync(kFull, done && !(exhausted && im.id < 0));
+    if (__popc(idle) >= kGroupIdle * G || __ballot_sync(kFull, t.node != kTravDone) == 0) {
+      Hit h;
+      const bool good = group_hit(t, shift, h);
+      const auto begin = [&](const DevScene &s, float3 o, float3 d, float bound) { group_begin(s, t, o, d, bound); };
+      if (done && im.id >= 0) {
+        im.plain = !good;
+        if (good) item_hit(src, w, im, h, sub == 0, begin);
+      }
+      __syncwarp();
+      const int idx = fetch_items<G>(it.fetch, im.id < 0 && !exhausted);
+      if (idx >= 0) {
+        exhausted = idx >= it.total;
+        if (!exhausted) item_start(src, w, it, idx, im, begin);
+      }
+      if (__ballot_sync(kFull, t.node != kTravDone) == 0) {
+        if (!run_plain<W>(src, w, im, sub == 0, exhausted, eb)) break;
+        continue;
+      }
+    }
+    const DevScene &s = src.scene(im.view);
+    const float eps = src.config(im.view).eps;
+#pragma unroll 1
+    for (int i = 0; i < kGroupSteps; ++i) group_step(s, t, stack, stride, sub, shift, eps);
+  }
+}
+
 // trace(k): shadow chains of shade(k-1), then extension hits of Qk.
-// Persistent lanes with per-lane refill: each lane traverses its current ray
-// for at most `budget` steps; lanes whose ray has finished then take new work
-// items (one atomic per warp), so a warp does not idle behind its longest ray.
 // kLoop: one iteration of the regenerating loop (queue lengths from *L).
-template <int W, bool kLoop = false>
-__global__ void __launch_bounds__(kMaxBlock, 4) k_trace(DevScene s, DevConfig c, int depth, Film f, WaveBuffers w,
-                                                     uint32_t *__restrict__ err, int budget, int ext_sorted,
-                                                     int shadow_sorted, WaveLoop *L) {
-  uint32_t eb = 0;
-  int nsh, next, *fetch;
-  const int *q;
-  bool shared = false;
+template <bool kLoop>
+__device__ __forceinline__ TraceItems trace_items(const DevConfig &c, int depth, const WaveBuffers &w, int ext_sorted,
+                                                  int shadow_sorted, WaveLoop *L) {
+  TraceItems it;
+  int next;
   if (kLoop) {
     const int a = L->iter & 1;
-    nsh = L->sh[a ^ 1];
+    it.nsh = L->sh[a ^ 1];
     next = L->ext[a];
-    q = w.queue[a];
-    fetch = L->fetch + 0;
-    shared = L->shared != 0;
-    ext_sorted = shadow_sorted = 0;
+    it.q = w.queue[a];
+    it.fetch = L->fetch + 0;
+    it.shadow_order = nullptr;
   } else {
-    nsh = depth > 0 ? w.counts[kCntSh + depth - 1] : 0;
+    it.nsh = depth > 0 ? w.counts[kCntSh + depth - 1] : 0;
     next = depth < c.max_depth ? w.counts[kCntExt + depth] : 0;
-    q = ext_sorted ? w.trace_order : w.queue[depth & 1];
-    fetch = w.counts + kCntFetchT + depth;
+    it.q = ext_sorted ? w.trace_order : w.queue[depth & 1];
+    it.fetch = w.counts + kCntFetchT + depth;
+    it.shadow_order = shadow_sorted ? w.shadow_order : nullptr;
   }
-  const int total = nsh + next;
-  const int lane = threadIdx.x & 31;
-  int item = -1, pid = 0, pixel = 0, band = 0, dep_band = 0;
-  bool exhausted = false;
-  Traversal t;
-  int2 stack[StackSize<W>::value];
-#ifdef TS_SHORT_STACK
-  // measurement variant: the newest TS_SHORT_STACK entries of each lane's
-  // wide-node stack in shared memory (dynamic, TS_SHORT_STACK x block entries)
-  extern __shared__ int2 short_stack_smem[];
-  ShortStack<TS_SHORT_STACK> sst{short_stack_smem, stack, (int)blockDim.x, (int)threadIdx.x, 0};
-#endif
-  ShadowQuery sq;
-  ShadowState ss;
-  for (;;) {
-    const bool need = item < 0 && !exhausted;
-    const unsigned m = __ballot_sync(0xffffffffu, need);
-    if (m) {
-      const int leader = __ffs(m) - 1;
-      int base = 0;
-      if (lane == leader) base = atomicAdd(fetch, __popc(m));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (need) {
-        const int idx = base + __popc(m & ((1u << lane) - 1u));
-        if (idx >= total) {
-          exhausted = true;
-        } else if (idx < nsh) {
-          item = idx;
-          const int qi = shadow_sorted ? w.shadow_order[idx] : idx;
-          const float4 o = w.sq_origin[qi], d = w.sq_dir[qi];
-          const int4 mm = w.sq_meta[qi];
-          sq.origin = xyz(o);
-          sq.max_dist = o.w;
-          sq.dir = xyz(d);
-          sq.contrib = d.w;
-          sq.light_slot = mm.y;
-          sq.vol = mm.z;
-          pixel = mm.x;
-          band = mm.w & 0xff;
-          dep_band = mm.w >> 8;
-          ss.pos = sq.origin;
-          ss.total = 1.f;
-          ss.traveled = 0.f;
-          ss.vol = sq.vol;
-          ss.seg = 0;
-          trav_begin(s, t, ss.pos, sq.dir, shadow_bound(s, c, sq, ss, band));
-        } else {
-          item = idx;
-          pid = q[idx - nsh];
-          const float4 pt = w.pos_thr[pid], ds = w.dir_spdf[pid];
-          trav_begin(s, t, xyz(pt), xyz(ds), c.escape);
-        }
-      }
-    }
-    if (__ballot_sync(0xffffffffu, item >= 0) == 0) break;
-    bool done = false;
-#if defined(TS_IDLE_REFILL)
-    // measurement variant: the warp steps its rays one traversal step at a
-    // time and refills as soon as TS_IDLE_REFILL lanes could take new work
-    // (dynamic fetch), within the same bound of `budget` steps
-    for (int st = 0; st < budget; ++st) {
-      if (item >= 0 && !done) done = trav_advance<W>(s, t, stack, c.eps, 1, eb);
-      if (__popc(__ballot_sync(0xffffffffu, done || (item < 0 && !exhausted))) >= TS_IDLE_REFILL) break;
-    }
-#else
-    if (item >= 0) {
-#ifdef TS_SHORT_STACK
-      if constexpr (W == 4 || W == 8) done = trav_steps_wide<W>(s, t, sst, c.eps, budget, eb);
-      else done = trav_advance<W>(s, t, stack, c.eps, budget, eb);
-#else
-      done = trav_advance<W>(s, t, stack, c.eps, budget, eb);
-#endif
-    }
-#endif
-    if (done) {
-      if (item < nsh) {
-        if (shadow_segment(s, c, sq, t.h, band, ss)) {
-          if (ss.total > 1e-6f) deposit(f, pixel, dep_band, sq.contrib * ss.total, shared);
-          item = -1;
-        } else {
-          trav_begin(s, t, ss.pos, sq.dir, shadow_bound(s, c, sq, ss, band));
-        }
-      } else {
-        w.hit[pid] = make_float4(t.h.t, t.h.u, t.h.v, __int_as_float(t.h.slot));
-        item = -1;
-      }
-    }
-  }
+  it.total = it.nsh + next;
+  return it;
+}
+
+template <int W, bool kLoop, bool kGroups>
+__global__ void __launch_bounds__(kMaxBlock, 4) k_trace(const __grid_constant__ DevScene s,
+                                                     const __grid_constant__ DevConfig c, int depth,
+                                                     const __grid_constant__ Film f,
+                                                     const __grid_constant__ WaveBuffers w,
+                                                     uint32_t *__restrict__ err, int ext_sorted,
+                                                     int shadow_sorted, WaveLoop *L) {
+  extern __shared__ int2 group_stacks[];  // kGroups: [kGroupStack][groups of the block]
+  uint32_t eb = 0;
+  const TraceItems it = trace_items<kLoop>(c, depth, w, ext_sorted, shadow_sorted, L);
+  const OneScene src{s, c, f, kLoop && L->shared != 0};
+  if constexpr (kGroups) trace_groups<W>(src, w, it, group_stacks, eb);
+  else trace_lanes<W>(src, w, it, eb);
   if (eb) atomicOr(err, eb);
 }
 
+// Groups of lanes up to this many path slots, a ray per lane above.  A ray per
+// lane costs half the instructions of a group per step once the schedulers are
+// full; below that the length of a warp's step counts, where a group's is a
+// third.  Measured per pass (ms, lanes / groups): box 256^2 1.10 / 0.88, 384^2
+// 1.23 / 1.15, 512^2 1.44 / 1.56; terrain (647k triangles) 256^2 1.36 / 0.89,
+// 512^2 1.72 / 1.38, 1024^2 2.76 / 3.21; volume 256^2 7.6 / 5.1, 384^2 8.7 / 7.4,
+// 512^2 10.4 / 10.9.
+constexpr int kGroupPaths = 148 * 1024 * 3 / 2;
+
+template <int W, bool kLoop>
+void launch_trace_w(const DevScene &s, const DevConfig &c, int depth, Film f, const WaveBuffers &w, uint32_t *err,
+                    int grid, int block, cudaStream_t st, int ext_sorted, int shadow_sorted, WaveLoop *L,
+                    int paths) {
+  if constexpr (W != 5 && W != 9) {
+    if (paths <= kGroupPaths) {
+      const size_t smem = (size_t)(block / (W == 8 ? 8 : 4)) * kGroupStack * sizeof(int2);
+      k_trace<W, kLoop, true><<<grid, block, smem, st>>>(s, c, depth, f, w, err, ext_sorted, shadow_sorted, L);
+      return;
+    }
+  }
+  k_trace<W, kLoop, false><<<grid, block, 0, st>>>(s, c, depth, f, w, err, ext_sorted, shadow_sorted, L);
+}
+
+// paths: path slots in use, the most extension rays (and shadow queries) the stage can have
 template <bool kLoop = false>
 void launch_trace(const DevScene &s, const DevConfig &c, int depth, Film f, const WaveBuffers &w, uint32_t *err,
-                  int grid, int block, cudaStream_t st, int budget, int ext_sorted = 0, int shadow_sorted = 0,
-                  WaveLoop *L = nullptr) {
-#ifdef TS_SHORT_STACK
-  const size_t smem = (size_t)TS_SHORT_STACK * block * sizeof(int2);
-#else
-  const size_t smem = 0;
-#endif
-  if (s.node_width == 9)
-    k_trace<9, kLoop><<<grid, block, smem, st>>>(s, c, depth, f, w, err, budget, ext_sorted, shadow_sorted, L);
-  else if (s.node_width == 5)
-    k_trace<5, kLoop><<<grid, block, smem, st>>>(s, c, depth, f, w, err, budget, ext_sorted, shadow_sorted, L);
-  else if (s.node_width == 8)
-    k_trace<8, kLoop><<<grid, block, smem, st>>>(s, c, depth, f, w, err, budget, ext_sorted, shadow_sorted, L);
-  else if (s.node_width == 4)
-    k_trace<4, kLoop><<<grid, block, smem, st>>>(s, c, depth, f, w, err, budget, ext_sorted, shadow_sorted, L);
-  else if (c.speculative)
-    k_trace<3, kLoop><<<grid, block, smem, st>>>(s, c, depth, f, w, err, budget, ext_sorted, shadow_sorted, L);
-  else
-    k_trace<2, kLoop><<<grid, block, smem, st>>>(s, c, depth, f, w, err, budget, ext_sorted, shadow_sorted, L);
+                  int grid, int block, cudaStream_t st, int paths, int ext_sorted = 0,
+                  int shadow_sorted = 0, WaveLoop *L = nullptr) {
+  const auto go = s.node_width == 9   ? launch_trace_w<9, kLoop>
+                  : s.node_width == 5 ? launch_trace_w<5, kLoop>
+                  : s.node_width == 8 ? launch_trace_w<8, kLoop>
+                  : s.node_width == 4 ? launch_trace_w<4, kLoop>
+                                      : launch_trace_w<2, kLoop>;
+  go(s, c, depth, f, w, err, grid, block, st, ext_sorted, shadow_sorted, L, paths);
 }
 
 // ---- queue sorting ------------------------------------------------------
@@ -262,7 +450,7 @@ __device__ __forceinline__ int sort_key(const DevScene &s, const WaveBuffers &w,
   return kind == kSortShade ? (key < nkeys ? key : nkeys - 1) : (key & (nkeys - 1));
 }
 
-__global__ void k_sort_count(DevScene s, int depth, WaveBuffers w, int kind, int nkeys) {
+__global__ void k_sort_count(const __grid_constant__ DevScene s, int depth, WaveBuffers w, int kind, int nkeys) {
   __shared__ int hist[kMaxKeys];
   for (int k = threadIdx.x; k < nkeys; k += blockDim.x) hist[k] = 0;
   __syncthreads();
@@ -286,7 +474,7 @@ __global__ void k_sort_scan(WaveBuffers w, int nkeys) {
   }
 }
 
-__global__ void k_sort_scatter(DevScene s, int depth, WaveBuffers w, int kind, int nkeys, int *__restrict__ out) {
+__global__ void k_sort_scatter(const __grid_constant__ DevScene s, int depth, WaveBuffers w, int kind, int nkeys, int *__restrict__ out) {
   const int n = sort_count_of(w, kind, depth);
   const int lane = threadIdx.x & 31;
   const int stride = gridDim.x * blockDim.x;
@@ -410,7 +598,7 @@ __device__ __forceinline__ void append_ext(int *count, int *q, int pid, bool wan
   else atomicOr(err, kErrQueueOverflow);
 }
 
-__global__ void __launch_bounds__(kMaxBlock) k_shade(DevScene s, DevConfig c, uint32_t pass, int band, int depth,
+__global__ void __launch_bounds__(kMaxBlock) k_shade(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass, int band, int depth,
                                                Film f, WaveBuffers w, int use_sorted, uint32_t *err) {
   const int n = w.counts[kCntExt + depth];
   const int *q = use_sorted ? w.sorted : w.queue[depth & 1];
@@ -450,7 +638,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_shade(DevScene s, DevConfig c, ui
 // share cells (several passes with fluorescence moving deposits across bands).
 
 // paths [0, n0) of the launch into slots [0, n0), and the loop state
-__global__ void k_loop_init(DevScene s, DevConfig c, WaveBuffers w, WaveLoop *L, uint32_t pass0, int band0,
+__global__ void k_loop_init(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, WaveBuffers w, WaveLoop *L, uint32_t pass0, int band0,
                             int npass, int n0, int limit, int shared) {
   const int npix = c.W * c.H;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n0; q += gridDim.x * blockDim.x) {
@@ -482,7 +670,7 @@ __global__ void k_loop_init(DevScene s, DevConfig c, WaveBuffers w, WaveLoop *L,
 
 // 64 registers (4 resident 256-thread blocks per SM; a few spills): faster
 // than the unbounded 111-register build by 4-6 % on whole-bundle loops
-__global__ void __launch_bounds__(kMaxBlock, 4) k_shade_loop(DevScene s, DevConfig c, Film f, WaveBuffers w, WaveLoop *L,
+__global__ void __launch_bounds__(kMaxBlock, 4) k_shade_loop(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, Film f, WaveBuffers w, WaveLoop *L,
                                                           uint32_t *err) {
   const int a = L->iter & 1;
   const int n = L->ext[a];
@@ -555,16 +743,16 @@ __global__ void k_loop_control(WaveLoop *L, cudaGraphConditionalHandle h, int in
 
 cudaError_t launch_wave_chunk(const DevScene &s, const DevConfig &c, uint32_t pass, int band, Film f,
                               const WaveBuffers &w, uint32_t *err, int grid, int block, int sort_keys,
-                              cudaStream_t st, int trace_budget, int p0, int n);
+                              cudaStream_t st, int p0, int n);
 
 cudaError_t launch_wave_pass(const DevScene &s, const DevConfig &c, uint32_t pass, int band, Film f,
                              const WaveBuffers &w, uint32_t *err, int grid, int block, int sort_keys,
-                             cudaStream_t st, int trace_budget, int capacity) {
+                             cudaStream_t st, int capacity) {
   // the frame in chunks of at most `capacity` paths (their queues stay in L2)
   const int npix = c.W * c.H;
   const int chunk = capacity > 0 && capacity < npix ? capacity : npix;
   for (int p0 = 0; p0 < npix; p0 += chunk) {
-    const cudaError_t e = launch_wave_chunk(s, c, pass, band, f, w, err, grid, block, sort_keys, st, trace_budget, p0,
+    const cudaError_t e = launch_wave_chunk(s, c, pass, band, f, w, err, grid, block, sort_keys, st, p0,
                                             npix - p0 < chunk ? npix - p0 : chunk);
     if (e != cudaSuccess) return e;
   }
@@ -573,7 +761,7 @@ cudaError_t launch_wave_pass(const DevScene &s, const DevConfig &c, uint32_t pas
 
 cudaError_t launch_wave_chunk(const DevScene &s, const DevConfig &c, uint32_t pass, int band, Film f,
                               const WaveBuffers &w, uint32_t *err, int grid, int block, int sort_keys,
-                              cudaStream_t st, int trace_budget, int p0, int n) {
+                              cudaStream_t st, int p0, int n) {
   if (c.max_depth > kMaxDepth) return cudaErrorInvalidValue;
   cudaError_t e = cudaMemsetAsync(w.counts, 0, kCntTotal * sizeof(int), st);
   if (e != cudaSuccess) return e;
@@ -593,7 +781,7 @@ cudaError_t launch_wave_chunk(const DevScene &s, const DevConfig &c, uint32_t pa
     const int sh_sorted = (sort_keys & 4) && d > 0 ? 1 : 0;
     if (ext_sorted) launch_sort(s, d, w, kSortExt, kExtKeys, w.trace_order, sort_grid, st);
     if (sh_sorted) launch_sort(s, d - 1, w, kSortShadow, kShadowKeys, w.shadow_order, sort_grid, st);
-    launch_trace(s, c, d, f, w, err, grid, block, st, trace_budget, ext_sorted, sh_sorted);
+    launch_trace(s, c, d, f, w, err, grid, block, st, n, ext_sorted, sh_sorted);
     if (sort_keys & 1) launch_sort(s, d, w, kSortShade, nmat, w.sorted, sort_grid, st);
     k_shade<<<grid, block, 0, st>>>(s, c, pass, band, d, f, w, (sort_keys & 1) ? 1 : 0, err);
   }
@@ -601,7 +789,7 @@ cudaError_t launch_wave_chunk(const DevScene &s, const DevConfig &c, uint32_t pa
   if (c.max_depth > 0) {
     const int sh_sorted = (sort_keys & 4) ? 1 : 0;
     if (sh_sorted) launch_sort(s, c.max_depth - 1, w, kSortShadow, kShadowKeys, w.shadow_order, sort_grid, st);
-    launch_trace(s, c, c.max_depth, f, w, err, grid, block, st, trace_budget, 0, sh_sorted);
+    launch_trace(s, c, c.max_depth, f, w, err, grid, block, st, n, 0, sh_sorted);
   }
   return cudaGetLastError();
 }
@@ -624,7 +812,7 @@ void free_wave_loop(WaveLoopGraph *g) {
 namespace {
 
 cudaError_t build_wave_loop(WaveLoopGraph &G, const DevScene &s, const DevConfig &c, Film f, const WaveBuffers &w,
-                            uint32_t *err, int grid, int block, int budget) {
+                            uint32_t *err, int grid, int block, int paths) {
   if (G.exec) cudaGraphExecDestroy(G.exec);
   if (G.graph) cudaGraphDestroy(G.graph);
   G.exec = nullptr;
@@ -645,7 +833,7 @@ cudaError_t build_wave_loop(WaveLoopGraph &G, const DevScene &s, const DevConfig
   if ((e = cudaStreamBeginCaptureToGraph(G.capture, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
       cudaSuccess)
     return e;
-  launch_trace<true>(s, c, 0, f, w, err, grid, block, G.capture, budget, 0, 0, w.loop);
+  launch_trace<true>(s, c, 0, f, w, err, grid, block, G.capture, paths, 0, 0, w.loop);
   k_shade_loop<<<grid, block, 0, G.capture>>>(s, c, f, w, w.loop, err);
   k_loop_control<<<1, 32, 0, G.capture>>>(w.loop, h, 1, err);
   const cudaError_t le = cudaGetLastError();
@@ -659,8 +847,7 @@ cudaError_t build_wave_loop(WaveLoopGraph &G, const DevScene &s, const DevConfig
 }  // namespace
 
 cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pass0, int band0, int npass, Film f,
-                             const WaveBuffers &w, uint32_t *err, int grid, int block, cudaStream_t st,
-                             int trace_budget, int capacity, WaveLoopGraph **graph, bool host_driven,
+                             const WaveBuffers &w, uint32_t *err, int grid, int block, cudaStream_t st, int capacity, WaveLoopGraph **graph, bool host_driven,
                              int limit_override) {
   const int64_t npix = (int64_t)c.W * c.H;
   const int64_t total = npix * npass;
@@ -681,7 +868,7 @@ cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pas
     Film f;
     WaveBuffers w;
     uint32_t *err;
-    int grid, block, budget;
+    int grid, block, paths;
   } k;
   memset(&k, 0, sizeof k);
   memcpy(&k.s, &s, sizeof s);
@@ -696,13 +883,13 @@ cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pas
   k.err = err;
   k.grid = grid;
   k.block = block;
-  k.budget = trace_budget;
+  k.paths = n0;
   const unsigned char *kb = reinterpret_cast<const unsigned char *>(&k);
   if (host_driven) {
     const int init_grid = (int)((n0 + 255) / 256 < 4096 ? (n0 + 255) / 256 : 4096);
     k_loop_init<<<init_grid, 256, 0, st>>>(s, c, w, w.loop, pass0, band0, npass, n0, limit, shared);
     for (int it = 0; it < limit; ++it) {
-      launch_trace<true>(s, c, 0, f, w, err, grid, block, st, trace_budget, 0, 0, w.loop);
+      launch_trace<true>(s, c, 0, f, w, err, grid, block, st, n0, 0, 0, w.loop);
       k_shade_loop<<<grid, block, 0, st>>>(s, c, f, w, w.loop, err);
       k_loop_control<<<1, 32, 0, st>>>(w.loop, 0, 0, err);
       int go = 0;
@@ -717,7 +904,7 @@ cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pas
   WaveLoopGraph &G = **graph;
   if (!G.exec || G.key.size() != sizeof k || memcmp(G.key.data(), kb, sizeof k) != 0) {
     G.key.clear();
-    const cudaError_t e = build_wave_loop(G, s, c, f, w, err, grid, block, trace_budget);
+    const cudaError_t e = build_wave_loop(G, s, c, f, w, err, grid, block, n0);
     if (e != cudaSuccess) return e;
     G.key.assign(kb, kb + sizeof k);
   }
@@ -793,82 +980,26 @@ __global__ void k_bloop_init(const BatchSlot *__restrict__ slots, int n, const B
   }
 }
 
-// trace stage of the batch loop: k_trace<W, true> with each item's view
+// trace stage of the batch loop: k_trace with each item's view
+struct BatchScenes {
+  const BatchSlot *__restrict__ slots;
+  __device__ __forceinline__ int view_of_query(const WaveBuffers &w, int qi) const { return w.sq_view[qi]; }
+  __device__ __forceinline__ int view_of_path(const WaveBuffers &w, int pid) const { return w.view[pid]; }
+  __device__ __forceinline__ const DevScene &scene(int v) const { return slots[v].s; }
+  __device__ __forceinline__ const DevConfig &config(int v) const { return slots[v].c; }
+  __device__ __forceinline__ const Film &film(int v) const { return slots[v].f; }
+  __device__ __forceinline__ bool shared(int v) const { return slot_shared(slots[v]); }
+};
+
 template <int W>
-__global__ void __launch_bounds__(kMaxBlock, 4) k_trace_bloop(const BatchSlot *__restrict__ slots, WaveBuffers w,
-                                                           uint32_t *__restrict__ err, int budget, WaveLoop *L) {
+__global__ void __launch_bounds__(kMaxBlock, 4) k_trace_bloop(const BatchSlot *__restrict__ slots,
+                                                           const __grid_constant__ WaveBuffers w,
+                                                           uint32_t *__restrict__ err, WaveLoop *L) {
   uint32_t eb = 0;
   const int a = L->iter & 1;
   const int nsh = L->sh[a ^ 1];
-  const int next = L->ext[a];
-  const int *q = w.queue[a];
-  int *fetch = L->fetch + 0;
-  const int total = nsh + next;
-  const int lane = threadIdx.x & 31;
-  int item = -1, pid = 0, pixel = 0, band = 0, dep_band = 0, v = 0;
-  bool exhausted = false;
-  Traversal t;
-  int2 stack[StackSize<W>::value];
-  ShadowQuery sq;
-  ShadowState ss;
-  for (;;) {
-    const bool need = item < 0 && !exhausted;
-    const unsigned m = __ballot_sync(0xffffffffu, need);
-    if (m) {
-      const int leader = __ffs(m) - 1;
-      int base = 0;
-      if (lane == leader) base = atomicAdd(fetch, __popc(m));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (need) {
-        const int idx = base + __popc(m & ((1u << lane) - 1u));
-        if (idx >= total) {
-          exhausted = true;
-        } else if (idx < nsh) {
-          item = idx;
-          v = w.sq_view[idx];
-          const BatchSlot &sl = slots[v];
-          const float4 o = w.sq_origin[idx], d = w.sq_dir[idx];
-          const int4 mm = w.sq_meta[idx];
-          sq.origin = xyz(o);
-          sq.max_dist = o.w;
-          sq.dir = xyz(d);
-          sq.contrib = d.w;
-          sq.light_slot = mm.y;
-          sq.vol = mm.z;
-          pixel = mm.x;
-          band = mm.w & 0xff;
-          dep_band = mm.w >> 8;
-          ss.pos = sq.origin;
-          ss.total = 1.f;
-          ss.traveled = 0.f;
-          ss.vol = sq.vol;
-          ss.seg = 0;
-          trav_begin(sl.s, t, ss.pos, sq.dir, shadow_bound(sl.s, sl.c, sq, ss, band));
-        } else {
-          item = idx;
-          pid = q[idx - nsh];
-          v = w.view[pid];
-          const float4 pt = w.pos_thr[pid], ds = w.dir_spdf[pid];
-          trav_begin(slots[v].s, t, xyz(pt), xyz(ds), slots[v].c.escape);
-        }
-      }
-    }
-    if (__ballot_sync(0xffffffffu, item >= 0) == 0) break;
-    const BatchSlot &sl = slots[v];
-    if (item >= 0 && trav_advance<W>(sl.s, t, stack, sl.c.eps, budget, eb)) {
-      if (item < nsh) {
-        if (shadow_segment(sl.s, sl.c, sq, t.h, band, ss)) {
-          if (ss.total > 1e-6f) deposit(sl.f, pixel, dep_band, sq.contrib * ss.total, slot_shared(sl));
-          item = -1;
-        } else {
-          trav_begin(sl.s, t, ss.pos, sq.dir, shadow_bound(sl.s, sl.c, sq, ss, band));
-        }
-      } else {
-        w.hit[pid] = make_float4(t.h.t, t.h.u, t.h.v, __int_as_float(t.h.slot));
-        item = -1;
-      }
-    }
-  }
+  const TraceItems it{nsh, nsh + L->ext[a], w.queue[a], nullptr, L->fetch + 0};
+  trace_lanes<W>(BatchScenes{slots}, w, it, eb);
   if (eb) atomicOr(err, eb);
 }
 
@@ -934,20 +1065,18 @@ void free_batch_loop(BatchLoopGraph *g) {
 namespace {
 
 cudaError_t launch_trace_bloop(const BatchSlot *slots, const WaveBuffers &w, uint32_t *err, int width, int grid,
-                               int block, int budget, cudaStream_t st) {
-  if (width == 9) k_trace_bloop<9><<<grid, block, 0, st>>>(slots, w, err, budget, w.loop);
-  else if (width == 5) k_trace_bloop<5><<<grid, block, 0, st>>>(slots, w, err, budget, w.loop);
-  else if (width == 8) k_trace_bloop<8><<<grid, block, 0, st>>>(slots, w, err, budget, w.loop);
-  else if (width == 4) k_trace_bloop<4><<<grid, block, 0, st>>>(slots, w, err, budget, w.loop);
-  else if (width == 3) k_trace_bloop<3><<<grid, block, 0, st>>>(slots, w, err, budget, w.loop);
-  else k_trace_bloop<2><<<grid, block, 0, st>>>(slots, w, err, budget, w.loop);
+                               int block, cudaStream_t st) {
+  if (width == 9) k_trace_bloop<9><<<grid, block, 0, st>>>(slots, w, err, w.loop);
+  else if (width == 5) k_trace_bloop<5><<<grid, block, 0, st>>>(slots, w, err, w.loop);
+  else if (width == 8) k_trace_bloop<8><<<grid, block, 0, st>>>(slots, w, err, w.loop);
+  else if (width == 4) k_trace_bloop<4><<<grid, block, 0, st>>>(slots, w, err, w.loop);
+  else k_trace_bloop<2><<<grid, block, 0, st>>>(slots, w, err, w.loop);
   return cudaGetLastError();
 }
 
 // the loop body: one iteration (trace, shade, control)
-cudaError_t bloop_body(BatchSlot *slots, int n, const WaveBuffers &w, uint32_t *err, int width, int grid, int block,
-                       int budget, cudaGraphConditionalHandle h, int in_graph, cudaStream_t st) {
-  cudaError_t e = launch_trace_bloop(slots, w, err, width, grid, block, budget, st);
+cudaError_t bloop_body(BatchSlot *slots, int n, const WaveBuffers &w, uint32_t *err, int width, int grid, int block, cudaGraphConditionalHandle h, int in_graph, cudaStream_t st) {
+  cudaError_t e = launch_trace_bloop(slots, w, err, width, grid, block, st);
   if (e != cudaSuccess) return e;
   k_shade_bloop<<<grid, block, 0, st>>>(slots, n, w, w.loop, err);
   k_loop_control<<<1, 32, 0, st>>>(w.loop, h, in_graph, err);
@@ -965,7 +1094,7 @@ cudaError_t bloop_head(BatchSlot *slots, int n, BatchHeader *h, const int *activ
 
 // the whole step as one graph: head -> while(loop body) -> finish
 cudaError_t build_bloop_graph(BatchLoopGraph &G, BatchSlot *slots, int n, BatchHeader *h, const int *active,
-                              uint32_t *err, const WaveBuffers &w, int width, int grid, int block, int budget,
+                              uint32_t *err, const WaveBuffers &w, int width, int grid, int block,
                               int capacity, int limit, int acc_blocks) {
   cudaError_t e;
   if (!G.capture && (e = cudaStreamCreateWithFlags(&G.capture, cudaStreamNonBlocking)) != cudaSuccess) return e;
@@ -998,7 +1127,7 @@ cudaError_t build_bloop_graph(BatchLoopGraph &G, BatchSlot *slots, int n, BatchH
   if ((e = cudaStreamBeginCaptureToGraph(G.capture, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                          cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
     return e;
-  le = bloop_body(slots, n, w, err, width, grid, block, budget, cond, 1, G.capture);
+  le = bloop_body(slots, n, w, err, width, grid, block, cond, 1, G.capture);
   cudaGraph_t body = nullptr;
   e = cudaStreamEndCapture(G.capture, &body);
   if (le != cudaSuccess) return le;
@@ -1017,7 +1146,7 @@ cudaError_t build_bloop_graph(BatchLoopGraph &G, BatchSlot *slots, int n, BatchH
 }  // namespace
 
 cudaError_t launch_batch_loop_step(BatchSlot *slots, int n, BatchHeader *h, const int *active, uint32_t *err,
-                                   const WaveBuffers &w, int width, int grid, int block, int budget, int capacity,
+                                   const WaveBuffers &w, int width, int grid, int block, int capacity,
                                    int limit, int acc_blocks, cudaStream_t st, BatchLoopGraph **graph,
                                    bool use_graph) {
   if (capacity < 1 || capacity > w.capacity || !w.view || !w.sq_view || !w.tag || !w.loop || limit < 1)
@@ -1032,7 +1161,7 @@ cudaError_t launch_batch_loop_step(BatchSlot *slots, int n, BatchHeader *h, cons
       if (e == cudaSuccess) e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) return e;
       if (!go) break;
-      e = bloop_body(slots, n, w, err, width, grid, block, budget, 0, 0, st);
+      e = bloop_body(slots, n, w, err, width, grid, block, 0, 0, st);
       if (e != cudaSuccess) return e;
     }
     return launch_batch_finish(slots, n, acc_blocks, st);
@@ -1041,7 +1170,7 @@ cudaError_t launch_batch_loop_step(BatchSlot *slots, int n, BatchHeader *h, cons
   BatchLoopGraph &G = **graph;
   if (!G.exec) {
     const cudaError_t e =
-        build_bloop_graph(G, slots, n, h, active, err, w, width, grid, block, budget, capacity, limit, acc_blocks);
+        build_bloop_graph(G, slots, n, h, active, err, w, width, grid, block, capacity, limit, acc_blocks);
     if (e != cudaSuccess) {
       if (G.graph) cudaGraphDestroy(G.graph);
       G.graph = nullptr;
@@ -1084,7 +1213,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch
 
 // camera rays for the pixels of one tile; path slot s <-> pixel
 // (x0 + s % tw, y0 + s / tw) of the full frame (pixel ids key the random streams)
-__global__ void k_generate_tile(DevScene s, DevConfig c, uint32_t pass, int band, WaveBuffers w, int x0, int y0,
+__global__ void k_generate_tile(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass, int band, WaveBuffers w, int x0, int y0,
                                 int tw, int th) {
   const int n = tw * th;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
@@ -1155,7 +1284,7 @@ cudaError_t noalloc_setup(int device, void **ptr) {
 
 cudaError_t launch_wave_tile_noalloc(const DevScene &s, const DevConfig &c, uint32_t pass, int band, Film f,
                                      void *scratch, int x0, int y0, int tw, int th, uint32_t *err, int grid,
-                                     int block, cudaStream_t st, int trace_budget) {
+                                     int block, cudaStream_t st) {
   if (c.max_depth > kMaxDepth) return cudaErrorInvalidValue;
   unsigned char *b = static_cast<unsigned char *>(scratch);
   WaveBuffers w{};
@@ -1180,10 +1309,10 @@ cudaError_t launch_wave_tile_noalloc(const DevScene &s, const DevConfig &c, uint
   const int n = tw * th;
   k_generate_tile<<<(n + 255) / 256, 256, 0, st>>>(s, c, pass, band, w, x0, y0, tw, th);
   for (int d = 0; d < c.max_depth; ++d) {
-    launch_trace(s, c, d, f, w, err, grid, block, st, trace_budget);
+    launch_trace(s, c, d, f, w, err, grid, block, st, n);
     k_shade<<<grid, block, 0, st>>>(s, c, pass, band, d, f, w, 0, err);
   }
-  if (c.max_depth > 0) launch_trace(s, c, c.max_depth, f, w, err, grid, block, st, trace_budget);
+  if (c.max_depth > 0) launch_trace(s, c, c.max_depth, f, w, err, grid, block, st, n);
   return cudaGetLastError();
 }
 

@@ -8,7 +8,7 @@
 // operation (no FMA contraction) so that distances are bit-identical to the
 // CPU oracle's.
 //
-// trace_closest() is the fast path: two-child 64-byte nodes, nearest child
+// trace_closest() is the fast path: wide nodes, nearest child
 // first, and boxes whose entry distance lies beyond the current best hit (by
 // a relative margin of 2^-16, far larger than the rounding error of the box
 // and triangle distances) are skipped.  The reference never skips boxes, so
@@ -67,188 +67,89 @@ struct TraceCount {
   uint32_t nodes = 0, tris = 0;
 };
 
-// Resumable fast traversal.  The state lives in registers; the stack of
-// (node, entry-distance bits) pairs is owned by the caller so that a lane can
-// stop after a budget of steps and resume later (the persistent trace kernel
-// refills idle lanes between budgets).
 constexpr int kTravDone = -2147483647 - 1;  // never a leaf code: first slot < 2^27 - 1
 
+// ------------------------------------------------------------ packed pairs
+// Two float32 lanes in one register pair.  sm_100's packed add and multiply
+// round each lane like the scalar instruction and take one issue slot.
+typedef unsigned long long f32x2;
+TS_D f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+TS_D void unpack2(f32x2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+TS_D f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+TS_D f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+TS_D float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+TS_D float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// A 32-byte record in one load.  A scattered load costs L1 one pass per sector
+// and lane, so two 16-byte halves cost it twice.
+struct Rec32 {
+  f32x2 a, b, c, d;
+};
+TS_D Rec32 load32(const void *p) {
+  Rec32 r;
+  asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(r.a), "=l"(r.b), "=l"(r.c), "=l"(r.d) : "l"(p));
+  return r;
+}
+
+// State of a traversal, in registers; the stack of (node, entry-distance bits)
+// pairs is owned by the caller, so that a lane can stop between steps.
 struct Traversal {
-  float3 o, d, inv;
+  f32x2 no[3], inv[3];  // per axis the negated origin and the reciprocal direction, in both lanes of a pair
+  float3 d;
   float tcull;
   Hit h;
   int node, sp;
+  int tie;              // another triangle lies at exactly h.t
 };
 
-// bound: distance beyond which hits do not matter to the caller.  Boxes past
-// it are skipped; a hit beyond it may still be returned (callers treat such a
-// hit like a miss), so results are the same as with bound = 1e9.
-TS_D void trav_begin(const DevScene &s, Traversal &t, float3 o, float3 d, float bound) {
-  t.o = o;
-  t.d = d;
-  t.inv = f3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
-  t.h.t = 1e9f;
-  t.h.u = t.h.v = 0.f;
-  t.h.slot = -1;
-  t.tcull = cull_bound(fminf(bound, 1e9f));
-  t.node = s.num_nodes > 0 ? 0 : kTravDone;
-  t.sp = 0;
-}
-
-// Advance by at most `budget` steps (one inner node, or one leaf and the pop
-// that follows).  Returns true once the traversal has finished.
-template <bool kCount = false>
-TS_D bool trav_steps(const DevScene &s, Traversal &t, int2 *stack, float eps, int budget, uint32_t &errbits,
-                     TraceCount *tc = nullptr) {
-  for (int it = 0; it < budget; ++it) {
-    if (t.node == kTravDone) return true;
-    if (t.node >= 0) {
-      const float4 *n = s.node + 4 * (size_t)t.node;
-      if (kCount) tc->nodes++;
-      const float4 a = __ldg(n + 0), b = __ldg(n + 1), c = __ldg(n + 2);
-      const int4 l = __ldg(reinterpret_cast<const int4 *>(n) + 3);
-      float e0, x0, e1, x1;
-      box_hit(a.x, a.y, a.z, a.w, c.x, c.y, t.o, t.inv, e0, x0);
-      box_hit(b.x, b.y, b.z, b.w, c.z, c.w, t.o, t.inv, e1, x1);
-      const bool h0 = e0 < x0 && x0 > 0.f && e0 <= t.tcull;
-      const bool h1 = e1 < x1 && x1 > 0.f && e1 <= t.tcull;
-      if (h0 && h1) {
-        int nr = l.x, fr = l.y;
-        float fe = e1;
-        if (e1 < e0) { nr = l.y; fr = l.x; fe = e0; }
-        if (t.sp < kStackDepth) {
-          stack[t.sp++] = make_int2(fr, __float_as_int(fe));
-        } else {
-          errbits |= kErrStackOverflow;
-        }
-        t.node = nr;
-        continue;
-      }
-      if (h0) { t.node = l.x; continue; }
-      if (h1) { t.node = l.y; continue; }
+// one triangle against the ray; keeps the first of equal distances
+TS_D void trav_triangle(const DevScene &s, Traversal &t, float3 o, int slot, float eps) {
+  const float4 *tp = s.tri + 3 * (size_t)slot;
+  const float4 A = __ldg(tp + 0), E1 = __ldg(tp + 1), E2 = __ldg(tp + 2);
+  float u, v;
+  const float tt = tri_hit(o, t.d, A, E1, E2, eps, u, v);
+  if (tt > eps && tt <= t.h.t) {
+    if (tt == t.h.t) {
+      t.tie = 1;
     } else {
-      const int code = ~t.node;
-      const int first = code >> 4;
-      const int cnt = (code & 15) + 1;
-      if (kCount) tc->tris += cnt;
-      for (int i = 0; i < cnt; ++i) {
-        const float4 *tp = s.tri + 3 * (size_t)(first + i);
-        const float4 A = __ldg(tp + 0), E1 = __ldg(tp + 1), E2 = __ldg(tp + 2);
-        float u, v;
-        const float tt = tri_hit(t.o, t.d, A, E1, E2, eps, u, v);
-        if (tt > eps && tt < t.h.t) {
-          t.h.t = tt;
-          t.h.u = u;
-          t.h.v = v;
-          t.h.slot = first + i;
-          t.tcull = fminf(t.tcull, cull_bound(tt));
-        }
-      }
-    }
-    // pop the next box that is still closer than the cull bound
-    for (;;) {
-      if (t.sp == 0) {
-        t.node = kTravDone;
-        return true;
-      }
-      const int2 e = stack[--t.sp];
-      if (__int_as_float(e.y) <= t.tcull) {
-        t.node = e.x;
-        break;
-      }
+      t.h.t = tt;
+      t.h.u = u;
+      t.h.v = v;
+      t.h.slot = slot;
+      t.tcull = fminf(t.tcull, cull_bound(tt));
+      t.tie = 0;
     }
   }
-  return t.node == kTravDone;
 }
 
-// Speculative while-while traversal of the two-child layout (Aila & Laine,
-// "Understanding the efficiency of ray traversal on GPUs", HPG 2009): a lane
-// that reaches a leaf postpones it and keeps descending, and the warp tests
-// leaves only once every active lane holds one (or has finished), so leaf
-// tests and inner-node steps are not interleaved across the warp.  Same
-// results as trav_steps.
-template <bool kCount = false>
-TS_D bool trav_steps_spec(const DevScene &s, Traversal &t, int2 *stack, float eps, int budget, uint32_t &errbits,
-                          TraceCount *tc = nullptr) {
-  int leaf = 0;  // postponed leaf code (< 0), or 0
-  for (int it = 0; it < budget; ++it) {
-    if (t.node == kTravDone && leaf == 0) return true;
-    // ---- inner nodes
-    while (t.node >= 0) {
-      const float4 *n = s.node + 4 * (size_t)t.node;
-      if (kCount) tc->nodes++;
-      const float4 a = __ldg(n + 0), b = __ldg(n + 1), c = __ldg(n + 2);
-      const int4 l = __ldg(reinterpret_cast<const int4 *>(n) + 3);
-      float e0, x0, e1, x1;
-      box_hit(a.x, a.y, a.z, a.w, c.x, c.y, t.o, t.inv, e0, x0);
-      box_hit(b.x, b.y, b.z, b.w, c.z, c.w, t.o, t.inv, e1, x1);
-      const bool h0 = e0 < x0 && x0 > 0.f && e0 <= t.tcull;
-      const bool h1 = e1 < x1 && x1 > 0.f && e1 <= t.tcull;
-      if (h0 && h1) {
-        int nr = l.x, fr = l.y;
-        float fe = e1;
-        if (e1 < e0) { nr = l.y; fr = l.x; fe = e0; }
-        if (t.sp < kStackDepth) stack[t.sp++] = make_int2(fr, __float_as_int(fe));
-        else errbits |= kErrStackOverflow;
-        t.node = nr;
-      } else if (h0) {
-        t.node = l.x;
-      } else if (h1) {
-        t.node = l.y;
-      } else {
-        t.node = kTravDone;
-        while (t.sp > 0) {
-          const int2 e = stack[--t.sp];
-          if (__int_as_float(e.y) <= t.tcull) { t.node = e.x; break; }
-        }
-      }
-      // postpone the first leaf found and keep descending from the stack
-      if (t.node < 0 && t.node != kTravDone && leaf == 0) {
-        leaf = t.node;
-        t.node = kTravDone;
-        while (t.sp > 0) {
-          const int2 e = stack[--t.sp];
-          if (__int_as_float(e.y) <= t.tcull) { t.node = e.x; break; }
-        }
-      }
-      if (!__any_sync(__activemask(), leaf == 0)) break;
-    }
-    // ---- leaves
-    for (;;) {
-      int code = 0;
-      if (leaf < 0) {
-        code = ~leaf;
-        leaf = 0;
-      } else if (t.node < 0 && t.node != kTravDone) {
-        code = ~t.node;
-        t.node = kTravDone;
-        while (t.sp > 0) {
-          const int2 e = stack[--t.sp];
-          if (__int_as_float(e.y) <= t.tcull) { t.node = e.x; break; }
-        }
-      } else {
-        break;
-      }
-      const int first = code >> 4;
-      const int cnt = (code & 15) + 1;
-      if (kCount) tc->tris += cnt;
-      for (int i = 0; i < cnt; ++i) {
-        const float4 *tp = s.tri + 3 * (size_t)(first + i);
-        const float4 A = __ldg(tp + 0), E1 = __ldg(tp + 1), E2 = __ldg(tp + 2);
-        float u, v;
-        const float tt = tri_hit(t.o, t.d, A, E1, E2, eps, u, v);
-        if (tt > eps && tt < t.h.t) {
-          t.h.t = tt;
-          t.h.u = u;
-          t.h.v = v;
-          t.h.slot = first + i;
-          t.tcull = fminf(t.tcull, cull_bound(tt));
-        }
-      }
-    }
-    if (t.node == kTravDone && leaf == 0) return true;
-  }
-  return t.node == kTravDone && leaf == 0;
+TS_D float lane0(f32x2 v) {
+  float a, b;
+  unpack2(v, a, b);
+  return a;
+}
+
+TS_D float3 trav_origin(const Traversal &t) {
+  return f3(-lane0(t.no[0]), -lane0(t.no[1]), -lane0(t.no[2]));
 }
 
 // ---- wide nodes (4 or 8 children) ---------------------------------------
@@ -280,230 +181,15 @@ TS_D void sort_children(float *k, int *r) {
   }
 }
 
-// Traversal stacks of (node, entry-distance bits): a plain per-lane array
-// (local memory, kept in L1), or a short stack whose newest S entries of each
-// lane sit in a shared-memory column laid out [entry][thread] -- consecutive
-// threads, consecutive 8-byte words, so a warp touches no bank twice at any
-// mix of depths -- with older entries spilled to the lane's local array.
-TS_D void spush(int2 *st, Traversal &t, int2 e) { st[t.sp++] = e; }
-TS_D int2 spop(int2 *st, Traversal &t) { return st[--t.sp]; }
-
-template <int S>
-struct ShortStack {
-  static_assert((S & (S - 1)) == 0, "ring size must be a power of two");
-  int2 *sm;    // shared: [S][stride] entries
-  int2 *loc;   // local: entries by absolute position (the older ones)
-  int stride;  // threads per block
-  int lane;    // this thread's column
-  int ins;     // top entries held in shared memory (0 after trav_begin)
-};
-template <int S>
-TS_D void spush(ShortStack<S> &st, Traversal &t, int2 e) {
-  const int pos = t.sp;
-  if (st.ins > pos) st.ins = pos;  // a new traversal (trav_begin) emptied the stack
-  if (st.ins == S) {  // ring full: the oldest shared entry moves to local memory
-    const int old = pos - S;
-    st.loc[old] = st.sm[(old & (S - 1)) * st.stride + st.lane];
-    --st.ins;
-  }
-  st.sm[(pos & (S - 1)) * st.stride + st.lane] = e;
-  ++st.ins;
-  ++t.sp;
-}
-template <int S>
-TS_D int2 spop(ShortStack<S> &st, Traversal &t) {
-  const int pos = --t.sp;
-  if (st.ins > 0) {
-    --st.ins;
-    return st.sm[(pos & (S - 1)) * st.stride + st.lane];
-  }
-  return st.loc[pos];
-}
-
-// Same contract as trav_steps, for the wide layout: the children a node's
-// ray enters are sorted by entry distance; the nearest is visited next and
-// the others are pushed (farthest first) with their entry distances.
-template <int W, bool kCount = false, class Stk = int2 *>
-TS_D bool trav_steps_wide(const DevScene &s, Traversal &t, Stk &stack, float eps, int budget, uint32_t &errbits,
-                          TraceCount *tc = nullptr) {
-  constexpr int P = W / 4;  // float4s per row
-  for (int it = 0; it < budget; ++it) {
-    if (t.node == kTravDone) return true;
-    if (t.node >= 0) {
-      const float4 *n = s.node + (size_t)(6 * P + P + (W == 4 ? 1 : 2)) * t.node;
-      if (kCount) tc->nodes++;
-      float row[6][W];
-#pragma unroll
-      for (int r = 0; r < 6; ++r)
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-          const float4 v = __ldg(n + r * P + q);
-          row[r][4 * q + 0] = v.x; row[r][4 * q + 1] = v.y; row[r][4 * q + 2] = v.z; row[r][4 * q + 3] = v.w;
-        }
-      int ref[W];
-#pragma unroll
-      for (int q = 0; q < P; ++q) {
-        const int4 l = __ldg(reinterpret_cast<const int4 *>(n + 6 * P + q));
-        ref[4 * q + 0] = l.x; ref[4 * q + 1] = l.y; ref[4 * q + 2] = l.z; ref[4 * q + 3] = l.w;
-      }
-      float key[W];
-      int nh = 0;
-#pragma unroll
-      for (int k = 0; k < W; ++k) {
-        float te, tx;
-        box_hit(row[0][k], row[1][k], row[2][k], row[3][k], row[4][k], row[5][k], t.o, t.inv, te, tx);
-        const bool h = te < tx && tx > 0.f && te <= t.tcull;
-        key[k] = h ? te : INFINITY;
-        nh += h;
-      }
-      if (nh > 0) {
-        sort_children<W>(key, ref);
-        if (t.sp + nh - 1 <= kWideStack) {
-#pragma unroll
-          for (int k = W - 1; k >= 1; --k)
-            if (k < nh) spush(stack, t, make_int2(ref[k], __float_as_int(key[k])));
-        } else {
-          errbits |= kErrStackOverflow;
-        }
-        t.node = ref[0];
-        continue;
-      }
-    } else {
-      const int code = ~t.node;
-      const int first = code >> 4;
-      const int cnt = (code & 15) + 1;
-      if (kCount) tc->tris += cnt;
-      for (int i = 0; i < cnt; ++i) {
-        const float4 *tp = s.tri + 3 * (size_t)(first + i);
-        const float4 A = __ldg(tp + 0), E1 = __ldg(tp + 1), E2 = __ldg(tp + 2);
-        float u, v;
-        const float tt = tri_hit(t.o, t.d, A, E1, E2, eps, u, v);
-        if (tt > eps && tt < t.h.t) {
-          t.h.t = tt;
-          t.h.u = u;
-          t.h.v = v;
-          t.h.slot = first + i;
-          t.tcull = fminf(t.tcull, cull_bound(tt));
-        }
-      }
-    }
-    for (;;) {
-      if (t.sp == 0) {
-        t.node = kTravDone;
-        return true;
-      }
-      const int2 e = spop(stack, t);
-      if (__int_as_float(e.y) <= t.tcull) {
-        t.node = e.x;
-        break;
-      }
-    }
-  }
-  return t.node == kTravDone;
-}
-
-// Speculative while-while traversal of the wide layout (Aila & Laine, HPG
-// 2009, as trav_steps_spec does for two-child nodes): a lane that reaches a
-// leaf postpones it and keeps descending; the warp tests leaves only once
-// every active lane holds one (or has finished).  Same results as
-// trav_steps_wide.
-template <int W, bool kCount = false>
-TS_D bool trav_steps_wide_spec(const DevScene &s, Traversal &t, int2 *stack, float eps, int budget,
-                               uint32_t &errbits, TraceCount *tc = nullptr) {
-  constexpr int P = W / 4;  // float4s per row
-  int leaf = 0;             // postponed leaf code (< 0), or 0
-  auto pop = [&]() {
-    t.node = kTravDone;
-    while (t.sp > 0) {
-      const int2 e = stack[--t.sp];
-      if (__int_as_float(e.y) <= t.tcull) {
-        t.node = e.x;
-        break;
-      }
-    }
-  };
-  for (int it = 0; it < budget; ++it) {
-    if (t.node == kTravDone && leaf == 0) return true;
-    // ---- inner nodes
-    while (t.node >= 0) {
-      const float4 *n = s.node + (size_t)(6 * P + P + (W == 4 ? 1 : 2)) * t.node;
-      if (kCount) tc->nodes++;
-      float row[6][W];
-#pragma unroll
-      for (int r = 0; r < 6; ++r)
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-          const float4 v = __ldg(n + r * P + q);
-          row[r][4 * q + 0] = v.x; row[r][4 * q + 1] = v.y; row[r][4 * q + 2] = v.z; row[r][4 * q + 3] = v.w;
-        }
-      int ref[W];
-#pragma unroll
-      for (int q = 0; q < P; ++q) {
-        const int4 l = __ldg(reinterpret_cast<const int4 *>(n + 6 * P + q));
-        ref[4 * q + 0] = l.x; ref[4 * q + 1] = l.y; ref[4 * q + 2] = l.z; ref[4 * q + 3] = l.w;
-      }
-      float key[W];
-      int nh = 0;
-#pragma unroll
-      for (int k = 0; k < W; ++k) {
-        float te, tx;
-        box_hit(row[0][k], row[1][k], row[2][k], row[3][k], row[4][k], row[5][k], t.o, t.inv, te, tx);
-        const bool h = te < tx && tx > 0.f && te <= t.tcull;
-        key[k] = h ? te : INFINITY;
-        nh += h;
-      }
-      if (nh > 0) {
-        sort_children<W>(key, ref);
-        if (t.sp + nh - 1 <= kWideStack) {
-#pragma unroll
-          for (int k = W - 1; k >= 1; --k)
-            if (k < nh) stack[t.sp++] = make_int2(ref[k], __float_as_int(key[k]));
-        } else {
-          errbits |= kErrStackOverflow;
-        }
-        t.node = ref[0];
-      } else {
-        pop();
-      }
-      // postpone the first leaf found and keep descending from the stack
-      if (t.node < 0 && t.node != kTravDone && leaf == 0) {
-        leaf = t.node;
-        pop();
-      }
-      if (!__any_sync(__activemask(), leaf == 0)) break;
-    }
-    // ---- leaves
-    for (;;) {
-      int code = 0;
-      if (leaf < 0) {
-        code = ~leaf;
-        leaf = 0;
-      } else if (t.node < 0 && t.node != kTravDone) {
-        code = ~t.node;
-        pop();
-      } else {
-        break;
-      }
-      const int first = code >> 4;
-      const int cnt = (code & 15) + 1;
-      if (kCount) tc->tris += cnt;
-      for (int i = 0; i < cnt; ++i) {
-        const float4 *tp = s.tri + 3 * (size_t)(first + i);
-        const float4 A = __ldg(tp + 0), E1 = __ldg(tp + 1), E2 = __ldg(tp + 2);
-        float u, v;
-        const float tt = tri_hit(t.o, t.d, A, E1, E2, eps, u, v);
-        if (tt > eps && tt < t.h.t) {
-          t.h.t = tt;
-          t.h.u = u;
-          t.h.v = v;
-          t.h.slot = first + i;
-          t.tcull = fminf(t.tcull, cull_bound(tt));
-        }
-      }
-    }
-    if (t.node == kTravDone && leaf == 0) return true;
-  }
-  return t.node == kTravDone && leaf == 0;
+// Slab test of one child record (lo.x hi.x lo.y hi.y | lo.z hi.z link -): the
+// arithmetic of box_hit(), both planes of an axis in one packed operation.
+TS_D void child_hit(const Rec32 &c, const f32x2 *no, const f32x2 *inv, float &te, float &tx) {
+  float ax, bx, ay, by, az, bz;
+  unpack2(mul2(add2(c.a, no[0]), inv[0]), ax, bx);
+  unpack2(mul2(add2(c.b, no[1]), inv[1]), ay, by);
+  unpack2(mul2(add2(c.c, no[2]), inv[2]), az, bz);
+  te = max3(fminf(ax, bx), fminf(ay, by), fminf(az, bz));
+  tx = min3(fmaxf(ax, bx), fmaxf(ay, by), fmaxf(az, bz));
 }
 
 // ---- quantized wide nodes (layout ids 5: 4 children in 64 B, 9: 8 children in 96 B)
@@ -515,123 +201,366 @@ TS_D bool trav_steps_wide_spec(const DevScene &s, Traversal &t, int2 *stack, flo
 // the exact one: the slab test accepts at least the rays the exact box would,
 // entry distances are no larger, and culling stays conservative -- the
 // closest hit is the same as with full-precision boxes.
-template <int WQ, bool kCount = false>
-TS_D bool trav_steps_q(const DevScene &s, Traversal &t, int2 *stack, float eps, int budget, uint32_t &errbits,
-                       TraceCount *tc = nullptr) {
+template <int WQ>
+TS_D int node_children_q(const DevScene &s, const Traversal &t, float *key, int *ref) {
   constexpr int N = WQ == 9 ? 8 : 4;  // children per node
   constexpr int R = N / 4;            // float4s of refs (and 32-bit words per byte plane)
   constexpr int F = WQ == 9 ? 6 : 4;  // float4s per node
-  for (int it = 0; it < budget; ++it) {
-    if (t.node == kTravDone) return true;
+  const float3 o = trav_origin(t), inv = f3(lane0(t.inv[0]), lane0(t.inv[1]), lane0(t.inv[2]));
+  const float4 *n = s.node + (size_t)F * t.node;
+  const float4 h = __ldg(n);
+  const uint32_t meta = __float_as_uint(h.w);
+  const float sx = __uint_as_float((meta & 0xffu) << 23);
+  const float sy = __uint_as_float(((meta >> 8) & 0xffu) << 23);
+  const float sz = __uint_as_float(((meta >> 16) & 0xffu) << 23);
+  const int nc = (int)(meta >> 24);
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const int4 l = __ldg(reinterpret_cast<const int4 *>(n + 1 + q));
+    ref[4 * q + 0] = l.x; ref[4 * q + 1] = l.y; ref[4 * q + 2] = l.z; ref[4 * q + 3] = l.w;
+  }
+  uint32_t wq[6 * R];  // plane r, children 4j..4j+3 in word r * R + j
+  {
+    const uint4 *b = reinterpret_cast<const uint4 *>(n + 1 + R);
+#pragma unroll
+    for (int i = 0; i < (6 * R + 3) / 4; ++i) {
+      const uint4 v = __ldg(b + i);
+      if (4 * i + 0 < 6 * R) wq[4 * i + 0] = v.x;
+      if (4 * i + 1 < 6 * R) wq[4 * i + 1] = v.y;
+      if (4 * i + 2 < 6 * R) wq[4 * i + 2] = v.z;
+      if (4 * i + 3 < 6 * R) wq[4 * i + 3] = v.w;
+    }
+  }
+  int nh = 0;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const int j = k >> 2, sh = 8 * (k & 3);
+    const float lox = xadd(h.x, xmul((float)((wq[0 * R + j] >> sh) & 0xffu), sx));
+    const float hix = xadd(h.x, xmul((float)((wq[1 * R + j] >> sh) & 0xffu), sx));
+    const float loy = xadd(h.y, xmul((float)((wq[2 * R + j] >> sh) & 0xffu), sy));
+    const float hiy = xadd(h.y, xmul((float)((wq[3 * R + j] >> sh) & 0xffu), sy));
+    const float loz = xadd(h.z, xmul((float)((wq[4 * R + j] >> sh) & 0xffu), sz));
+    const float hiz = xadd(h.z, xmul((float)((wq[5 * R + j] >> sh) & 0xffu), sz));
+    float te, tx;
+    box_hit(lox, hix, loy, hiy, loz, hiz, o, inv, te, tx);
+    const bool hit = k < nc && te < tx && tx > 0.f && te <= t.tcull;
+    key[k] = hit ? te : INFINITY;
+    nh += hit;
+  }
+  if (nh > 0) sort_children<N>(key, ref);
+  return nh;
+}
+
+// The children of a wide node that the ray enters, as sorted (entry distance,
+// link) pairs; returns how many.
+// W: 4 or 8, 5 and 9 for quantized nodes.
+template <int W>
+TS_D int node_children(const DevScene &s, const Traversal &t, float *key, int *ref) {
+  if (W == 5 || W == 9) return node_children_q<W>(s, t, key, ref);
+  const float4 *n = s.node + (size_t)t.node * (2 * W);
+  int nh = 0;
+#pragma unroll
+  for (int k = 0; k < W; ++k) {
+    const Rec32 c = load32(n + 2 * k);
+    float te, tx;
+    child_hit(c, t.no, t.inv, te, tx);
+    const bool h = te < tx && tx > 0.f && te <= t.tcull;
+    key[k] = h ? te : INFINITY;
+    ref[k] = (int)(uint32_t)c.d;
+    nh += h;
+  }
+  if (nh > 0) sort_children<W>(key, ref);
+  return nh;
+}
+
+// children per node of a layout
+template <int W>
+struct Children {
+  static constexpr int value = W >= 8 ? 8 : 4;
+};
+
+TS_D void trav_pop(Traversal &t, const int2 *stack) {
+  // the next box that is still closer than the cull bound
+  for (;;) {
+    if (t.sp == 0) {
+      t.node = kTravDone;
+      return;
+    }
+    const int2 e = stack[--t.sp];
+    if (__int_as_float(e.y) <= t.tcull) {
+      t.node = e.x;
+      return;
+    }
+  }
+}
+
+// an inner node: the nearest child the ray enters is visited next, the others
+// are pushed (farthest first) with their entry distances
+template <int W>
+TS_D void trav_inner(const DevScene &s, Traversal &t, int2 *stack, uint32_t &errbits) {
+  constexpr int N = Children<W>::value;
+  float key[N];
+  int ref[N];
+  const int nh = node_children<W>(s, t, key, ref);
+  if (nh == 0) {
+    trav_pop(t, stack);
+    return;
+  }
+  if (t.sp + nh - 1 <= kWideStack) {
+#pragma unroll
+    for (int k = N - 1; k >= 1; --k)
+      if (k < nh) stack[t.sp++] = make_int2(ref[k], __float_as_int(key[k]));
+  } else {
+    errbits |= kErrStackOverflow;
+  }
+  t.node = ref[0];
+}
+
+// A traversal by itself, to its end.
+template <int W, bool kCount = false>
+TS_D void trav_run(const DevScene &s, Traversal &t, int2 *stack, float eps, uint32_t &errbits,
+                   TraceCount *tc = nullptr) {
+  while (t.node != kTravDone) {
     if (t.node >= 0) {
-      const float4 *n = s.node + (size_t)F * t.node;
       if (kCount) tc->nodes++;
-      const float4 h = __ldg(n);
-      const uint32_t meta = __float_as_uint(h.w);
-      const float sx = __uint_as_float((meta & 0xffu) << 23);
-      const float sy = __uint_as_float(((meta >> 8) & 0xffu) << 23);
-      const float sz = __uint_as_float(((meta >> 16) & 0xffu) << 23);
-      const int nc = (int)(meta >> 24);
-      int ref[N];
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const int4 l = __ldg(reinterpret_cast<const int4 *>(n + 1 + q));
-        ref[4 * q + 0] = l.x; ref[4 * q + 1] = l.y; ref[4 * q + 2] = l.z; ref[4 * q + 3] = l.w;
+      trav_inner<W>(s, t, stack, errbits);
+    } else {
+      const int first = ~t.node >> 4, cnt = (~t.node & 15) + 1;
+      if (kCount) tc->tris += cnt;
+      const float3 o = trav_origin(t);
+      for (int i = 0; i < cnt; ++i) trav_triangle(s, t, o, first + i, eps);
+      trav_pop(t, stack);
+    }
+  }
+}
+
+// One phase of a warp whose lanes step together: inner nodes, or one triangle of
+// a leaf.  A lane at a leaf waits until kLeafLanes lanes are at one, or none has
+// a node to test, so that both phases run with many lanes.  When every lane went
+// on by itself (a budget of steps, leaves tested as a lane came to them), nodes
+// ran with 16 to 19 lanes of 32, but triangles with 4 to 6 and the end of a ray
+// with 2 to 4, and these were half of the instructions; in phases the same
+// launches take 25 to 29 % fewer instructions.
+// Returns false when no lane has anything left (node == kTravDone in all).
+constexpr int kLeafLanes = 12;  // 8: 1 % slower, 16: the same, 20: 1 % slower (terrain, box, volume)
+
+template <int W>
+TS_D bool warp_phase(const DevScene &s, Traversal &t, int2 *stack, float eps, uint32_t &errbits,
+                     unsigned mask = 0xffffffffu) {
+  const bool at_leaf = t.node < 0 && t.node != kTravDone;
+  const unsigned inner = __ballot_sync(mask, t.node >= 0);
+  const unsigned leaf = __ballot_sync(mask, at_leaf);
+  if (inner && __popc(leaf) < kLeafLanes) {
+    if (t.node >= 0) trav_inner<W>(s, t, stack, errbits);
+  } else if (leaf) {
+    if (at_leaf) {
+      const int code = ~t.node;
+      trav_triangle(s, t, trav_origin(t), code >> 4, eps);
+      if (code & 15) t.node = ~(code + 15);  // the leaf's next triangle: first + 1, count - 1
+      else trav_pop(t, stack);
+    }
+  } else {
+    return false;
+  }
+  __syncwarp(mask);
+  return true;
+}
+
+// ---- the layouts' own visiting orders -------------------------------------
+// Plain loops with box_hit() in the visiting order that defines a layout's
+// results: which of two triangles at exactly the same distance wins.  They
+// run for the rays that the fast loops hand over -- a tie, where those loops
+// visit in another order -- and for the counting pass.
+
+// two children per node, nearest first, over the reference-layout table
+template <bool kCount = false>
+TS_D Hit trace_two_child(const DevScene &s, float3 o, float3 d, float eps, uint32_t &errbits, TraceCount *tc,
+                         float bound) {
+  Hit h;
+  h.t = 1e9f;
+  h.u = h.v = 0.f;
+  h.slot = -1;
+  if (s.num_ref_nodes <= 0) return h;
+  const float3 inv = f3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
+  float tcull = cull_bound(fminf(bound, 1e9f));
+  int2 stack[kStackDepth];
+  int sp = 0;
+  auto entry = [&](int ni, float &te) {
+    const float *mn = s.ref_min + 3 * (size_t)ni, *mx = s.ref_max + 3 * (size_t)ni;
+    float tx;
+    box_hit(__ldg(mn), __ldg(mx), __ldg(mn + 1), __ldg(mx + 1), __ldg(mn + 2), __ldg(mx + 2), o, inv, te, tx);
+    return te < tx && tx > 0.f && te <= tcull;
+  };
+  int ni = 0;
+  int4 l = __ldg(s.ref_link);
+  bool go = true;
+  if (l.z > 0) {  // the root is a leaf: a node with one child
+    float te;
+    if (kCount) tc->nodes++;
+    go = entry(0, te);
+  }
+  while (go) {
+    bool down = false;
+    if (l.z <= 0) {
+      float e0, e1;
+      if (kCount) tc->nodes++;
+      const bool h0 = entry(l.x, e0), h1 = entry(l.y, e1);
+      if (h0 && h1) {
+        const bool sw = e1 < e0;
+        if (sp < kStackDepth) stack[sp++] = sw ? make_int2(l.x, __float_as_int(e0)) : make_int2(l.y, __float_as_int(e1));
+        else errbits |= kErrStackOverflow;
+        ni = sw ? l.y : l.x;
+      } else {
+        ni = h0 ? l.x : l.y;
       }
-      uint32_t wq[6 * R];  // plane r, children 4j..4j+3 in word r * R + j
-      {
-        const uint4 *b = reinterpret_cast<const uint4 *>(n + 1 + R);
-#pragma unroll
-        for (int i = 0; i < (6 * R + 3) / 4; ++i) {
-          const uint4 v = __ldg(b + i);
-          if (4 * i + 0 < 6 * R) wq[4 * i + 0] = v.x;
-          if (4 * i + 1 < 6 * R) wq[4 * i + 1] = v.y;
-          if (4 * i + 2 < 6 * R) wq[4 * i + 2] = v.z;
-          if (4 * i + 3 < 6 * R) wq[4 * i + 3] = v.w;
+      down = h0 || h1;
+    } else {
+      if (kCount) tc->tris += l.z;
+      for (int i = 0; i < l.z; ++i) {
+        const int slot = l.w + i;
+        const float4 *tp = s.tri + 3 * (size_t)slot;
+        float u, v;
+        const float tt = tri_hit(o, d, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), eps, u, v);
+        if (tt > eps && tt < h.t) {
+          h.t = tt;
+          h.u = u;
+          h.v = v;
+          h.slot = slot;
+          tcull = fminf(tcull, cull_bound(tt));
         }
       }
-      float key[N];
+    }
+    while (!down && sp > 0) {
+      const int2 e = stack[--sp];
+      if (__int_as_float(e.y) <= tcull) {
+        ni = e.x;
+        down = true;
+      }
+    }
+    go = down;
+    if (go) l = __ldg(s.ref_link + ni);
+  }
+  return h;
+}
+
+// 4 or 8 children per node, all that are entered sorted by distance
+template <int W, bool kCount = false>
+TS_D Hit trace_wide_plain(const DevScene &s, float3 o, float3 d, float eps, uint32_t &errbits, TraceCount *tc,
+                          float bound) {
+  Hit h;
+  h.t = 1e9f;
+  h.u = h.v = 0.f;
+  h.slot = -1;
+  if (s.num_nodes <= 0) return h;
+  const float3 inv = f3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
+  float tcull = cull_bound(fminf(bound, 1e9f));
+  int2 stack[kWideStack];
+  int sp = 0, node = 0;
+  for (;;) {
+    if (node >= 0) {
+      const float *n = reinterpret_cast<const float *>(s.node) + (size_t)(W == 4 ? 32 : 64) * node;
+      if (kCount) tc->nodes++;
+      float key[W];
+      int ref[W];
       int nh = 0;
 #pragma unroll
-      for (int k = 0; k < N; ++k) {
-        const int j = k >> 2, sh = 8 * (k & 3);
-        const float lox = xadd(h.x, xmul((float)((wq[0 * R + j] >> sh) & 0xffu), sx));
-        const float hix = xadd(h.x, xmul((float)((wq[1 * R + j] >> sh) & 0xffu), sx));
-        const float loy = xadd(h.y, xmul((float)((wq[2 * R + j] >> sh) & 0xffu), sy));
-        const float hiy = xadd(h.y, xmul((float)((wq[3 * R + j] >> sh) & 0xffu), sy));
-        const float loz = xadd(h.z, xmul((float)((wq[4 * R + j] >> sh) & 0xffu), sz));
-        const float hiz = xadd(h.z, xmul((float)((wq[5 * R + j] >> sh) & 0xffu), sz));
+      for (int k = 0; k < W; ++k) {
         float te, tx;
-        box_hit(lox, hix, loy, hiy, loz, hiz, t.o, t.inv, te, tx);
-        const bool hit = k < nc && te < tx && tx > 0.f && te <= t.tcull;
+        const float *r = n + 8 * k;
+        box_hit(__ldg(r), __ldg(r + 1), __ldg(r + 2), __ldg(r + 3), __ldg(r + 4), __ldg(r + 5), o, inv, te, tx);
+        const bool hit = te < tx && tx > 0.f && te <= tcull;
         key[k] = hit ? te : INFINITY;
+        ref[k] = __float_as_int(__ldg(r + 6));
         nh += hit;
       }
       if (nh > 0) {
-        sort_children<N>(key, ref);
-        if (t.sp + nh - 1 <= kWideStack) {
+        sort_children<W>(key, ref);
+        if (sp + nh - 1 <= kWideStack) {
 #pragma unroll
-          for (int k = N - 1; k >= 1; --k)
-            if (k < nh) stack[t.sp++] = make_int2(ref[k], __float_as_int(key[k]));
+          for (int k = W - 1; k >= 1; --k)
+            if (k < nh) stack[sp++] = make_int2(ref[k], __float_as_int(key[k]));
         } else {
           errbits |= kErrStackOverflow;
         }
-        t.node = ref[0];
+        node = ref[0];
         continue;
       }
     } else {
-      const int code = ~t.node;
+      const int code = ~node;
       const int first = code >> 4;
       const int cnt = (code & 15) + 1;
       if (kCount) tc->tris += cnt;
       for (int i = 0; i < cnt; ++i) {
         const float4 *tp = s.tri + 3 * (size_t)(first + i);
-        const float4 A = __ldg(tp + 0), E1 = __ldg(tp + 1), E2 = __ldg(tp + 2);
         float u, v;
-        const float tt = tri_hit(t.o, t.d, A, E1, E2, eps, u, v);
-        if (tt > eps && tt < t.h.t) {
-          t.h.t = tt;
-          t.h.u = u;
-          t.h.v = v;
-          t.h.slot = first + i;
-          t.tcull = fminf(t.tcull, cull_bound(tt));
+        const float tt = tri_hit(o, d, __ldg(tp), __ldg(tp + 1), __ldg(tp + 2), eps, u, v);
+        if (tt > eps && tt < h.t) {
+          h.t = tt;
+          h.u = u;
+          h.v = v;
+          h.slot = first + i;
+          tcull = fminf(tcull, cull_bound(tt));
         }
       }
     }
     for (;;) {
-      if (t.sp == 0) {
-        t.node = kTravDone;
-        return true;
-      }
-      const int2 e = stack[--t.sp];
-      if (__int_as_float(e.y) <= t.tcull) {
-        t.node = e.x;
+      if (sp == 0) return h;
+      const int2 e = stack[--sp];
+      if (__int_as_float(e.y) <= tcull) {
+        node = e.x;
         break;
       }
     }
   }
-  return t.node == kTravDone;
 }
 
-// Dispatch on the node layout (a compile-time choice of each kernel instance).
-// W = 2: two-child if-if loop; W = 3: two-child speculative while-while (same
-// layout); W = 4 / 8: wide nodes; W = 5 / 9: quantized 4- / 8-wide nodes.
-template <int W, bool kCount = false>
-TS_D bool trav_advance(const DevScene &s, Traversal &t, int2 *stack, float eps, int budget, uint32_t &errbits,
-                       TraceCount *tc = nullptr) {
-  if (W == 2) return trav_steps<kCount>(s, t, stack, eps, budget, errbits, tc);
-  if (W == 3) return trav_steps_spec<kCount>(s, t, stack, eps, budget, errbits, tc);
-  if (W == 5 || W == 9) return trav_steps_q<W, kCount>(s, t, stack, eps, budget, errbits, tc);
-#ifdef TS_WIDE_SPECULATIVE
-  return trav_steps_wide_spec<W, kCount>(s, t, stack, eps, budget, errbits, tc);
-#else
-  return trav_steps_wide<W, kCount>(s, t, stack, eps, budget, errbits, tc);
-#endif
-}
-
+// Not inlined: rare, and one copy per kernel.
 template <int W>
-struct StackSize {
-  static constexpr int value = W <= 3 ? kStackDepth : kWideStack;
+__device__ __noinline__ Hit trace_plain(const DevScene &s, float3 o, float3 d, float eps, uint32_t &errbits,
+                                        float bound) {
+  if (W == 2) return trace_two_child(s, o, d, eps, errbits, nullptr, bound);
+  return trace_wide_plain<W == 8 ? 8 : 4>(s, o, d, eps, errbits, nullptr, bound);
+}
+
+// ---- layouts ----------------------------------------------------------------
+// A compile-time choice of each kernel instance.  W = 2: two-child layout, which
+// the fast loop walks as four-child nodes collapsed from the same tree (half the
+// steps of a ray); its box tests accept the same leaves, so only a ray that meets
+// two triangles at exactly the same distance can differ, and that ray is traced
+// again in the two-child order.  W = 4 / 8: wide nodes; W = 5 / 9: quantized.
+
+// bound: distance beyond which hits do not matter to the caller.  Boxes past
+// it are skipped; a hit beyond it may still be returned (callers treat such a
+// hit like a miss), so results are the same as with bound = 1e9.
+template <int W>
+TS_D void trav_begin(const DevScene &s, Traversal &t, float3 o, float3 d, float bound) {
+  const float3 inv = f3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
+  t.no[0] = pack2(-o.x, -o.x);
+  t.no[1] = pack2(-o.y, -o.y);
+  t.no[2] = pack2(-o.z, -o.z);
+  t.inv[0] = pack2(inv.x, inv.x);
+  t.inv[1] = pack2(inv.y, inv.y);
+  t.inv[2] = pack2(inv.z, inv.z);
+  t.d = d;
+  t.h.t = 1e9f;
+  t.h.u = t.h.v = 0.f;
+  t.h.slot = -1;
+  t.tcull = cull_bound(fminf(bound, 1e9f));
+  t.node = s.num_nodes > 0 ? 0 : kTravDone;
+  t.sp = 0;
+  t.tie = W == 2 && s.num_nodes <= 0;  // a two-child tree too deep for the wide stack has no wide nodes
+}
+
+// a finished traversal's hit does not stand: trace_plain() has to decide a tie
+template <int W>
+TS_D bool trav_tied(const Traversal &t) {
+  return W == 2 && t.tie;
+}
+
+// the node layout behind a layout id
+template <int W>
+struct Nodes {
+  static constexpr int value = W == 2 ? 4 : W;
 };
 
 // Fast closest hit in one go (local-memory stack).  errbits gets
@@ -640,14 +569,175 @@ struct StackSize {
 // Not inlined: one copy of the traversal per kernel instead of one per call
 // site keeps the megakernels' instruction footprint small (instruction-fetch
 // stalls dominated them when inlined).
-template <int W, bool kCount = false>
+// kCount counts the layout's own node visits and triangle tests.
+// kTogether: the lanes that arrive together step together (warp_phase): 9 % less
+// time for the adjoint's replays and the batch kernel, 15 % for ray queries; a
+// single pass of few paths waits more than it gains.
+template <int W, bool kCount = false, bool kTogether = true>
 __device__ __noinline__ Hit trace_closest(const DevScene &s, float3 o, float3 d, float eps, uint32_t &errbits,
                                           TraceCount *tc = nullptr, float bound = 1e9f) {
+  if (kCount && W == 2) return trace_two_child<true>(s, o, d, eps, errbits, tc, bound);
+  if (kCount && (W == 4 || W == 8)) return trace_wide_plain<W == 8 ? 8 : 4, true>(s, o, d, eps, errbits, tc, bound);
   Traversal t;
-  int2 stack[StackSize<W>::value];
-  trav_begin(s, t, o, d, bound);
-  trav_advance<W, kCount>(s, t, stack, eps, 0x7fffffff, errbits, tc);
+  int2 stack[kWideStack];
+  trav_begin<W>(s, t, o, d, bound);
+  if (kCount || !kTogether) {
+    trav_run<Nodes<W>::value, kCount>(s, t, stack, eps, errbits, tc);
+  } else {
+    const unsigned mask = __activemask();
+    while (warp_phase<Nodes<W>::value>(s, t, stack, eps, errbits, mask)) {}
+  }
+  if (trav_tied<W>(t)) return trace_plain<W>(s, o, d, eps, errbits, bound);
   return t.h;
+}
+
+// ---- group traversal ---------------------------------------------------------
+// G lanes (the node width, 4 or 8) walk one ray: lane k tests child k of a node
+// and triangles k, k + G, ... of a leaf.  Against a ray per lane a step is a
+// third of the instructions (one box, no sorting network, one triangle) and a
+// node costs one or two contiguous loads of the warp instead of eight scattered
+// ones per lane, and a warp serialises G times fewer rays.  All lanes of a warp run
+// the same loop: its votes and shuffles take the whole warp.
+constexpr int kGroupStack = 32;  // entries per ray, in shared memory; a ray that needs more goes to trace_plain()
+
+template <int G>
+struct GroupRay {
+  // the same in all lanes of the group
+  f32x2 no[3], inv[3];
+  float3 d;
+  float tcull;
+  int node, sp;
+  bool over;   // stack overflow: the result does not stand
+  // best of the triangles this lane tested
+  Hit h;
+  bool tie;
+};
+
+template <int G>
+TS_D void group_begin(const DevScene &s, GroupRay<G> &r, float3 o, float3 d, float bound) {
+  const float3 inv = f3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
+  r.no[0] = pack2(-o.x, -o.x);
+  r.no[1] = pack2(-o.y, -o.y);
+  r.no[2] = pack2(-o.z, -o.z);
+  r.inv[0] = pack2(inv.x, inv.x);
+  r.inv[1] = pack2(inv.y, inv.y);
+  r.inv[2] = pack2(inv.z, inv.z);
+  r.d = d;
+  r.tcull = cull_bound(fminf(bound, 1e9f));
+  r.node = s.num_nodes > 0 ? 0 : kTravDone;
+  r.sp = 0;
+  r.over = s.num_nodes <= 0;
+  r.h.t = 1e9f;
+  r.h.u = r.h.v = 0.f;
+  r.h.slot = -1;
+  r.tie = false;
+}
+
+// One step of every group of the warp: an inner node, the leaf it may lead to
+// and the pop that follows.  stack: shared, this group's column of [entry][stride].
+template <int G>
+TS_D void group_step(const DevScene &s, GroupRay<G> &r, int2 *stack, int stride, int sub, int shift, float eps) {
+  constexpr unsigned kFull = 0xffffffffu, kBits = (1u << G) - 1u;
+  bool pop = false;
+  const bool inner = r.node >= 0;
+  if (__any_sync(kFull, inner)) {
+    bool hit = false;
+    int key = 0x7fffffff, ref = 0;
+    if (inner) {
+      const Rec32 c = load32(s.node + (size_t)r.node * (2 * G) + 2 * sub);
+      float te, tx;
+      child_hit(c, r.no, r.inv, te, tx);
+      hit = te < tx && tx > 0.f && te <= r.tcull;
+      ref = (int)(uint32_t)c.d;
+      // order by entry distance, then child: bits of a non-negative float with
+      // the child in the lowest ones (rounded down: culling stays conservative)
+      if (hit) key = (__float_as_int(fmaxf(te, 0.f)) & ~(G - 1)) | sub;
+    }
+    const unsigned gm = (__ballot_sync(kFull, hit) >> shift) & kBits;
+    int rank = 0, best = key;
+#pragma unroll
+    for (int x = 1; x < G; ++x) {
+      const int other = __shfl_xor_sync(kFull, key, x);
+      rank += other < key;
+      best = min(best, other);
+    }
+    const int near = __shfl_sync(kFull, ref, shift + (best & (G - 1)));
+    if (inner) {
+      const int far = __popc(gm) - 1;  // children to push
+      if (far < 0) {
+        pop = true;
+      } else if (r.sp + far > kGroupStack) {
+        r.over = true;
+        r.node = kTravDone;
+      } else {
+        if (hit && rank > 0) stack[(r.sp + far - rank) * stride] = make_int2(ref, key & ~(G - 1));
+        r.sp += far;
+        r.node = near;
+      }
+    }
+  }
+  const bool leaf = r.node < 0 && r.node != kTravDone;
+  if (__any_sync(kFull, leaf)) {
+    int first = 0, cnt = 0;
+    if (leaf) {
+      first = ~r.node >> 4;
+      cnt = (~r.node & 15) + 1;
+      pop = true;
+    }
+    for (int i = sub; __any_sync(kFull, i - sub < cnt); i += G) {
+      if (i < cnt) {
+        const float4 *tp = s.tri + 3 * (size_t)(first + i);
+        const float4 A = __ldg(tp + 0), E1 = __ldg(tp + 1), E2 = __ldg(tp + 2);
+        const float3 o = f3(-lane0(r.no[0]), -lane0(r.no[1]), -lane0(r.no[2]));
+        float u, v;
+        const float tt = tri_hit(o, r.d, A, E1, E2, eps, u, v);
+        if (tt > eps && tt <= r.h.t) {
+          r.tie = tt == r.h.t;
+          if (!r.tie) {
+            r.h.t = tt;
+            r.h.u = u;
+            r.h.v = v;
+            r.h.slot = first + i;
+          }
+        }
+      }
+    }
+    float m = r.h.t;
+#pragma unroll
+    for (int x = 1; x < G; x <<= 1) m = fminf(m, __shfl_xor_sync(kFull, m, x));
+    r.tcull = fminf(r.tcull, cull_bound(m));
+  }
+  __syncwarp();
+  if (pop) {
+    r.node = kTravDone;
+    while (r.sp > 0) {
+      const int2 e = stack[--r.sp * stride];
+      if (__int_as_float(e.y) <= r.tcull) {
+        r.node = e.x;
+        break;
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// The finished groups' hits, the same in all their lanes; false where the hit
+// does not stand and trace_plain() has to be asked.  Run by the whole warp.
+template <int G>
+TS_D bool group_hit(const GroupRay<G> &r, int shift, Hit &h) {
+  constexpr unsigned kFull = 0xffffffffu, kBits = (1u << G) - 1u;
+  float m = r.h.t;
+#pragma unroll
+  for (int x = 1; x < G; x <<= 1) m = fminf(m, __shfl_xor_sync(kFull, m, x));
+  const bool own = r.h.slot >= 0 && r.h.t == m;
+  const unsigned owners = (__ballot_sync(kFull, own) >> shift) & kBits;
+  const unsigned ties = (__ballot_sync(kFull, own && r.tie) >> shift) & kBits;
+  const int src = shift + (owners ? __ffs(owners) - 1 : 0);
+  h.t = m;
+  h.u = __shfl_sync(kFull, r.h.u, src);
+  h.v = __shfl_sync(kFull, r.h.v, src);
+  h.slot = __shfl_sync(kFull, r.h.slot, src);
+  return !r.over && !ties && (owners & (owners - 1)) == 0;
 }
 
 // Exact reference-order closest hit on the reference-layout table.
