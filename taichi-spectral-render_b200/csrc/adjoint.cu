@@ -259,6 +259,7 @@ __global__ void __launch_bounds__(128, kPhase ? 4 : 5) k_adjoint(const __grid_co
           } else {
             if (phase) arem = weight[idx];
             rng.init(c.seed, pass, (uint32_t)pix, c.scene_id);
+            rng.fill<1>();
             camera_ray(s, c, pix % c.W, pix / c.W, rng, p, band);
             sp.reset();
             k = 0;
@@ -274,6 +275,7 @@ __global__ void __launch_bounds__(128, kPhase ? 4 : 5) k_adjoint(const __grid_co
 
     // ---- one path vertex, exactly as the forward megakernel takes it
     bool done = false;
+    rng.fill();
     const Hit h = trace_closest<W, false>(s, p.pos, p.dir, c.eps, errbits, nullptr, c.escape);
     const VolEvent ev = volume_event(s, c, p, h, rng);
     if (ev.travel < 0.f) {

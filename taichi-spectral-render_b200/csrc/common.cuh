@@ -129,21 +129,32 @@ TS_HD uint4 philox4x32_10(uint4 c, uint2 k) {
 // Per-path stream.  Draw n is word (n & 3) of block n >> 2, so a path's
 // sequence depends only on (seed, pass, pixel, scene) and the draw index; the
 // state that must survive between kernels is just the draw index.
+// The words of a vertex are drawn ahead by all lanes of a warp together
+// (fill): lanes stand at different words of their blocks, so with a block
+// computed where its first word is drawn nearly every draw cost the warp the
+// ten rounds -- a quarter of the instructions of shading.  fill() comes before
+// the draws of a vertex, which are at most 12 (free flight 1, light 3, surface
+// 3 + 1 + 2 + 2; a camera ray draws 2): they lie in the blocks drawn ahead.
 struct Rng {
+  static constexpr int kAhead = 4;  // blocks: 12 words from any word of the first
   uint2 key;
   uint32_t pix, scene, n;
-  uint4 buf;
+  uint32_t base;      // first draw of w
+  uint4 w[kAhead];
   TS_D void init(uint32_t seed, uint32_t pass, uint32_t pixel, uint32_t scene_id, uint32_t draw = 0) {
     key = make_uint2(seed, pass);
     pix = pixel;
     scene = scene_id;
     n = draw;
-    if (n & 3u) buf = philox4x32_10(make_uint4(pix, n >> 2, scene, 0u), key);
+  }
+  template <int kBlocks = kAhead>
+  TS_D void fill() {
+    base = n & ~3u;
+#pragma unroll 2
+    for (int j = 0; j < kBlocks; ++j) w[j] = philox4x32_10(make_uint4(pix, (n >> 2) + j, scene, 0u), key);
   }
   TS_D float next() {
-    if ((n & 3u) == 0) buf = philox4x32_10(make_uint4(pix, n >> 2, scene, 0u), key);
-    const uint32_t w = n & 3u;
-    const uint32_t x = w == 0 ? buf.x : (w == 1 ? buf.y : (w == 2 ? buf.z : buf.w));
+    const uint32_t x = reinterpret_cast<const uint32_t *>(w)[n - base];
     ++n;
     return (float)(x >> 8) * (1.0f / 16777216.0f);
   }

@@ -49,6 +49,7 @@ __device__ __forceinline__ void mega_start(const DevScene &s, const DevConfig &c
   L.moved = false;
   L.band = band;
   L.rng.init(c.seed, pass, (uint32_t)pixel, c.scene_id);
+  L.rng.fill<1>();
   camera_ray(s, c, pixel % c.W, pixel / c.W, L.rng, L.p, band);
   L.k = 0;
   L.dep = 0.0;
@@ -61,6 +62,7 @@ __device__ __forceinline__ bool mega_vertex(const DevScene &s, const DevConfig &
   PathState &p = L.p;
   const int band = L.band;
   bool done = false;
+  L.rng.fill();
   // hits beyond ESCAPE count as escapes (main.py:1209-1214): traverse no further
   const Hit h = trace_closest<W, kCount, kTogether>(s, p.pos, p.dir, c.eps, errbits, &cnt.tc, c.escape);
   const VolEvent ev = volume_event(s, c, p, h, L.rng);

@@ -37,11 +37,41 @@ constexpr int kCntFetchT = kCntSh + kMaxDepth + 1;
 constexpr int kCntFetchS = kCntFetchT + kMaxDepth + 1;
 constexpr int kCntTotal = kCntFetchS + kMaxDepth + 1;
 
-__device__ __forceinline__ int warp_fetch(int *ctr) {
+// ---- work fetching
+// The blocks of k_shade* and trace_groups are all resident (resident_grid: what the
+// kernel's registers allow), so every warp has its first items without asking:
+// warp w those from w * share.  Later ones come from the counter.  An empty stage
+// then costs a launch and no atomics (11 us before, 2,368 blocks asking in turn).
+// trace_lanes asks for all of its items: it has many, and the code for the first
+// ones cost it 10 %.
+constexpr int kSMs = 148;
+constexpr int kStageThreads = 1024;  // resident threads per SM: trace_lanes, k_shade_loop (64 registers)
+constexpr int kWideThreads = 512;    // trace_groups, k_shade (128 registers)
+
+inline int resident_grid(int grid, int block, int threads_per_sm) {
+  const int most = kSMs * (threads_per_sm / block > 0 ? threads_per_sm / block : 1);
+  return grid < most ? grid : most;
+}
+
+__device__ __forceinline__ int warps_of_grid() { return (int)(gridDim.x * (blockDim.x >> 5)); }
+__device__ __forceinline__ int warp_of_grid() {
+  return (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+}
+
+// Items a warp takes at a time: of few items fewer in each warp rather than fewer
+// warps, so that a warp runs fewer of its lanes' branches one after the other.
+__device__ __forceinline__ int warp_share(int total, int most) {
+  const int warps = warps_of_grid();
+  return min(most, max(1, (total + warps - 1) / warps));
+}
+
+// the next n items for the warp
+__device__ __forceinline__ int warp_fetch(int *ctr, int n, bool first) {
+  if (first) return warp_of_grid() * n;
   const int lane = threadIdx.x & 31;
   int base = 0;
-  if (lane == 0) base = atomicAdd(ctr, 32);
-  return __shfl_sync(0xffffffffu, base, 0);
+  if (lane == 0) base = atomicAdd(ctr, n);
+  return warps_of_grid() * n + __shfl_sync(0xffffffffu, base, 0);
 }
 
 // append with one atomic per warp; returns the slot for lanes with want=true
@@ -70,6 +100,7 @@ __device__ __forceinline__ void start_path(float3 o, float3 cu, float3 cv, float
                                            uint32_t pass, int band, int pix, const WaveBuffers &w, int slot) {
   Rng rng;
   rng.init(c.seed, pass, (uint32_t)pix, c.scene_id);
+  rng.fill<1>();
   PathState ps;
   camera_ray(o, cu, cv, cw, c, pix % c.W, pix / c.W, rng, ps, band);
   w.pos_thr[slot] = make_float4(ps.pos.x, ps.pos.y, ps.pos.z, ps.thr);
@@ -112,17 +143,19 @@ struct OneScene {
   __device__ __forceinline__ bool shared(int) const { return shared_film; }
 };
 
-// the next work item for each lane that wants one (one atomic per warp; G lanes
-// of a group share one), -1 for the others
+// The next work item for each lane that wants one (one atomic per warp; the G
+// lanes of a group share one), -1 for the others.  share: items a warp starts
+// with (0: none); first: those, which the first lanes or groups take.
 template <int G>
-__device__ __forceinline__ int fetch_items(int *fetch, bool want) {
+__device__ __forceinline__ int fetch_items(int *fetch, bool want, int share, bool first) {
+  const int lane = threadIdx.x & 31;
+  if (first) return want ? warp_of_grid() * share + lane / G : -1;
   const unsigned m = __ballot_sync(0xffffffffu, want);
   if (!m) return -1;
-  const int lane = threadIdx.x & 31;
   const int leader = __ffs(m) - 1;
   int base = 0;
   if (lane == leader) base = atomicAdd(fetch, __popc(m) / G);
-  base = __shfl_sync(0xffffffffu, base, leader);
+  base = warps_of_grid() * share + __shfl_sync(0xffffffffu, base, leader);
   return want ? base + __popc(m & ((1u << (lane & ~(G - 1))) - 1u)) / G : -1;
 }
 
@@ -269,7 +302,8 @@ __device__ __forceinline__ void trace_lanes(const Src &src, const WaveBuffers &w
         if (!im.plain) item_hit(src, w, im, t.h, true, begin);
       }
       __syncwarp();
-      const int idx = fetch_items<1>(it.fetch, im.id < 0 && !exhausted);
+      const int idx =  fetch_items<1>(it.fetch, im.id < 0 && !exhausted, 0, false);
+
       if (idx >= 0) {
         exhausted = idx >= it.total;
         if (!exhausted) item_start(src, w, it, idx, im, begin);
@@ -308,11 +342,13 @@ __device__ __forceinline__ void trace_groups(const Src &src, const WaveBuffers &
   t.h.u = t.h.v = 0.f;
   t.h.slot = -1;
   t.tie = false;
-  bool exhausted = false;
+  const int rays = warp_share(it.total, 32 / G);
+  const int stop = rays > 3 ? kGroupIdle * G : G;
+  bool exhausted = lane / G >= rays, first = true;
   for (;;) {
     const bool done = t.node == kTravDone && !im.plain;
     const unsigned idle = __ballot_sync(kFull, done && !(exhausted && im.id < 0));
-    if (__popc(idle) >= kGroupIdle * G || __ballot_sync(kFull, t.node != kTravDone) == 0) {
+    if (__popc(idle) >= stop || __ballot_sync(kFull, t.node != kTravDone) == 0) {
       Hit h;
       const bool good = group_hit(t, shift, h);
       const auto begin = [&](const DevScene &s, float3 o, float3 d, float bound) { group_begin(s, t, o, d, bound); };
@@ -321,7 +357,8 @@ __device__ __forceinline__ void trace_groups(const Src &src, const WaveBuffers &
         if (good) item_hit(src, w, im, h, sub == 0, begin);
       }
       __syncwarp();
-      const int idx = fetch_items<G>(it.fetch, im.id < 0 && !exhausted);
+      const int idx = fetch_items<G>(it.fetch, im.id < 0 && !exhausted, rays, first);
+      first = false;
       if (idx >= 0) {
         exhausted = idx >= it.total;
         if (!exhausted) item_start(src, w, it, idx, im, begin);
@@ -364,7 +401,7 @@ __device__ __forceinline__ TraceItems trace_items(const DevConfig &c, int depth,
 }
 
 template <int W, bool kLoop, bool kGroups>
-__global__ void __launch_bounds__(kMaxBlock, 4) k_trace(const __grid_constant__ DevScene s,
+__global__ void __launch_bounds__(kMaxBlock, (kGroups ? kWideThreads : kStageThreads) / kMaxBlock) k_trace(const __grid_constant__ DevScene s,
                                                      const __grid_constant__ DevConfig c, int depth,
                                                      const __grid_constant__ Film f,
                                                      const __grid_constant__ WaveBuffers w,
@@ -373,6 +410,7 @@ __global__ void __launch_bounds__(kMaxBlock, 4) k_trace(const __grid_constant__ 
   extern __shared__ int2 group_stacks[];  // kGroups: [kGroupStack][groups of the block]
   uint32_t eb = 0;
   const TraceItems it = trace_items<kLoop>(c, depth, w, ext_sorted, shadow_sorted, L);
+  if (it.total <= 0) return;
   const OneScene src{s, c, f, kLoop && L->shared != 0};
   if constexpr (kGroups) trace_groups<W>(src, w, it, group_stacks, eb);
   else trace_lanes<W>(src, w, it, eb);
@@ -395,7 +433,7 @@ void launch_trace_w(const DevScene &s, const DevConfig &c, int depth, Film f, co
   if constexpr (W != 5 && W != 9) {
     if (paths <= kGroupPaths) {
       const size_t smem = (size_t)(block / (W == 8 ? 8 : 4)) * kGroupStack * sizeof(int2);
-      k_trace<W, kLoop, true><<<grid, block, smem, st>>>(s, c, depth, f, w, err, ext_sorted, shadow_sorted, L);
+      k_trace<W, kLoop, true><<<resident_grid(grid, block, kWideThreads), block, smem, st>>>(s, c, depth, f, w, err, ext_sorted, shadow_sorted, L);
       return;
     }
   }
@@ -527,6 +565,7 @@ __device__ __forceinline__ void shade_path(const DevScene &s, const DevConfig &c
   p.vol = m.z;
   Rng rng;
   rng.init(c.seed, pass, (uint32_t)m.x, c.scene_id, (uint32_t)m.w);
+  rng.fill();
   Hit h;
   h.t = hh.x;
   h.u = hh.y;
@@ -538,17 +577,17 @@ __device__ __forceinline__ void shade_path(const DevScene &s, const DevConfig &c
   p.thr *= ev.est;
   bool done = false;
   float indirect = 0.f;
+  int surf = -1;
   if (ev.action == 1) {
     const Mat sm = get_mat(s, c.B, ev.hit_mat, band);
     if (sm.surf_emis) {
       indirect = emitter_hit(s, c, p, ev, sm.emission);
       done = true;
     } else {
-      r.nee = nee_setup(s, c, p, band, ev.snormal, ev.hit_mat, rng, r.sq);
+      surf = ev.hit_mat;
     }
-  } else {
-    r.nee = nee_setup(s, c, p, band, ev.snormal, -1, rng, r.sq);
   }
+  if (!done) r.nee = nee_setup(s, c, p, band, ev.snormal, surf, rng, r.sq);  // one site: surfaces and media sample their light together
   r.sq.band = p.active;
   if (ev.action == 1 && !done) {
     p.plen++;
@@ -598,17 +637,18 @@ __device__ __forceinline__ void append_ext(int *count, int *q, int pid, bool wan
   else atomicOr(err, kErrQueueOverflow);
 }
 
-__global__ void __launch_bounds__(kMaxBlock) k_shade(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass, int band, int depth,
+__global__ void __launch_bounds__(kMaxBlock, kWideThreads / kMaxBlock) k_shade(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass, int band, int depth,
                                                Film f, WaveBuffers w, int use_sorted, uint32_t *err) {
   const int n = w.counts[kCntExt + depth];
   const int *q = use_sorted ? w.sorted : w.queue[depth & 1];
   int *qn = w.queue[(depth + 1) & 1];
   int *fetch = w.counts + kCntFetchS + depth;
   const bool last = depth + 1 >= c.max_depth;
-  for (;;) {
-    const int base = warp_fetch(fetch);
+  const int share = warp_share(n, 32);
+  for (bool first = true;; first = false) {
+    const int base = warp_fetch(fetch, share, first);
     if (base >= n) break;
-    const int i = base + (threadIdx.x & 31);
+    const int i = (threadIdx.x & 31) < share ? base + (int)(threadIdx.x & 31) : n;
     Shaded r;
     r.cont = r.nee = false;
     r.pix = -1;
@@ -670,7 +710,7 @@ __global__ void k_loop_init(const __grid_constant__ DevScene s, const __grid_con
 
 // 64 registers (4 resident 256-thread blocks per SM; a few spills): faster
 // than the unbounded 111-register build by 4-6 % on whole-bundle loops
-__global__ void __launch_bounds__(kMaxBlock, 4) k_shade_loop(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, Film f, WaveBuffers w, WaveLoop *L,
+__global__ void __launch_bounds__(kMaxBlock, kStageThreads / kMaxBlock) k_shade_loop(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, Film f, WaveBuffers w, WaveLoop *L,
                                                           uint32_t *err) {
   const int a = L->iter & 1;
   const int n = L->ext[a];
@@ -683,10 +723,11 @@ __global__ void __launch_bounds__(kMaxBlock, 4) k_shade_loop(const __grid_consta
   // total by at most one claim per slot
   const bool more = L->next_item < total;
   const int npix = c.W * c.H;
-  for (;;) {
-    const int base = warp_fetch(L->fetch + 1);
+  const int share = warp_share(n, 32);
+  for (bool first = true;; first = false) {
+    const int base = warp_fetch(L->fetch + 1, share, first);
     if (base >= n) break;
-    const int i = base + (threadIdx.x & 31);
+    const int i = (threadIdx.x & 31) < share ? base + (int)(threadIdx.x & 31) : n;
     Shaded r;
     r.cont = r.nee = false;
     r.pix = -1;
@@ -783,7 +824,7 @@ cudaError_t launch_wave_chunk(const DevScene &s, const DevConfig &c, uint32_t pa
     if (sh_sorted) launch_sort(s, d - 1, w, kSortShadow, kShadowKeys, w.shadow_order, sort_grid, st);
     launch_trace(s, c, d, f, w, err, grid, block, st, n, ext_sorted, sh_sorted);
     if (sort_keys & 1) launch_sort(s, d, w, kSortShade, nmat, w.sorted, sort_grid, st);
-    k_shade<<<grid, block, 0, st>>>(s, c, pass, band, d, f, w, (sort_keys & 1) ? 1 : 0, err);
+    k_shade<<<resident_grid(grid, block, kWideThreads), block, 0, st>>>(s, c, pass, band, d, f, w, (sort_keys & 1) ? 1 : 0, err);
   }
   // the last depth's shadow queries
   if (c.max_depth > 0) {
@@ -834,7 +875,7 @@ cudaError_t build_wave_loop(WaveLoopGraph &G, const DevScene &s, const DevConfig
       cudaSuccess)
     return e;
   launch_trace<true>(s, c, 0, f, w, err, grid, block, G.capture, paths, 0, 0, w.loop);
-  k_shade_loop<<<grid, block, 0, G.capture>>>(s, c, f, w, w.loop, err);
+  k_shade_loop<<<resident_grid(grid, block, kStageThreads), block, 0, G.capture>>>(s, c, f, w, w.loop, err);
   k_loop_control<<<1, 32, 0, G.capture>>>(w.loop, h, 1, err);
   const cudaError_t le = cudaGetLastError();
   cudaGraph_t captured = nullptr;
@@ -890,7 +931,7 @@ cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pas
     k_loop_init<<<init_grid, 256, 0, st>>>(s, c, w, w.loop, pass0, band0, npass, n0, limit, shared);
     for (int it = 0; it < limit; ++it) {
       launch_trace<true>(s, c, 0, f, w, err, grid, block, st, n0, 0, 0, w.loop);
-      k_shade_loop<<<grid, block, 0, st>>>(s, c, f, w, w.loop, err);
+      k_shade_loop<<<resident_grid(grid, block, kStageThreads), block, 0, st>>>(s, c, f, w, w.loop, err);
       k_loop_control<<<1, 32, 0, st>>>(w.loop, 0, 0, err);
       int go = 0;
       cudaError_t e = cudaMemcpyAsync(&go, &w.loop->go, sizeof(int), cudaMemcpyDeviceToHost, st);
@@ -992,7 +1033,7 @@ struct BatchScenes {
 };
 
 template <int W>
-__global__ void __launch_bounds__(kMaxBlock, 4) k_trace_bloop(const BatchSlot *__restrict__ slots,
+__global__ void __launch_bounds__(kMaxBlock, kStageThreads / kMaxBlock) k_trace_bloop(const BatchSlot *__restrict__ slots,
                                                            const __grid_constant__ WaveBuffers w,
                                                            uint32_t *__restrict__ err, WaveLoop *L) {
   uint32_t eb = 0;
@@ -1006,7 +1047,7 @@ __global__ void __launch_bounds__(kMaxBlock, 4) k_trace_bloop(const BatchSlot *_
 // shade stage of the batch loop: k_shade_loop with each item's view; an ended
 // path's slot starts the next work item of the whole pool, whichever view it
 // belongs to
-__global__ void __launch_bounds__(kMaxBlock, 4) k_shade_bloop(const BatchSlot *__restrict__ slots, int nslots,
+__global__ void __launch_bounds__(kMaxBlock, kStageThreads / kMaxBlock) k_shade_bloop(const BatchSlot *__restrict__ slots, int nslots,
                                                            WaveBuffers w, WaveLoop *L, uint32_t *err) {
   const int a = L->iter & 1;
   const int n = L->ext[a];
@@ -1014,10 +1055,11 @@ __global__ void __launch_bounds__(kMaxBlock, 4) k_shade_bloop(const BatchSlot *_
   int *qn = w.queue[a ^ 1];
   const int total = L->total;
   const bool more = L->next_item < total;
-  for (;;) {
-    const int base = warp_fetch(L->fetch + 1);
+  const int share = warp_share(n, 32);
+  for (bool first = true;; first = false) {
+    const int base = warp_fetch(L->fetch + 1, share, first);
     if (base >= n) break;
-    const int i = base + (threadIdx.x & 31);
+    const int i = (threadIdx.x & 31) < share ? base + (int)(threadIdx.x & 31) : n;
     Shaded r;
     r.cont = r.nee = false;
     r.pix = -1;
@@ -1078,7 +1120,7 @@ cudaError_t launch_trace_bloop(const BatchSlot *slots, const WaveBuffers &w, uin
 cudaError_t bloop_body(BatchSlot *slots, int n, const WaveBuffers &w, uint32_t *err, int width, int grid, int block, cudaGraphConditionalHandle h, int in_graph, cudaStream_t st) {
   cudaError_t e = launch_trace_bloop(slots, w, err, width, grid, block, st);
   if (e != cudaSuccess) return e;
-  k_shade_bloop<<<grid, block, 0, st>>>(slots, n, w, w.loop, err);
+  k_shade_bloop<<<resident_grid(grid, block, kStageThreads), block, 0, st>>>(slots, n, w, w.loop, err);
   k_loop_control<<<1, 32, 0, st>>>(w.loop, h, in_graph, err);
   return cudaGetLastError();
 }
@@ -1221,6 +1263,7 @@ __global__ void k_generate_tile(const __grid_constant__ DevScene s, const __grid
     const int pixel = j * c.W + i;
     Rng rng;
     rng.init(c.seed, pass, (uint32_t)pixel, c.scene_id);
+    rng.fill<1>();
     PathState ps;
     camera_ray(s, c, i, j, rng, ps, band);
     w.pos_thr[p] = make_float4(ps.pos.x, ps.pos.y, ps.pos.z, ps.thr);
@@ -1310,7 +1353,7 @@ cudaError_t launch_wave_tile_noalloc(const DevScene &s, const DevConfig &c, uint
   k_generate_tile<<<(n + 255) / 256, 256, 0, st>>>(s, c, pass, band, w, x0, y0, tw, th);
   for (int d = 0; d < c.max_depth; ++d) {
     launch_trace(s, c, d, f, w, err, grid, block, st, n);
-    k_shade<<<grid, block, 0, st>>>(s, c, pass, band, d, f, w, 0, err);
+    k_shade<<<resident_grid(grid, block, kWideThreads), block, 0, st>>>(s, c, pass, band, d, f, w, 0, err);
   }
   if (c.max_depth > 0) launch_trace(s, c, c.max_depth, f, w, err, grid, block, st, n);
   return cudaGetLastError();
