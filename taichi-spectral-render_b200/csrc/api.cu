@@ -39,7 +39,7 @@ struct ts_ctx {
   int *d_counter = nullptr;
   uint32_t *d_err = nullptr;
   float *d_xyz = nullptr;
-  float *d_m9 = nullptr;  // XYZ->RGB matrix for ts_resolve_rgb
+  float *d_frame_rgb = nullptr;  // ts_resolve_rgb's image at render resolution
   float4 *d_mat = nullptr;  // packed material table (scene allocation), rewritten by ts_update_materials
   float *d_eem = nullptr, *d_qy = nullptr, *d_cdf = nullptr;
   float *d_adj_weight = nullptr;  // adjoint scratch: per-path weighted totals
@@ -191,7 +191,7 @@ ts_status ts_create(const ts_config *cfg, ts_ctx **out) {
   e = cudaMalloc((void **)&c->d_counter, 64 * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_err, sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xyz, (size_t)k.width * k.height * 3 * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_m9, 9 * sizeof(float));
+  if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_frame_rgb, (size_t)k.width * k.height * 3 * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, sizeof(uint32_t));
   if (e != cudaSuccess) {
     ts_destroy(c);
@@ -238,7 +238,7 @@ ts_status ts_destroy(ts_ctx *c) {
   cudaFree(c->d_counter);
   cudaFree(c->d_err);
   cudaFree(c->d_xyz);
-  cudaFree(c->d_m9);
+  cudaFree(c->d_frame_rgb);
   cudaFree(c->d_adj_weight);
   cudaFree(c->d_rec);
   delete c;
@@ -808,9 +808,9 @@ ts_status ts_resolve_rgb(ts_ctx *c, double scale, const float M[9], float exposu
   if (!c || !M || !rgb_dev || iw <= 0 || ih <= 0) return fail(c, TS_ERR_INVALID_ARG, "ts_resolve_rgb: bad argument");
   if (!c->has_scene) return fail(c, TS_ERR_NO_SCENE, "ts_resolve_rgb: no scene (CMF) uploaded");
   cudaSetDevice(c->cfg.device);
-  TS_CUDA(c, cudaMemcpyAsync(c->d_m9, M, 9 * sizeof(float), cudaMemcpyHostToDevice, as_stream(stream)),
-          "resolve rgb matrix");
-  TS_CUDA(c, ts::launch_resolve_rgb(film_of(c), c->d_cmf, scale, c->d_m9, exposure, gamma, iw, ih, rgb_dev,
+  ts::ColorMatrix m;
+  std::copy(M, M + 9, m.m);
+  TS_CUDA(c, ts::launch_resolve_rgb(film_of(c), c->d_cmf, scale, c->d_frame_rgb, m, exposure, gamma, iw, ih, rgb_dev,
                                     as_stream(stream)),
           "resolve rgb");
   return TS_OK;

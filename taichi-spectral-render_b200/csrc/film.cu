@@ -1,6 +1,8 @@
 // Film kernels (average_and_reset_block, color_rays, clear_pixel_space,
 // visualize_normals of the reference, main.py:1592-1674) and the batched
 // closest-hit query used by parity checks.
+#include <algorithm>
+
 #include "estimator.cuh"
 #include "kernels.cuh"
 
@@ -39,48 +41,104 @@ __global__ void k_clear(Film f) {
   }
 }
 
+// The colour-matching functions as doubles, once per block: converting them at
+// each pixel and band kept the conversion unit busier than the memory.
+constexpr int kMaxBands = 64;
+__device__ __forceinline__ void load_cmf(const float *__restrict__ cmf, int B, double *sh) {
+  for (int i = threadIdx.x; i < 3 * B; i += blockDim.x) sh[i] = (double)cmf[i];
+  __syncthreads();
+}
+
+// sum_k mean_k * cmf_k of one pixel, in band order
+__device__ __forceinline__ void pixel_xyz(const Film &f, const double *cmf, int npix, int p, double scale, float &x,
+                                          float &y, float &z) {
+  double X = 0.0, Y = 0.0, Z = 0.0;
+#pragma unroll 5
+  for (int k = 0; k < f.B; ++k) {
+    const double a = f.mean[(size_t)k * npix + p];
+    X += a * cmf[3 * k + 0];
+    Y += a * cmf[3 * k + 1];
+    Z += a * cmf[3 * k + 2];
+  }
+  x = (float)(X * scale);
+  y = (float)(Y * scale);
+  z = (float)(Z * scale);
+}
+
 // XYZ half of color_rays (main.py:1617-1620): sum_k mean_k * cmf_k * scale,
 // scale = step / normalisation.  Output [j][i][3] float32 at render resolution.
-__global__ void k_resolve_xyz(Film f, const float *__restrict__ cmf, double scale, float *__restrict__ xyz) {
+// HBM-bound: 200 B read and 12 B written per pixel.  Five bands' loads in flight
+// per thread; 1024^2: 47 us with a band at a time, 34 us now (34 us at a copy's rate).
+__global__ void k_resolve_xyz(const Film f, const float *__restrict__ cmf, double scale, float *__restrict__ xyz) {
+  __shared__ double cmf64[3 * kMaxBands];
+  load_cmf(cmf, f.B, cmf64);
   const int npix = f.W * f.H;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
-    double X = 0.0, Y = 0.0, Z = 0.0;
-    for (int k = 0; k < f.B; ++k) {
-      const double a = f.mean[(size_t)k * npix + p];
-      X += a * (double)cmf[3 * k + 0];
-      Y += a * (double)cmf[3 * k + 1];
-      Z += a * (double)cmf[3 * k + 2];
-    }
-    xyz[3 * (size_t)p + 0] = (float)(X * scale);
-    xyz[3 * (size_t)p + 1] = (float)(Y * scale);
-    xyz[3 * (size_t)p + 2] = (float)(Z * scale);
+    float x, y, z;
+    pixel_xyz(f, cmf64, npix, p, scale, x, y, z);
+    xyz[3 * (size_t)p + 0] = x;
+    xyz[3 * (size_t)p + 1] = y;
+    xyz[3 * (size_t)p + 2] = z;
   }
 }
 
-// Whole color_rays (main.py:1609-1629): nearest-neighbour upscale to the image
-// resolution, XYZ -> RGB, Reinhard with exposure, gamma.  Output [j][i][3].
-__global__ void k_resolve_rgb(Film f, const float *__restrict__ cmf, double scale, const float *__restrict__ M,
+// XYZ -> RGB, Reinhard with exposure, gamma (main.py:1621-1629)
+__device__ __forceinline__ void display_rgb(float x, float y, float z, const ColorMatrix &M, float exposure,
+                                            float gamma, float *__restrict__ rgb) {
+  for (int ch = 0; ch < 3; ++ch) {
+    const float h = M.m[3 * ch + 0] * x + M.m[3 * ch + 1] * y + M.m[3 * ch + 2] * z;
+    const float e = exposure * h;
+    const float mapped = e / (e + 1.0f);
+    rgb[ch] = powf(mapped, 1.0f / gamma);
+  }
+}
+
+// source pixel of image pixel i of n (nearest neighbour, main.py:1613-1615)
+__device__ __forceinline__ int source_of(int i, int n, int size) {
+  return (int)((float)i / (float)n * (float)size);
+}
+
+// Whole color_rays (main.py:1609-1629) of an image with fewer pixels than the
+// frame: nearest-neighbour, XYZ -> RGB, tone mapping.  Output [j][i][3].
+__global__ void k_resolve_rgb(const Film f, const float *__restrict__ cmf, double scale, const __grid_constant__ ColorMatrix M,
                               float exposure, float gamma, int iw, int ih, float *__restrict__ rgb) {
+  __shared__ double cmf64[3 * kMaxBands];
+  load_cmf(cmf, f.B, cmf64);
   const int npix = f.W * f.H;
   const int n = iw * ih;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
     const int i = p % iw, j = p / iw;
-    const int ri = (int)((float)i / (float)iw * (float)f.W);
-    const int rj = (int)((float)j / (float)ih * (float)f.H);
-    const int rp = rj * f.W + ri;
-    double X = 0.0, Y = 0.0, Z = 0.0;
-    for (int k = 0; k < f.B; ++k) {
-      const double a = f.mean[(size_t)k * npix + rp];
-      X += a * (double)cmf[3 * k + 0];
-      Y += a * (double)cmf[3 * k + 1];
-      Z += a * (double)cmf[3 * k + 2];
-    }
-    const float x = (float)(X * scale), y = (float)(Y * scale), z = (float)(Z * scale);
-    for (int ch = 0; ch < 3; ++ch) {
-      const float h = M[3 * ch + 0] * x + M[3 * ch + 1] * y + M[3 * ch + 2] * z;
-      const float e = exposure * h;
-      const float mapped = e / (e + 1.0f);
-      rgb[3 * (size_t)p + ch] = powf(mapped, 1.0f / gamma);
+    float x, y, z;
+    pixel_xyz(f, cmf64, npix, source_of(j, ih, f.H) * f.W + source_of(i, iw, f.W), scale, x, y, z);
+    display_rgb(x, y, z, M, exposure, gamma, rgb + 3 * (size_t)p);
+  }
+}
+
+// color_rays at render resolution: the colours that the image repeats
+__global__ void k_frame_rgb(const Film f, const float *__restrict__ cmf, double scale, const __grid_constant__ ColorMatrix M,
+                            float exposure, float gamma, float *__restrict__ rgb) {
+  __shared__ double cmf64[3 * kMaxBands];
+  load_cmf(cmf, f.B, cmf64);
+  const int npix = f.W * f.H;
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
+    float x, y, z;
+    pixel_xyz(f, cmf64, npix, p, scale, x, y, z);
+    display_rgb(x, y, z, M, exposure, gamma, rgb + 3 * (size_t)p);
+  }
+}
+
+// nearest-neighbour upscale, a row of the image per block row
+__global__ void k_upscale(const float *__restrict__ src, int W, int H, int iw, int ih, float *__restrict__ dst) {
+  for (int j = blockIdx.y; j < ih; j += gridDim.y) {
+    const float *row = src + 3 * (size_t)source_of(j, ih, H) * W;
+    float *out = dst + 3 * (size_t)j * iw;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < iw; i += gridDim.x * blockDim.x) {
+      const float *s = row + 3 * (size_t)source_of(i, iw, W);
+      const float r = s[0], g = s[1], b = s[2];
+      float *o = out + 3 * (size_t)i;
+      o[0] = r;
+      o[1] = g;
+      o[2] = b;
     }
   }
 }
@@ -137,9 +195,18 @@ cudaError_t launch_resolve_xyz(Film f, const float *cmf, double scale, float *xy
   k_resolve_xyz<<<grid_for((size_t)f.W * f.H), kThreads, 0, st>>>(f, cmf, scale, xyz);
   return cudaGetLastError();
 }
-cudaError_t launch_resolve_rgb(Film f, const float *cmf, double scale, const float *M, float exposure, float gamma,
-                               int iw, int ih, float *rgb, cudaStream_t st) {
-  k_resolve_rgb<<<grid_for((size_t)iw * ih), kThreads, 0, st>>>(f, cmf, scale, M, exposure, gamma, iw, ih, rgb);
+cudaError_t launch_resolve_rgb(Film f, const float *cmf, double scale, float *frame_rgb, ColorMatrix M, float exposure,
+                               float gamma, int iw, int ih, float *rgb, cudaStream_t st) {
+  // An image of at least the frame's pixels repeats them: each is resolved and
+  // tone-mapped once, then copied.  1024^2 frame, 1600^2 image: 135 us when every
+  // image pixel read the film and took its own powers, 59 us so.
+  if ((int64_t)iw * ih >= (int64_t)f.W * f.H) {
+    k_frame_rgb<<<grid_for((size_t)f.W * f.H), kThreads, 0, st>>>(f, cmf, scale, M, exposure, gamma, frame_rgb);
+    const dim3 grid((unsigned)((iw - 1) / kThreads + 1), (unsigned)std::min(ih, 65535));
+    k_upscale<<<grid, kThreads, 0, st>>>(frame_rgb, f.W, f.H, iw, ih, rgb);
+  } else {
+    k_resolve_rgb<<<grid_for((size_t)iw * ih), kThreads, 0, st>>>(f, cmf, scale, M, exposure, gamma, iw, ih, rgb);
+  }
   return cudaGetLastError();
 }
 cudaError_t launch_render_normals(const DevScene &s, const DevConfig &c, float *out, uint32_t *err,

@@ -34,8 +34,12 @@ cudaError_t launch_trace_batch(const DevScene &s, float eps, const float *rays, 
 cudaError_t launch_accumulate_block(Film f, int num_blocks_completed, cudaStream_t st);
 cudaError_t launch_clear_film(Film f, cudaStream_t st);
 cudaError_t launch_resolve_xyz(Film f, const float *cmf, double scale, float *xyz, cudaStream_t st);
-cudaError_t launch_resolve_rgb(Film f, const float *cmf, double scale, const float *xyz_to_rgb, float exposure,
-                               float gamma, int img_w, int img_h, float *rgb, cudaStream_t st);
+struct ColorMatrix {
+  float m[9];  // XYZ -> RGB, row-major
+};
+// frame_rgb: [H][W][3] scratch
+cudaError_t launch_resolve_rgb(Film f, const float *cmf, double scale, float *frame_rgb, ColorMatrix xyz_to_rgb,
+                               float exposure, float gamma, int img_w, int img_h, float *rgb, cudaStream_t st);
 cudaError_t launch_render_normals(const DevScene &s, const DevConfig &c, float *out, uint32_t *err,
                                   cudaStream_t st);
 
