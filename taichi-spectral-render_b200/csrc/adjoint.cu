@@ -205,8 +205,14 @@ __device__ void grad_surface(const DevScene &s, const DevConfig &c, int pmat, co
 
 namespace {
 
+// Replay 1 in blocks of 256 whose warps go through a vertex together (kTogether):
+// its 200 KB of code do not fit the instruction caches, and warps that each stood
+// elsewhere in it waited 14 of 22 cycles per instruction for the next.  Volume scene
+// 256^2, 25 passes: forward and adjoint 285 ms apart, 207 / 206 / 210 ms together in
+// blocks of 128 / 256 / 512.  Replay 0 has half the code and loses 2 % by it.
+constexpr int kAdjBlock = 256;
 template <int W, int kPhase>
-__global__ void __launch_bounds__(128, kPhase ? 4 : 5) k_adjoint(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass0, int npass, int band0,
+__global__ void __launch_bounds__(kPhase ? kAdjBlock : 128, kPhase ? 512 / kAdjBlock : 5) k_adjoint(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass0, int npass, int band0,
                                                  const double *__restrict__ adj, double *__restrict__ grad,
                                                  float *__restrict__ weight, int pm_shared, int pmat,
                                                  int *__restrict__ counter, uint32_t *__restrict__ err,
@@ -225,6 +231,7 @@ __global__ void __launch_bounds__(128, kPhase ? 4 : 5) k_adjoint(const __grid_co
   int band = 0;
   bool exhausted = false;
   constexpr bool phase = kPhase == 1;
+  constexpr bool kTogether = phase;
   int item = 0;
   PathState p;
   Rng rng;
@@ -270,23 +277,34 @@ __global__ void __launch_bounds__(128, kPhase ? 4 : 5) k_adjoint(const __grid_co
       }
     }
     // lanes that took a recorded item fetch again; stop when every lane is idle and out of items
-    if (__ballot_sync(0xffffffffu, pix >= 0 || !exhausted) == 0) break;
-    if (pix < 0) continue;
+    if (kTogether ? __syncthreads_or(pix >= 0 || !exhausted) == 0
+                  : __ballot_sync(0xffffffffu, pix >= 0 || !exhausted) == 0)
+      break;
+    if (!kTogether && pix < 0) continue;
+    const bool run = pix >= 0;
 
     // ---- one path vertex, exactly as the forward megakernel takes it
-    bool done = false;
-    rng.fill();
-    const Hit h = trace_closest<W, false>(s, p.pos, p.dir, c.eps, errbits, nullptr, c.escape);
-    const VolEvent ev = volume_event(s, c, p, h, rng);
-    if (ev.travel < 0.f) {
-      done = true;
-    } else {
+    bool done = false, alive = false, nee = false, emitter = false;
+    float indirect = 0.f, direct = 0.f, ew = 0.f, epl = 0.f, tsh = 0.f;
+    int nseg = 0;
+    VolEvent ev;
+    ShadowQuery q;
+    Hit h;
+    if (run) {
+      rng.fill();
+      h = trace_closest<W, false>(s, p.pos, p.dir, c.eps, errbits, nullptr, c.escape);
+    }
+    if (kTogether) __syncthreads();
+    if (run) {
+      ev = volume_event(s, c, p, h, rng);
+      alive = ev.travel >= 0.f;
+      done = !alive;
+    }
+    if (alive) {
       p.pos = p.pos + p.dir * ev.travel;
       if (phase) grad_volume(s, c, pmat, p, ev, arem, g);
       p.thr *= ev.est;
-      float indirect = 0.f, direct = 0.f, ew = 0.f, epl = 0.f;
-      bool nee = false, emitter = false;
-      ShadowQuery q;
+      int surf = -1;
       if (ev.action == 1) {
         const Mat sm = get_mat(s, B, ev.hit_mat, band);
         if (sm.surf_emis) {
@@ -294,39 +312,40 @@ __global__ void __launch_bounds__(128, kPhase ? 4 : 5) k_adjoint(const __grid_co
           emitter = true;
           done = true;
         } else {
-          nee = nee_setup(s, c, p, band, ev.snormal, ev.hit_mat, rng, q);
-        }
-      } else {
-        nee = nee_setup(s, c, p, band, ev.snormal, -1, rng, q);
-      }
-      int nseg = 0;
-      float tsh = 0.f;
-      if (nee) {
-        ShadowState ss;
-        ss.pos = q.origin;
-        ss.total = 1.f;
-        ss.traveled = 0.f;
-        ss.vol = q.vol;
-        ss.seg = 0;
-        for (;;) {
-          // the gradient replay needs true segment lengths even where the forward
-          // pass could stop at the light (non-attenuating media): no bound there
-          const Hit sh = trace_closest<W, false>(s, ss.pos, q.dir, c.eps, errbits, nullptr,
-                                                 phase ? 1e9f : shadow_bound(s, c, q, ss, p.active));
-          if (phase && nseg < kAdjMaxSeg) {
-            const float left = q.max_dist - ss.traveled;
-            const bool reach = sh.t >= left || sh.slot == q.light_slot;
-            seg_m[nseg] = ss.vol;
-            seg_l[nseg] = reach ? sh.t + left : sh.t;
-            ++nseg;
-          }
-          if (shadow_segment(s, c, q, sh, p.active, ss)) break;
-        }
-        if (ss.total > 1e-6f) {
-          tsh = ss.total;
-          direct = q.contrib * ss.total;
+          surf = ev.hit_mat;
         }
       }
+      if (!done) nee = nee_setup(s, c, p, band, ev.snormal, surf, rng, q);
+    }
+    if (kTogether) __syncthreads();
+    if (nee) {
+      ShadowState ss;
+      ss.pos = q.origin;
+      ss.total = 1.f;
+      ss.traveled = 0.f;
+      ss.vol = q.vol;
+      ss.seg = 0;
+      for (;;) {
+        // the gradient replay needs true segment lengths even where the forward
+        // pass could stop at the light (non-attenuating media): no bound there
+        const Hit sh = trace_closest<W, false>(s, ss.pos, q.dir, c.eps, errbits, nullptr,
+                                               phase ? 1e9f : shadow_bound(s, c, q, ss, p.active));
+        if (phase && nseg < kAdjMaxSeg) {
+          const float left = q.max_dist - ss.traveled;
+          const bool reach = sh.t >= left || sh.slot == q.light_slot;
+          seg_m[nseg] = ss.vol;
+          seg_l[nseg] = reach ? sh.t + left : sh.t;
+          ++nseg;
+        }
+        if (shadow_segment(s, c, q, sh, p.active, ss)) break;
+      }
+      if (ss.total > 1e-6f) {
+        tsh = ss.total;
+        direct = q.contrib * ss.total;
+      }
+    }
+    if (kTogether) __syncthreads();
+    if (alive) {
       // deposits of this vertex go to the band the path carries after it
       const int bdep = ev.action == 3 ? ev.new_wl : p.active_px;
       const float w = (float)__ldg(adj + (size_t)bdep * npix + pix);
@@ -375,9 +394,14 @@ __global__ void __launch_bounds__(128, kPhase ? 4 : 5) k_adjoint(const __grid_co
         arem -= w * indirect;
         arem -= w * direct;
       }
+    }
+    if (kTogether) __syncthreads();
+    SurfEvent se;
+    if (alive && ev.action == 1 && !done) se = scatter_surface(s, c, p, ev, rng);
+    if (kTogether) __syncthreads();
+    if (alive) {
       if (ev.action == 1 && !done) {
         p.plen++;
-        const SurfEvent se = scatter_surface(s, c, p, ev, rng);
         if (phase) grad_surface(s, c, pmat, p, ev, se, arem, g, sp);
         apply_surface(c, p, ev, se);
       } else if (ev.action == 2) {
@@ -413,7 +437,7 @@ void launch_pair(const DevScene &s, const DevConfig &c, uint32_t pass, int npass
                  cudaStream_t st, const float *rec) {
   const int block = 128;
   k_adjoint<W, 0><<<grid, block, 0, st>>>(s, c, pass, npass, band, adj, grad, weight, 0, pmat, counter, err, rec);
-  k_adjoint<W, 1><<<grid, block, (size_t)psh * sizeof(double), st>>>(s, c, pass, npass, band, adj, grad, weight, psh,
+  k_adjoint<W, 1><<<grid * 128 / kAdjBlock, kAdjBlock, (size_t)psh * sizeof(double), st>>>(s, c, pass, npass, band, adj, grad, weight, psh,
                                                                      pmat, counter + 1, err, nullptr);
 }
 }  // namespace

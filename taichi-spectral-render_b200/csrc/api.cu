@@ -945,6 +945,7 @@ struct ts_batch {
   size_t wave_bytes = 0;
   ts::BatchLoopGraph *loop = nullptr;
   int loop_cap = 0, loop_limit = 0;
+  bool together = true;  // every scene is small enough for mega_vertex's warps together
   std::string err;
 };
 
@@ -1041,6 +1042,7 @@ ts_status ts_batch_create(const ts_batch_config *cfg, ts_ctx *const *ctxs, int32
     sl.c = b->ctxs[k]->dc;
     sl.f = film_of(b->ctxs[k]);
     sl.active = 1;
+    b->together = b->together && sl.s.num_tris <= ts::kTogetherTris;
   }
   cudaError_t e = cudaMalloc((void **)&b->d_slots, sizeof(ts::BatchSlot) * n);
   if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_hdr, sizeof(ts::BatchHeader));
@@ -1131,14 +1133,14 @@ ts_status ts_batch_step(ts_batch *b, void *stream) {
   }
   if (!b->cfg.use_graph) {
     TS_BCUDA(b, ts::launch_batch_step(b->d_slots, b->n, b->d_hdr, b->d_active, b->d_err, b->width, grid,
-                                      b->cfg.block_size, acc_blocks, as_stream(stream), b->cfg.occupancy),
+                                      b->cfg.block_size, acc_blocks, as_stream(stream), b->cfg.occupancy, b->together),
              "ts_batch_step");
     return TS_OK;
   }
   if (!b->exec) {
     TS_BCUDA(b, cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal), "ts_batch_step: capture");
     const cudaError_t le = ts::launch_batch_step(b->d_slots, b->n, b->d_hdr, b->d_active, b->d_err, b->width, grid,
-                                                 b->cfg.block_size, acc_blocks, b->cap, b->cfg.occupancy);
+                                                 b->cfg.block_size, acc_blocks, b->cap, b->cfg.occupancy, b->together);
     const cudaError_t ce = cudaStreamEndCapture(b->cap, &b->graph);
     TS_BCUDA(b, le, "ts_batch_step: capture");
     TS_BCUDA(b, ce, "ts_batch_step: capture");

@@ -57,8 +57,8 @@ cudaError_t launch_batch_loop_step(BatchSlot *slots, int n, BatchHeader *h, cons
                                    int limit, int acc_blocks, cudaStream_t st, BatchLoopGraph **graph, bool use_graph);
 void free_batch_loop(BatchLoopGraph *g);
 cudaError_t batch_set_smem_limit(int n);
-// one step: prepare (item ranges), render (persistent pool), accumulate, advance
+// one step: prepare (item ranges), render (persistent pool), accumulate, advance; together: mega_vertex's
 cudaError_t launch_batch_step(BatchSlot *slots, int n, BatchHeader *h, const int *active, uint32_t *err, int width,
-                              int grid, int block, int acc_blocks, cudaStream_t st, int occupancy);
+                              int grid, int block, int acc_blocks, cudaStream_t st, int occupancy, bool together);
 
 }  // namespace ts

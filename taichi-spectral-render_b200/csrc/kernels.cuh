@@ -20,6 +20,9 @@ struct Film {
   float *rec = nullptr;
 };
 
+// largest scene whose vertices a block's warps take together (mega_path.cuh)
+constexpr int kTogetherTris = 32768;
+
 // npass consecutive sample passes (cast_rays) from pass / band, band wrapping
 // mod B (npass <= B): persistent megakernel with per-lane path regeneration.
 // work != nullptr selects the counting variant (work[8], accumulated)

@@ -55,59 +55,75 @@ __device__ __forceinline__ void mega_start(const DevScene &s, const DevConfig &c
   L.dep = 0.0;
 }
 
-// Returns true when the path has ended (its deposit flushed).
-template <int W, bool kCount, bool kTogether = true>
-__device__ __forceinline__ bool mega_vertex(const DevScene &s, const DevConfig &c, const Film &f, MegaLane &L,
+// One vertex of every lane of the block that has a path (L.pix >= 0); a path that
+// has ended is flushed and its lane idle.
+// kTogether: the warps of the block go through the vertex together.  Its code
+// (100 KB) does not fit the instruction caches, and warps that each stand
+// elsewhere in it wait for instructions more than for anything else.
+// kStep: the traversal's lanes step together (trace_closest).
+template <int W, bool kCount, bool kTogether, bool kStep>
+__device__ __forceinline__ void mega_vertex(const DevScene &s, const DevConfig &c, const Film &f, MegaLane &L,
                                             uint32_t &errbits, MegaCounts &cnt, bool shared) {
   PathState &p = L.p;
   const int band = L.band;
-  bool done = false;
-  L.rng.fill();
-  // hits beyond ESCAPE count as escapes (main.py:1209-1214): traverse no further
-  const Hit h = trace_closest<W, kCount, kTogether>(s, p.pos, p.dir, c.eps, errbits, &cnt.tc, c.escape);
-  const VolEvent ev = volume_event(s, c, p, h, L.rng);
-  if (kCount) {
-    cnt.trace++;
-    cnt.hit += h.slot >= 0;
+  const bool run = L.pix >= 0;
+  bool done = false, alive = false, nee = false;
+  float indirect = 0.f, direct = 0.f;
+  Hit h;
+  VolEvent ev;
+  ShadowQuery q;
+  if (run) {
+    L.rng.fill();
+    // hits beyond ESCAPE count as escapes (main.py:1209-1214): traverse no further
+    h = trace_closest<W, kCount, kStep>(s, p.pos, p.dir, c.eps, errbits, &cnt.tc, c.escape);
   }
-  if (ev.travel < 0.f) {
-    done = true;  // escaped
-  } else {
+  if (kTogether) __syncthreads();
+  if (run) {
+    ev = volume_event(s, c, p, h, L.rng);
+    if (kCount) {
+      cnt.trace++;
+      cnt.hit += h.slot >= 0;
+    }
+    alive = ev.travel >= 0.f;
+    done = !alive;  // escaped
+  }
+  if (alive) {
     if (kCount) cnt.vert++;
     p.pos = p.pos + p.dir * ev.travel;
     p.thr *= ev.est;
-    float indirect = 0.f, direct = 0.f;
-    bool nee = false;
-    ShadowQuery q;
+    int surf = -1;
     if (ev.action == 1) {
       const Mat sm = get_mat(s, c.B, ev.hit_mat, band);
       if (sm.surf_emis) {
         indirect = emitter_hit(s, c, p, ev, sm.emission);
         done = true;
       } else {
-        nee = nee_setup(s, c, p, band, ev.snormal, ev.hit_mat, L.rng, q);
+        surf = ev.hit_mat;
       }
-    } else {
-      nee = nee_setup(s, c, p, band, ev.snormal, -1, L.rng, q);
     }
-    if (nee) {
-      ShadowState ss;
-      ss.pos = q.origin;
-      ss.total = 1.f;
-      ss.traveled = 0.f;
-      ss.vol = q.vol;
-      ss.seg = 0;
-      for (;;) {
-        const Hit sh =
-            trace_closest<W, kCount, kTogether>(s, ss.pos, q.dir, c.eps, errbits, &cnt.tc, shadow_bound(s, c, q, ss, p.active));
-        if (kCount) {
-          cnt.trace++;
-          cnt.hit += sh.slot >= 0 && sh.slot != q.light_slot;
-        }
-        if (shadow_segment(s, c, q, sh, p.active, ss)) break;
+    if (!done) nee = nee_setup(s, c, p, band, ev.snormal, surf, L.rng, q);
+  }
+  if (kTogether) __syncthreads();
+  if (nee) {
+    ShadowState ss;
+    ss.pos = q.origin;
+    ss.total = 1.f;
+    ss.traveled = 0.f;
+    ss.vol = q.vol;
+    ss.seg = 0;
+    for (;;) {
+      const Hit sh = trace_closest<W, kCount, kStep>(s, ss.pos, q.dir, c.eps, errbits, &cnt.tc,
+                                              shadow_bound(s, c, q, ss, p.active));
+      if (kCount) {
+        cnt.trace++;
+        cnt.hit += sh.slot >= 0 && sh.slot != q.light_slot;
       }
-      if (ss.total > 1e-6f) direct = q.contrib * ss.total;
+      if (shadow_segment(s, c, q, sh, p.active, ss)) break;
     }
+    if (ss.total > 1e-6f) direct = q.contrib * ss.total;
+  }
+  if (kTogether) __syncthreads();
+  if (alive) {
     if (ev.action == 1 && !done) {
       p.plen++;
       const SurfEvent se = scatter_surface(s, c, p, ev, L.rng);
@@ -138,7 +154,6 @@ __device__ __forceinline__ bool mega_vertex(const DevScene &s, const DevConfig &
     if (f.rec) f.rec[L.item] = L.moved ? -1.0f : (float)L.dep;
     L.pix = -1;
   }
-  return done;
 }
 
 }  // namespace ts

@@ -34,7 +34,8 @@ __global__ void k_batch_prepare(BatchSlot *slots, int n, BatchHeader *h, const i
   h->counter = 0;
 }
 
-template <int W, int kMinBlocks = 5>
+// kTogether: the block's warps take each vertex together (mega_vertex)
+template <int W, int kMinBlocks, bool kTogether>
 __global__ void __launch_bounds__(128, kMinBlocks) k_render_batch(const BatchSlot *__restrict__ slots, int n,
                                                       BatchHeader *__restrict__ h, uint32_t *__restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -78,10 +79,9 @@ __global__ void __launch_bounds__(128, kMinBlocks) k_render_batch(const BatchSlo
         }
       }
     }
-    if (__ballot_sync(0xffffffffu, L.pix >= 0) == 0) break;
-    if (L.pix < 0) continue;
+    if (kTogether ? __syncthreads_or(L.pix >= 0) == 0 : __ballot_sync(0xffffffffu, L.pix >= 0) == 0) break;
     const BatchSlot &sl = sh[slot];
-    mega_vertex<W, false>(sl.s, sl.c, sl.f, L, errbits, cnt, true);
+    mega_vertex<W, false, kTogether, true>(sl.s, sl.c, sl.f, L, errbits, cnt, true);
   }
   if (errbits) atomicOr(err, errbits);
 }
@@ -115,24 +115,26 @@ __global__ void k_batch_advance(BatchSlot *slots, int n) {
 size_t batch_smem_bytes(int n) { return (size_t)n * sizeof(BatchSlot); }
 
 namespace {
-template <int kMin>
-void launch_render_batch(BatchSlot *slots, int n, BatchHeader *h, uint32_t *err, int width, int grid, int block,
-                         size_t smem, cudaStream_t st) {
-  if (width == 9) k_render_batch<9, kMin><<<grid, block, smem, st>>>(slots, n, h, err);
-  else if (width == 5) k_render_batch<5, kMin><<<grid, block, smem, st>>>(slots, n, h, err);
-  else if (width == 8) k_render_batch<8, kMin><<<grid, block, smem, st>>>(slots, n, h, err);
-  else if (width == 4) k_render_batch<4, kMin><<<grid, block, smem, st>>>(slots, n, h, err);
-  else k_render_batch<2, kMin><<<grid, block, smem, st>>>(slots, n, h, err);
+template <int W>
+auto batch_kernel(int occupancy, bool together) {
+  if (occupancy >= 8) return together ? k_render_batch<W, 8, true> : k_render_batch<W, 8, false>;
+  return together ? k_render_batch<W, 5, true> : k_render_batch<W, 5, false>;
+}
+auto batch_kernel(int width, int occupancy, bool together) {
+  return width == 9   ? batch_kernel<9>(occupancy, together)
+         : width == 5 ? batch_kernel<5>(occupancy, together)
+         : width == 8 ? batch_kernel<8>(occupancy, together)
+         : width == 4 ? batch_kernel<4>(occupancy, together)
+                      : batch_kernel<2>(occupancy, together);
 }
 }  // namespace
 
 cudaError_t launch_batch_step(BatchSlot *slots, int n, BatchHeader *h, const int *active, uint32_t *err, int width,
-                              int grid, int block, int acc_blocks, cudaStream_t st, int occupancy) {
+                              int grid, int block, int acc_blocks, cudaStream_t st, int occupancy, bool together) {
   k_batch_prepare<<<1, 32, 0, st>>>(slots, n, h, active);
   const size_t smem = batch_smem_bytes(n);
   block = block > 128 ? 128 : block;
-  if (occupancy >= 8) launch_render_batch<8>(slots, n, h, err, width, grid, block, smem, st);
-  else launch_render_batch<5>(slots, n, h, err, width, grid, block, smem, st);
+  batch_kernel(width, occupancy, together)<<<grid, block, smem, st>>>(slots, n, h, err);
   k_batch_accumulate<<<dim3(acc_blocks, n), 256, 0, st>>>(slots);
   k_batch_advance<<<(n + 127) / 128, 128, 0, st>>>(slots, n);
   return cudaGetLastError();
@@ -151,20 +153,14 @@ cudaError_t launch_batch_finish(BatchSlot *slots, int n, int acc_blocks, cudaStr
 
 cudaError_t batch_set_smem_limit(int n) {
   const int bytes = (int)batch_smem_bytes(n);
-  cudaError_t e = cudaSuccess;
-  for (cudaError_t r :
-       {cudaFuncSetAttribute(k_render_batch<2, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-        cudaFuncSetAttribute(k_render_batch<4, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-        cudaFuncSetAttribute(k_render_batch<8, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-        cudaFuncSetAttribute(k_render_batch<5, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-        cudaFuncSetAttribute(k_render_batch<9, 5>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-        cudaFuncSetAttribute(k_render_batch<5, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-        cudaFuncSetAttribute(k_render_batch<9, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-        cudaFuncSetAttribute(k_render_batch<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-        cudaFuncSetAttribute(k_render_batch<4, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-        cudaFuncSetAttribute(k_render_batch<8, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)})
-    if (r != cudaSuccess) e = r;
-  return e;
+  for (int width : {2, 4, 5, 8, 9})
+    for (int occupancy : {0, 8})
+      for (bool together : {false, true}) {
+        const cudaError_t e = cudaFuncSetAttribute(batch_kernel(width, occupancy, together),
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
+      }
+  return cudaSuccess;
 }
 
 }  // namespace ts

@@ -21,7 +21,8 @@ namespace {
 // kMinBlocks: resident blocks of 128 threads per SM the compiler must allow
 // (5: 96 registers, no spills; 8: 64 registers with local-memory spills --
 // more warps to hide the node-fetch latency, faster on large frames).
-template <int W, bool kCount, int kMinBlocks = 5>
+// kTogether: the block's warps take each vertex together (mega_vertex).
+template <int W, bool kCount, int kMinBlocks = 5, bool kTogether = false>
 __global__ void __launch_bounds__(128, kMinBlocks) k_render_mega(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass0, int npass, int band0,
                                                      Film f, int *__restrict__ counter, uint32_t *__restrict__ err,
                                                      unsigned long long *__restrict__ work) {
@@ -54,9 +55,8 @@ __global__ void __launch_bounds__(128, kMinBlocks) k_render_mega(const __grid_co
         }
       }
     }
-    if (__ballot_sync(0xffffffffu, L.pix >= 0) == 0) break;
-    if (L.pix < 0) continue;
-    mega_vertex<W, kCount, false>(s, c, f, L, errbits, cnt, npass > 1);
+    if (kTogether ? __syncthreads_or(L.pix >= 0) == 0 : __ballot_sync(0xffffffffu, L.pix >= 0) == 0) break;
+    mega_vertex<W, kCount, kTogether, false>(s, c, f, L, errbits, cnt, npass > 1);
   }
   if (errbits) atomicOr(err, errbits);
   if (kCount) {
@@ -73,10 +73,16 @@ __global__ void __launch_bounds__(128, kMinBlocks) k_render_mega(const __grid_co
 template <int W>
 void launch_w(const DevScene &s, const DevConfig &c, uint32_t pass0, int npass, int band0, Film f, int *counter,
               uint32_t *err, int grid, int block, cudaStream_t st, unsigned long long *work, int occupancy) {
-  if (work) k_render_mega<W, true><<<grid, block, 0, st>>>(s, c, pass0, npass, band0, f, counter, err, work);
-  else if (occupancy >= 8)
-    k_render_mega<W, false, 8><<<grid, block, 0, st>>>(s, c, pass0, npass, band0, f, counter, err, nullptr);
-  else k_render_mega<W, false><<<grid, block, 0, st>>>(s, c, pass0, npass, band0, f, counter, err, nullptr);
+  // Together where shading, not the length of single traversals, takes the time:
+  // small trees and enough paths.  ms per pass apart / together: box (2,062
+  // triangles) 64^2 0.50 / 0.55, 128^2 0.55 / 0.59, 256^2 0.77 / 0.67, 512^2 1.57 / 1.20,
+  // bundles of 25 passes at 512^2 1.23 / 0.92; volume (20,014) 256^2 4.87 / 4.74,
+  // bundle 2.57 / 2.52; terrain (647,258) 256^2 0.57 / 0.59, 512^2 0.76 / 0.83.
+  const bool together = s.num_tris <= kTogetherTris && (int64_t)c.W * c.H * npass >= 65536;
+  const auto k = work          ? k_render_mega<W, true>
+                 : occupancy >= 8 ? (together ? k_render_mega<W, false, 8, true> : k_render_mega<W, false, 8>)
+                                  : (together ? k_render_mega<W, false, 5, true> : k_render_mega<W, false>);
+  k<<<grid, block, 0, st>>>(s, c, pass0, npass, band0, f, counter, err, work);
 }
 
 }  // namespace
