@@ -11,6 +11,9 @@ namespace ts {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kSMs = 148;
+constexpr int kTied = -2;               // tri_orig of a ray that k_trace_batch_ties decides
+constexpr int kGroupRays = 148 * 1024;  // largest query with a group of lanes per ray
 
 inline int grid_for(size_t n) {
   size_t g = (n + kThreads - 1) / kThreads;
@@ -164,15 +167,119 @@ __global__ void k_normals(const __grid_constant__ DevScene s, const __grid_const
   if (eb) atomicOr(err, eb);
 }
 
-template <int kMode, int W>
+// the reference-order query
 __global__ void k_trace_batch(const __grid_constant__ DevScene s, float eps, const float *__restrict__ rays, int n,
                               int32_t *__restrict__ tri_orig, float *__restrict__ t, float *__restrict__ u,
                               float *__restrict__ v, uint32_t *err) {
   uint32_t eb = 0;
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     const float *q = rays + 6 * (size_t)r;
-    const float3 o = f3(q[0], q[1], q[2]), d = f3(q[3], q[4], q[5]);
-    const Hit h = kMode == 0 ? trace_closest<W>(s, o, d, eps, eb) : trace_reference_order(s, o, d, eps, eb);
+    const Hit h = trace_reference_order(s, f3(q[0], q[1], q[2]), f3(q[3], q[4], q[5]), eps, eb);
+    tri_orig[r] = h.slot >= 0 ? __float_as_int(__ldg(s.tri + 3 * (size_t)h.slot).w) : -1;
+    t[r] = h.t;
+    if (u) u[r] = h.u;
+    if (v) v[r] = h.v;
+  }
+  if (eb) atomicOr(err, eb);
+}
+
+// The fast query with a ray per lane: a warp has `chunk` consecutive rays, and the
+// lanes whose rays have ended take the next of them once 16 wait (one look every
+// four phases), so that it does not idle behind its longest ray.
+template <int W>
+__global__ void __launch_bounds__(kThreads, 4) k_trace_batch_lanes(const __grid_constant__ DevScene s, float eps,
+                                                                   const float *__restrict__ rays, int n, int chunk,
+                                                                   int32_t *__restrict__ tri_orig,
+                                                                   float *__restrict__ t, float *__restrict__ u,
+                                                                   float *__restrict__ v, uint32_t *err) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  int next = (int)min((int64_t)n, warp * chunk);
+  const int end = (int)min((int64_t)n, (warp + 1) * chunk);
+  uint32_t eb = 0;
+  Traversal g;
+  g.node = kTravDone;
+  g.tie = 0;
+  int2 stack[kWideStack];
+  int r = -1;  // this lane's ray
+  for (;;) {
+    const bool done = g.node == kTravDone;
+    const unsigned idle = __ballot_sync(kFull, done && (r >= 0 || next < end));
+    if (__popc(idle) >= 16 || __ballot_sync(kFull, !done) == 0) {
+      if (done && r >= 0) {
+        tri_orig[r] = trav_tied<W>(g)    ? kTied
+                      : g.h.slot >= 0 ? __float_as_int(__ldg(s.tri + 3 * (size_t)g.h.slot).w)
+                                      : -1;
+        t[r] = g.h.t;
+        if (u) u[r] = g.h.u;
+        if (v) v[r] = g.h.v;
+        r = -1;
+      }
+      __syncwarp();
+      const unsigned want = __ballot_sync(kFull, r < 0);
+      const int mine = next + __popc(want & ((1u << lane) - 1u));
+      if (r < 0 && mine < end) {
+        r = mine;
+        const float *q = rays + 6 * (size_t)r;
+        trav_begin<W>(s, g, f3(q[0], q[1], q[2]), f3(q[3], q[4], q[5]), 1e9f);
+      }
+      next = min(end, next + __popc(want));
+      if (__ballot_sync(kFull, r >= 0) == 0) break;
+    }
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i)
+      if (!warp_phase<Nodes<W>::value>(s, g, stack, eps, eb)) break;
+  }
+  if (eb) atomicOr(err, eb);
+}
+
+// the rays whose hit a tie left open (two-child layout)
+__global__ void k_trace_batch_ties(const __grid_constant__ DevScene s, float eps, const float *__restrict__ rays, int n,
+                                   int32_t *__restrict__ tri_orig, float *__restrict__ t, float *__restrict__ u,
+                                   float *__restrict__ v, uint32_t *err) {
+  uint32_t eb = 0;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+    if (tri_orig[r] != kTied) continue;
+    const float *q = rays + 6 * (size_t)r;
+    const Hit h = trace_plain<2>(s, f3(q[0], q[1], q[2]), f3(q[3], q[4], q[5]), eps, eb, 1e9f);
+    tri_orig[r] = h.slot >= 0 ? __float_as_int(__ldg(s.tri + 3 * (size_t)h.slot).w) : -1;
+    t[r] = h.t;
+    if (u) u[r] = h.u;
+    if (v) v[r] = h.v;
+  }
+  if (eb) atomicOr(err, eb);
+}
+
+// The fast query with a group of lanes per ray, `share` rays to a warp
+template <int W>
+__global__ void __launch_bounds__(kThreads, 2) k_trace_batch_groups(const __grid_constant__ DevScene s, float eps,
+                                                                    const float *__restrict__ rays, int n, int share,
+                                                                    int32_t *__restrict__ tri_orig,
+                                                                    float *__restrict__ t, float *__restrict__ u,
+                                                                    float *__restrict__ v, uint32_t *err) {
+  constexpr int G = W == 8 ? 8 : 4;
+  __shared__ int2 stacks[kGroupStack * (kThreads / G)];
+  const int lane = threadIdx.x & 31, sub = lane & (G - 1), shift = lane & ~(G - 1);
+  const int warp = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  const int64_t r = (int64_t)warp * share + lane / G;
+  const bool active = lane / G < share && r < n;
+  uint32_t eb = 0;
+  GroupRay<G> g;
+  float3 o = f3(0.f, 0.f, 0.f), d = o;
+  if (active) {
+    const float *q = rays + 6 * (size_t)r;
+    o = f3(q[0], q[1], q[2]);
+    d = f3(q[3], q[4], q[5]);
+  }
+  group_begin(s, g, o, d, 1e9f);
+  if (!active) g.node = kTravDone;
+  while (__any_sync(0xffffffffu, g.node != kTravDone))
+    group_step(s, g, stacks + threadIdx.x / G, kThreads / G, sub, shift, eps);
+  Hit h;
+  const bool good = group_hit(g, shift, h);
+  if (active && sub == 0) {
+    if (!good) h = trace_plain<W>(s, o, d, eps, eb, 1e9f);
     tri_orig[r] = h.slot >= 0 ? __float_as_int(__ldg(s.tri + 3 * (size_t)h.slot).w) : -1;
     t[r] = h.t;
     if (u) u[r] = h.u;
@@ -222,13 +329,33 @@ cudaError_t launch_render_normals(const DevScene &s, const DevConfig &c, float *
 cudaError_t launch_trace_batch(const DevScene &s, float eps, const float *rays, int n, int mode, int32_t *tri_orig,
                                float *t, float *u, float *v, uint32_t *err, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  const int g = grid_for((size_t)n);
-  if (mode != 0) k_trace_batch<1, 2><<<g, kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v, err);
-  else if (s.node_width == 9) k_trace_batch<0, 9><<<g, kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v, err);
-  else if (s.node_width == 5) k_trace_batch<0, 5><<<g, kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v, err);
-  else if (s.node_width == 8) k_trace_batch<0, 8><<<g, kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v, err);
-  else if (s.node_width == 4) k_trace_batch<0, 4><<<g, kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v, err);
-  else k_trace_batch<0, 2><<<g, kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v, err);
+  if (mode != 0) {
+    k_trace_batch<<<grid_for((size_t)n), kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v, err);
+    return cudaGetLastError();
+  }
+  // A group of lanes per ray while a ray per lane would leave the schedulers idle.
+  // us, lanes / groups: 2,062 triangles 16k rays 36 / 24, 128k 61 / 58, 256k 81 / 95;
+  // 2.6M triangles 16k 87 / 57, 128k 124 / 104, 256k 181 / 178, 512k 300 / 342.
+  if (n <= kGroupRays && s.node_width != 5 && s.node_width != 9) {
+    const int share = std::min(s.node_width == 8 ? 4 : 8, std::max(1, n / (kSMs * 16)));
+    const int warps = (n - 1) / share + 1;
+    const auto k = s.node_width == 8   ? k_trace_batch_groups<8>
+                   : s.node_width == 4 ? k_trace_batch_groups<4>
+                                       : k_trace_batch_groups<2>;
+    k<<<(warps - 1) / (kThreads / 32) + 1, kThreads, 0, st>>>(s, eps, rays, n, share, tri_orig, t, u, v, err);
+    return cudaGetLastError();
+  }
+  const int blocks = std::min(kSMs * 4, (n - 1) / kThreads + 1);
+  const int warps = blocks * (kThreads / 32);
+  const auto k = s.node_width == 9   ? k_trace_batch_lanes<9>
+                 : s.node_width == 5 ? k_trace_batch_lanes<5>
+                 : s.node_width == 8 ? k_trace_batch_lanes<8>
+                 : s.node_width == 4 ? k_trace_batch_lanes<4>
+                                     : k_trace_batch_lanes<2>;
+  k<<<blocks, kThreads, 0, st>>>(s, eps, rays, n, (n - 1) / warps + 1, tri_orig, t, u, v, err);
+  if (s.node_width == 2)
+    k_trace_batch_ties<<<std::min(kSMs * 8, (n - 1) / kThreads + 1), kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v,
+                                                                                        err);
   return cudaGetLastError();
 }
 

@@ -52,6 +52,7 @@ struct WaveLoop {
   int ext[2];     // extension queue lengths: queue[a] is traced at the iterations of parity a
   int sh[2];      // shadow queries appended by the shade of parity a
   int fetch[2];   // trace / shade work counters of the current iteration
+  int ties[2];    // shadow queries and extension rays that trace_lanes left to k_trace_ties
   int next_item;  // next work item (pass offset * npix + pixel) to start
   int total;      // work items of the launch
   int iter, limit;
@@ -72,8 +73,8 @@ struct WaveBuffers {
   float4 *sq_dir;     // dir.xyz, contrib
   int4 *sq_meta;      // (pixel, light_slot, vol, band)
   int *queue[2];      // extension queues (ping-pong), path ids
-  int *shadow_queue;  // shadow queue, query ids == path ids
-  int *sorted;        // extension queue ordered by material key (shading)
+  int *shadow_queue;  // shadow queries whose hit a tie left open
+  int *sorted;        // extension queue ordered by material key (shading); before, rays whose hit a tie left open
   int *trace_order;   // extension queue ordered by direction octant (tracing)
   int *shadow_order;  // shadow query indices ordered by light triangle
   int *counts;        // [2*max_depth + 8]: ext counts per depth, shadow counts per depth, scratch

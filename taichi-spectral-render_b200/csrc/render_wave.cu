@@ -35,7 +35,9 @@ constexpr int kCntExt = 0;                      // [kMaxDepth+1] extension queue
 constexpr int kCntSh = kCntExt + kMaxDepth + 1;  // [kMaxDepth+1] shadow queue lengths
 constexpr int kCntFetchT = kCntSh + kMaxDepth + 1;
 constexpr int kCntFetchS = kCntFetchT + kMaxDepth + 1;
-constexpr int kCntTotal = kCntFetchS + kMaxDepth + 1;
+constexpr int kCntTies = kCntFetchS + kMaxDepth + 1;  // [2 * (kMaxDepth+1)] ties left by trace_lanes
+constexpr int kCntTotal = kCntTies + 2 * (kMaxDepth + 1);
+static_assert(kCntTotal <= 8192, "WaveBuffers::counts");
 
 // ---- work fetching
 // The blocks of k_shade* and trace_groups are all resident (resident_grid: what the
@@ -127,6 +129,7 @@ struct TraceItems {
   const int *q;             // path slots of the extension rays
   const int *shadow_order;  // nullptr: queries in order
   int *fetch;
+  int *ties;                // [2] counts of the lists of tied queries (w.shadow_queue) and rays (w.sorted)
 };
 
 // what a work item renders: one scene, or a view of a batch
@@ -240,8 +243,8 @@ __device__ __forceinline__ void item_hit(const Src &src, const WaveBuffers &w, T
   }
 }
 
-// The whole work item through trace_plain(), outside the hot loop, whose
-// registers a call would spill; a shadow chain starts over, with the same hits.
+// The whole work item through trace_plain(); a shadow chain starts over, with the
+// same hits.
 template <int W>
 __device__ __noinline__ void item_plain(const DevScene &s, const DevConfig &c, const Film &f, const WaveBuffers &w,
                                         int id, bool shadow, bool shared, uint32_t &eb) {
@@ -260,21 +263,6 @@ __device__ __noinline__ void item_plain(const DevScene &s, const DevConfig &c, c
   if (ss.total > 1e-6f) deposit(f, pixel, dep_band, q.contrib * ss.total, shared);
 }
 
-// Items whose result a tie left open, once no lane of the warp has a ray; returns
-// false when the warp is out of work.
-template <int W, class Src>
-__device__ __forceinline__ bool run_plain(const Src &src, const WaveBuffers &w, TraceItem &im, bool writer,
-                                          bool exhausted, uint32_t &eb) {
-  if (im.id >= 0 && im.plain) {
-    if (writer)
-      item_plain<W>(src.scene(im.view), src.config(im.view), src.film(im.view), w, im.id, im.shadow,
-                    src.shared(im.view), eb);
-    im.id = -1;
-  }
-  im.plain = false;
-  return __ballot_sync(0xffffffffu, im.id >= 0 || !exhausted) != 0;
-}
-
 // A ray per lane.  A warp looks every kPhases phases for lanes that have
 // finished, and ends their items and starts others once kIdleLanes of them wait:
 // the end of a shadow segment is as long as three node tests, and when every
@@ -282,6 +270,8 @@ __device__ __forceinline__ bool run_plain(const Src &src, const WaveBuffers &w, 
 constexpr int kPhases = 4;      // 1: 5 % slower, 8: the same
 constexpr int kIdleLanes = 16;  // 4 / 8 / 12: 11 / 5 / 1 % slower, 20: 3 % slower on the volume
 
+// A tied item goes to a list (k_trace_ties): a call to trace_plain() in this
+// kernel, wherever it stood, cost the two-child layout 16 to 20 %.
 template <int W, class Src>
 __device__ __forceinline__ void trace_lanes(const Src &src, const WaveBuffers &w, const TraceItems &it,
                                             uint32_t &eb) {
@@ -292,26 +282,26 @@ __device__ __forceinline__ void trace_lanes(const Src &src, const WaveBuffers &w
   t.tie = 0;
   int2 stack[kWideStack];
   bool exhausted = false;
+  const auto begin = [&](const DevScene &s, float3 o, float3 d, float bound) { trav_begin<W>(s, t, o, d, bound); };
   for (;;) {
-    const bool done = t.node == kTravDone && !im.plain;
+    const bool done = t.node == kTravDone;
     const unsigned idle = __ballot_sync(kFull, done && !(exhausted && im.id < 0));
-    if (__popc(idle) >= kIdleLanes || __ballot_sync(kFull, t.node != kTravDone) == 0) {
-      const auto begin = [&](const DevScene &s, float3 o, float3 d, float bound) { trav_begin<W>(s, t, o, d, bound); };
+    if (__popc(idle) >= kIdleLanes || __ballot_sync(kFull, !done) == 0) {
       if (done && im.id >= 0) {
-        im.plain = trav_tied<W>(t);
-        if (!im.plain) item_hit(src, w, im, t.h, true, begin);
+        if (trav_tied<W>(t)) {
+          (im.shadow ? w.shadow_queue : w.sorted)[atomicAdd(it.ties + (im.shadow ? 0 : 1), 1)] = im.id;
+          im.id = -1;
+        } else {
+          item_hit(src, w, im, t.h, true, begin);
+        }
       }
       __syncwarp();
-      const int idx =  fetch_items<1>(it.fetch, im.id < 0 && !exhausted, 0, false);
-
+      const int idx = fetch_items<1>(it.fetch, im.id < 0 && !exhausted, 0, false);
       if (idx >= 0) {
         exhausted = idx >= it.total;
         if (!exhausted) item_start(src, w, it, idx, im, begin);
       }
-      if (__ballot_sync(kFull, t.node != kTravDone) == 0) {
-        if (!run_plain<W>(src, w, im, true, exhausted, eb)) break;
-        continue;
-      }
+      if (__ballot_sync(kFull, im.id >= 0 || !exhausted) == 0) break;
     }
     const DevScene &s = src.scene(im.view);
     const float eps = src.config(im.view).eps;
@@ -333,46 +323,49 @@ __device__ __forceinline__ void trace_groups(const Src &src, const WaveBuffers &
   const int lane = threadIdx.x & 31, sub = lane & (G - 1), shift = lane & ~(G - 1);
   const int stride = blockDim.x / G;
   int2 *stack = stacks + threadIdx.x / G;
-  TraceItem im;
-  GroupRay<G> t;
-  t.node = kTravDone;
-  t.sp = 0;
-  t.over = false;
-  t.h.t = 1e9f;
-  t.h.u = t.h.v = 0.f;
-  t.h.slot = -1;
-  t.tie = false;
   const int rays = warp_share(it.total, 32 / G);
   const int stop = rays > 3 ? kGroupIdle * G : G;
   bool exhausted = lane / G >= rays, first = true;
-  for (;;) {
-    const bool done = t.node == kTravDone && !im.plain;
-    const unsigned idle = __ballot_sync(kFull, done && !(exhausted && im.id < 0));
-    if (__popc(idle) >= stop || __ballot_sync(kFull, t.node != kTravDone) == 0) {
-      Hit h;
-      const bool good = group_hit(t, shift, h);
-      const auto begin = [&](const DevScene &s, float3 o, float3 d, float bound) { group_begin(s, t, o, d, bound); };
-      if (done && im.id >= 0) {
-        im.plain = !good;
-        if (good) item_hit(src, w, im, h, sub == 0, begin);
+  do {
+    TraceItem im;
+    GroupRay<G> t;
+    t.node = kTravDone;
+    t.sp = 0;
+    t.over = false;
+    t.h.t = 1e9f;
+    t.h.u = t.h.v = 0.f;
+    t.h.slot = -1;
+    t.tie = false;
+    const auto begin = [&](const DevScene &s, float3 o, float3 d, float bound) { group_begin(s, t, o, d, bound); };
+    for (;;) {
+      const bool done = t.node == kTravDone && !im.plain;
+      const unsigned idle = __ballot_sync(kFull, done && !(exhausted && im.id < 0));
+      if (__popc(idle) >= stop || __ballot_sync(kFull, t.node != kTravDone) == 0) {
+        Hit h;
+        const bool good = group_hit(t, shift, h);
+        if (done && im.id >= 0) {
+          im.plain = !good;
+          if (good) item_hit(src, w, im, h, sub == 0, begin);
+        }
+        __syncwarp();
+        const int idx = fetch_items<G>(it.fetch, im.id < 0 && !exhausted, rays, first);
+        first = false;
+        if (idx >= 0) {
+          exhausted = idx >= it.total;
+          if (!exhausted) item_start(src, w, it, idx, im, begin);
+        }
+        if (__ballot_sync(kFull, t.node != kTravDone || (im.id >= 0 && !im.plain)) == 0) break;
       }
-      __syncwarp();
-      const int idx = fetch_items<G>(it.fetch, im.id < 0 && !exhausted, rays, first);
-      first = false;
-      if (idx >= 0) {
-        exhausted = idx >= it.total;
-        if (!exhausted) item_start(src, w, it, idx, im, begin);
-      }
-      if (__ballot_sync(kFull, t.node != kTravDone) == 0) {
-        if (!run_plain<W>(src, w, im, sub == 0, exhausted, eb)) break;
-        continue;
-      }
-    }
-    const DevScene &s = src.scene(im.view);
-    const float eps = src.config(im.view).eps;
+      const DevScene &s = src.scene(im.view);
+      const float eps = src.config(im.view).eps;
 #pragma unroll 1
-    for (int i = 0; i < kGroupSteps; ++i) group_step(s, t, stack, stride, sub, shift, eps);
-  }
+      for (int i = 0; i < kGroupSteps; ++i) group_step(s, t, stack, stride, sub, shift, eps);
+    }
+    if (im.id >= 0 && sub == 0)
+      item_plain<W>(src.scene(im.view), src.config(im.view), src.film(im.view), w, im.id, im.shadow,
+                    src.shared(im.view), eb);
+    __syncwarp();
+  } while (__ballot_sync(kFull, !exhausted) != 0);
 }
 
 // trace(k): shadow chains of shade(k-1), then extension hits of Qk.
@@ -388,12 +381,14 @@ __device__ __forceinline__ TraceItems trace_items(const DevConfig &c, int depth,
     next = L->ext[a];
     it.q = w.queue[a];
     it.fetch = L->fetch + 0;
+    it.ties = L->ties;
     it.shadow_order = nullptr;
   } else {
     it.nsh = depth > 0 ? w.counts[kCntSh + depth - 1] : 0;
     next = depth < c.max_depth ? w.counts[kCntExt + depth] : 0;
     it.q = ext_sorted ? w.trace_order : w.queue[depth & 1];
     it.fetch = w.counts + kCntFetchT + depth;
+    it.ties = w.counts + kCntTies + 2 * depth;
     it.shadow_order = shadow_sorted ? w.shadow_order : nullptr;
   }
   it.total = it.nsh + next;
@@ -414,6 +409,21 @@ __global__ void __launch_bounds__(kMaxBlock, (kGroups ? kWideThreads : kStageThr
   const OneScene src{s, c, f, kLoop && L->shared != 0};
   if constexpr (kGroups) trace_groups<W>(src, w, it, group_stacks, eb);
   else trace_lanes<W>(src, w, it, eb);
+  if (eb) atomicOr(err, eb);
+}
+
+// the items that trace_lanes left open (two-child layout)
+template <bool kLoop>
+__global__ void __launch_bounds__(128) k_trace_ties(const __grid_constant__ DevScene s,
+                                                    const __grid_constant__ DevConfig c, int depth,
+                                                    const __grid_constant__ Film f,
+                                                    const __grid_constant__ WaveBuffers w, uint32_t *__restrict__ err,
+                                                    WaveLoop *L) {
+  const int *n = kLoop ? L->ties : w.counts + kCntTies + 2 * depth;
+  const int nsh = n[0], total = nsh + n[1];
+  uint32_t eb = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
+    item_plain<2>(s, c, f, w, i < nsh ? w.shadow_queue[i] : w.sorted[i - nsh], i < nsh, kLoop && L->shared != 0, eb);
   if (eb) atomicOr(err, eb);
 }
 
@@ -438,6 +448,7 @@ void launch_trace_w(const DevScene &s, const DevConfig &c, int depth, Film f, co
     }
   }
   k_trace<W, kLoop, false><<<grid, block, 0, st>>>(s, c, depth, f, w, err, ext_sorted, shadow_sorted, L);
+  if (W == 2) k_trace_ties<kLoop><<<kSMs, 128, 0, st>>>(s, c, depth, f, w, err, L);
 }
 
 // paths: path slots in use, the most extension rays (and shadow queries) the stage can have
@@ -694,6 +705,7 @@ __global__ void k_loop_init(const __grid_constant__ DevScene s, const __grid_con
     L->ext[1] = 0;
     L->sh[0] = L->sh[1] = 0;
     L->fetch[0] = L->fetch[1] = 0;
+    L->ties[0] = L->ties[1] = 0;
     L->next_item = n0;
     L->total = npass * npix;
     L->iter = 0;
@@ -770,6 +782,7 @@ __global__ void k_loop_control(WaveLoop *L, cudaGraphConditionalHandle h, int in
   L->ext[a] = 0;
   L->sh[a ^ 1] = 0;
   L->fetch[0] = L->fetch[1] = 0;
+  L->ties[0] = L->ties[1] = 0;
   const int it = L->iter + 1;
   L->iter = it;
   if (go && it >= L->limit) {
@@ -1013,6 +1026,7 @@ __global__ void k_bloop_init(const BatchSlot *__restrict__ slots, int n, const B
     L->ext[1] = 0;
     L->sh[0] = L->sh[1] = 0;
     L->fetch[0] = L->fetch[1] = 0;
+    L->ties[0] = L->ties[1] = 0;
     L->next_item = n0;
     L->total = total;
     L->iter = 0;
@@ -1039,8 +1053,21 @@ __global__ void __launch_bounds__(kMaxBlock, kStageThreads / kMaxBlock) k_trace_
   uint32_t eb = 0;
   const int a = L->iter & 1;
   const int nsh = L->sh[a ^ 1];
-  const TraceItems it{nsh, nsh + L->ext[a], w.queue[a], nullptr, L->fetch + 0};
+  const TraceItems it{nsh, nsh + L->ext[a], w.queue[a], nullptr, L->fetch + 0, L->ties};
   trace_lanes<W>(BatchScenes{slots}, w, it, eb);
+  if (eb) atomicOr(err, eb);
+}
+
+__global__ void __launch_bounds__(128) k_trace_ties_bloop(const BatchSlot *__restrict__ slots,
+                                                          const __grid_constant__ WaveBuffers w,
+                                                          uint32_t *__restrict__ err, const WaveLoop *L) {
+  const int nsh = L->ties[0], total = nsh + L->ties[1];
+  uint32_t eb = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int id = i < nsh ? w.shadow_queue[i] : w.sorted[i - nsh];
+    const BatchSlot &sl = slots[i < nsh ? w.sq_view[id] : w.view[id]];
+    item_plain<2>(sl.s, sl.c, sl.f, w, id, i < nsh, slot_shared(sl), eb);
+  }
   if (eb) atomicOr(err, eb);
 }
 
@@ -1112,7 +1139,10 @@ cudaError_t launch_trace_bloop(const BatchSlot *slots, const WaveBuffers &w, uin
   else if (width == 5) k_trace_bloop<5><<<grid, block, 0, st>>>(slots, w, err, w.loop);
   else if (width == 8) k_trace_bloop<8><<<grid, block, 0, st>>>(slots, w, err, w.loop);
   else if (width == 4) k_trace_bloop<4><<<grid, block, 0, st>>>(slots, w, err, w.loop);
-  else k_trace_bloop<2><<<grid, block, 0, st>>>(slots, w, err, w.loop);
+  else {
+    k_trace_bloop<2><<<grid, block, 0, st>>>(slots, w, err, w.loop);
+    k_trace_ties_bloop<<<kSMs, 128, 0, st>>>(slots, w, err, w.loop);
+  }
   return cudaGetLastError();
 }
 
