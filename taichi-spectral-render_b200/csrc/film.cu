@@ -234,7 +234,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_trace_batch_lanes(const __grid_
   if (eb) atomicOr(err, eb);
 }
 
-// the rays whose hit a tie left open (two-child layout)
+// the rays whose hit a tie left open
+template <int W>
 __global__ void k_trace_batch_ties(const __grid_constant__ DevScene s, float eps, const float *__restrict__ rays, int n,
                                    int32_t *__restrict__ tri_orig, float *__restrict__ t, float *__restrict__ u,
                                    float *__restrict__ v, uint32_t *err) {
@@ -242,7 +243,7 @@ __global__ void k_trace_batch_ties(const __grid_constant__ DevScene s, float eps
   for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     if (tri_orig[r] != kTied) continue;
     const float *q = rays + 6 * (size_t)r;
-    const Hit h = trace_plain<2>(s, f3(q[0], q[1], q[2]), f3(q[3], q[4], q[5]), eps, eb, 1e9f);
+    const Hit h = trace_plain<W>(s, f3(q[0], q[1], q[2]), f3(q[3], q[4], q[5]), eps, eb, 1e9f);
     tri_orig[r] = h.slot >= 0 ? __float_as_int(__ldg(s.tri + 3 * (size_t)h.slot).w) : -1;
     t[r] = h.t;
     if (u) u[r] = h.u;
@@ -258,7 +259,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_trace_batch_groups(const __grid
                                                                     int32_t *__restrict__ tri_orig,
                                                                     float *__restrict__ t, float *__restrict__ u,
                                                                     float *__restrict__ v, uint32_t *err) {
-  constexpr int G = W == 8 ? 8 : 4;
+  constexpr int G = kGroupLanes;
   __shared__ int2 stacks[kGroupStack * (kThreads / G)];
   const int lane = threadIdx.x & 31, sub = lane & (G - 1), shift = lane & ~(G - 1);
   const int warp = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
@@ -306,8 +307,9 @@ cudaError_t launch_resolve_rgb(Film f, const float *cmf, double scale, float *fr
                                float gamma, int iw, int ih, float *rgb, cudaStream_t st) {
   // An image of at least the frame's pixels repeats them: each is resolved and
   // tone-mapped once, then copied.  1024^2 frame, 1600^2 image: 135 us when every
-  // image pixel read the film and took its own powers, 59 us so.
-  if ((int64_t)iw * ih >= (int64_t)f.W * f.H) {
+  // image pixel read the film and took its own powers, 59 us so.  Small images
+  // are shorter than the second launch.
+  if ((int64_t)iw * ih >= (int64_t)f.W * f.H && (int64_t)iw * ih > (1 << 18)) {
     k_frame_rgb<<<grid_for((size_t)f.W * f.H), kThreads, 0, st>>>(f, cmf, scale, M, exposure, gamma, frame_rgb);
     const dim3 grid((unsigned)((iw - 1) / kThreads + 1), (unsigned)std::min(ih, 65535));
     k_upscale<<<grid, kThreads, 0, st>>>(frame_rgb, f.W, f.H, iw, ih, rgb);
@@ -337,7 +339,7 @@ cudaError_t launch_trace_batch(const DevScene &s, float eps, const float *rays, 
   // us, lanes / groups: 2,062 triangles 16k rays 36 / 24, 128k 61 / 58, 256k 81 / 95;
   // 2.6M triangles 16k 87 / 57, 128k 124 / 104, 256k 181 / 178, 512k 300 / 342.
   if (n <= kGroupRays && s.node_width != 5 && s.node_width != 9) {
-    const int share = std::min(s.node_width == 8 ? 4 : 8, std::max(1, n / (kSMs * 16)));
+    const int share = std::min(32 / kGroupLanes, std::max(1, n / (kSMs * 16)));
     const int warps = (n - 1) / share + 1;
     const auto k = s.node_width == 8   ? k_trace_batch_groups<8>
                    : s.node_width == 4 ? k_trace_batch_groups<4>
@@ -353,9 +355,9 @@ cudaError_t launch_trace_batch(const DevScene &s, float eps, const float *rays, 
                  : s.node_width == 4 ? k_trace_batch_lanes<4>
                                      : k_trace_batch_lanes<2>;
   k<<<blocks, kThreads, 0, st>>>(s, eps, rays, n, (n - 1) / warps + 1, tri_orig, t, u, v, err);
-  if (s.node_width == 2)
-    k_trace_batch_ties<<<std::min(kSMs * 8, (n - 1) / kThreads + 1), kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v,
-                                                                                        err);
+  const int tg = std::min(kSMs * 8, (n - 1) / kThreads + 1);
+  if (s.node_width == 2) k_trace_batch_ties<2><<<tg, kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v, err);
+  if (s.node_width == 8) k_trace_batch_ties<8><<<tg, kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v, err);
   return cudaGetLastError();
 }
 

@@ -20,6 +20,7 @@ computes on the CPU: every render call is a CUDA launch through the C ABI.
 """
 import ctypes
 import dataclasses
+import functools
 from dataclasses import dataclass
 
 import numpy as np
@@ -53,8 +54,8 @@ class RenderConfig:
     block_size: int = 0
     blocks_per_sm: int = 0
     sort_keys: int = 0
-    trace_budget: int = 0
-    traversal: str = "default"      # two-child nodes: "default" (if-if loop) or "speculative" (while-while)
+    trace_budget: int = 0           # accepted, without effect (idle lanes are refilled as they gather)
+    traversal: str = "default"      # "default" or "speculative": accepted, both run the same loop
     occupancy: int = 0              # megakernel: 0 = 5 blocks/SM (96 registers), 8 = 8 blocks/SM (64 registers)
     queue_capacity: int = 0         # wavefront path slots (0 = one per pixel); see ts_config
     loop_host: int = 0              # wavefront loop iterations launched by the host (profiling)
@@ -102,6 +103,13 @@ class _CudaArray:
 def _stream():
     import torch
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+@functools.lru_cache(maxsize=None)
+def _default_rgb():
+    """The display matrix of color_rays when none is given."""
+    from .spectral_data import srgb_xyz_to_rgb
+    return (ctypes.c_float * 9)(*srgb_xyz_to_rgb().reshape(9).tolist())
 
 
 class Renderer:
@@ -428,9 +436,9 @@ class Renderer:
         self.flush()
         c = self.config
         if xyz_to_rgb is None:
-            from .spectral_data import srgb_xyz_to_rgb
-            xyz_to_rgb = srgb_xyz_to_rgb()
-        m = (ctypes.c_float * 9)(*np.asarray(xyz_to_rgb, np.float64).reshape(9).tolist())
+            m = _default_rgb()
+        else:
+            m = (ctypes.c_float * 9)(*np.asarray(xyz_to_rgb, np.float64).reshape(9).tolist())
         if out is None:
             out = torch.empty((c.image_height, c.image_width, 3), dtype=torch.float32, device=self.device)
         self._check(self.lib.ts_resolve_rgb(self._ctx, float(self.cmf_scale), m, c.exposure, c.gamma,

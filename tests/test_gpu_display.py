@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("frame,image", [((1, 1), (1, 1)), ((33, 17), (33, 17)), ((33, 17), (66, 34)),
                                          ((33, 17), (101, 40)), ((50, 20), (1003, 1)), ((64, 48), (31, 23)),
-                                         ((257, 255), (300, 511))])
+                                         ((257, 255), (300, 511)), ((257, 255), (600, 511))])
 def test_color_rays_of_any_image_size(frame, image):
     s, c, ex = configs.box_scene(width=frame[0], height=frame[1], sphere_slices=8, sphere_stacks=9)
     c.image_width, c.image_height = image
