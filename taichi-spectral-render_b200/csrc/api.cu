@@ -384,11 +384,13 @@ ts_status ts_upload_scene(ts_ctx *c, const ts_scene_desc *sd) {
   ts::DevScene ds{};
   size_t &by = c->scene_bytes;
   std::vector<void *> &ow = c->scene_allocs;
-  float4 *d_node, *d_tri, *d_shade, *d_mat;
+  float4 *d_node, *d_node_own = nullptr, *d_tri, *d_shade, *d_mat;
   float *d_rmin, *d_rmax, *d_eem, *d_qy, *d_cdf, *d_lcdf, *d_larea, *d_cmf;
   int4 *d_rlink;
   int32_t *d_meem, *d_lslot, *d_nl;
   TS_CUDA(c, upload(c, ow, bvh.node2.data(), bvh.node2.size(), &d_node, by), "upload nodes");
+  if (!bvh.node_own.empty())
+    TS_CUDA(c, upload(c, ow, bvh.node_own.data(), bvh.node_own.size(), &d_node_own, by), "upload nodes");
   TS_CUDA(c, upload(c, ow, tri.data(), tri.size(), &d_tri, by), "upload triangles");
   TS_CUDA(c, upload(c, ow, shade.data(), shade.size(), &d_shade, by), "upload normals");
   TS_CUDA(c, upload(c, ow, bvh.ref_min.data(), bvh.ref_min.size(), &d_rmin, by), "upload ref nodes");
@@ -405,10 +407,11 @@ ts_status ts_upload_scene(ts_ctx *c, const ts_scene_desc *sd) {
   TS_CUDA(c, upload(c, ow, larea.data(), larea.size(), &d_larea, by), "upload lights");
   TS_CUDA(c, upload(c, ow, sd->cmf, (size_t)3 * B, &d_cmf, by), "upload CMF");
   ds.node = d_node;
+  ds.node_own = d_node_own ? d_node_own : d_node;
   ds.tri = d_tri;
   ds.shade = d_shade;
   ds.node_width = ts::layout_id(bvh.width, bvh.quantized);  // selects the traversal instantiation
-  ds.num_nodes = (int)(bvh.node2.size() / ts::node_float4s(bvh.width, bvh.quantized));
+  ds.num_nodes = (int)(bvh.node2.size() / ts::node_float4s(bvh.quantized ? bvh.width : 4, bvh.quantized));
   ds.num_tris = T;
   ds.ref_min = d_rmin;
   ds.ref_max = d_rmax;
@@ -434,7 +437,9 @@ ts_status ts_upload_scene(ts_ctx *c, const ts_scene_desc *sd) {
   c->d_cmf = d_cmf;
   c->perm = bvh.perm;
   c->info.num_tris = T;
-  c->info.num_nodes = bvh.width == 2 ? bvh.two_child_nodes : ds.num_nodes;
+  c->info.num_nodes = bvh.width == 2            ? bvh.two_child_nodes
+                      : !bvh.node_own.empty() ? (int)(bvh.node_own.size() / ts::node_float4s(8))
+                                              : ds.num_nodes;
   c->info.num_ref_nodes = ds.num_ref_nodes;
   c->info.max_depth = bvh.max_depth;
   c->info.leaves = bvh.leaves;

@@ -449,8 +449,15 @@ bool flatten_tree(std::vector<BNode> &&tree, const std::vector<Prim> &prims, con
   out.leaves = leaves;
   out.stack_need = maxd;
   if (width == 4 || width == 8) {
-    if (flatten_wide(tree, width, out, quantize)) return true;
-    if (quantize && flatten_wide(tree, width, out, false)) return true;
+    if (quantize && flatten_wide(tree, width, out, true)) return true;
+    if (flatten_wide(tree, width, out, false)) {
+      if (width == 8) {  // walked as four-child nodes of the same tree
+        out.node_own.swap(out.node2);
+        if (!flatten_wide(tree, 4, out)) out.node2.clear();
+        out.width = 8;
+      }
+      return true;
+    }
   }
   // the two-child layout (asked for, or because the wide one cannot be built):
   // its device nodes are the same tree collapsed to four children, or none

@@ -45,7 +45,8 @@ struct BvhParams {
 
 struct BvhOut {
   std::vector<int32_t> perm;   // slot -> original triangle index
-  std::vector<float4> node2;   // device nodes: 8 float4 each for the layouts of width 2 and 4, 16 for 8
+  std::vector<float4> node2;   // nodes the device walks: 8 float4 each for full precision (four children)
+  std::vector<float4> node_own;  // width 8: the layout's own nodes, 16 float4 each
   int width = 2;               // node width of the layout (a wide layout falls back to 2 if its stack bound is exceeded)
   int two_child_nodes = 0;     // inner nodes of the binary tree (1 for a lone leaf)
   bool quantized = false;      // node2 holds quantized wide nodes
@@ -61,11 +62,11 @@ struct BvhOut {
 bool build_bvh_binned(int T, const float *v0, const float *v1, const float *v2, const BvhParams &p, BvhOut &out,
                       std::string &err);
 
-// float4s per node of the device layout for a node width (quantized: child
+// float4s per node of a node array of this many children (quantized: child
 // boxes as bytes relative to the node's origin -- 4 float4 for 4-wide, 6 for 8-wide).
 inline int node_float4s(int width, bool quantized = false) {
   if (quantized) return width == 8 ? 6 : 4;
-  return width == 8 ? 16 : 8;  // width 2: the binary tree collapsed to four children
+  return width == 8 ? 16 : 8;
 }
 // the device layout id: the node width, plus one for quantized child boxes (5, 9)
 inline int layout_id(int width, bool quantized) { return quantized && width >= 4 ? width + 1 : width; }

@@ -41,12 +41,13 @@ struct DevConfig {
 // Wide nodes (width 4 / 8): one 32-byte record per child,
 //   (lo.x, hi.x, lo.y, hi.y), (lo.z, hi.z, link, -)
 // A child >= 0 is an inner node, < 0 a leaf: ~child = (first_slot << 4) |
-// (count - 1).  The two-child layout's device nodes are its tree collapsed to
+// (count - 1).  Layouts of width 2 and 8 are walked as the same tree collapsed to
 // four children.
 // Reference-layout nodes (main.py:267-275) are kept for the exact-order
 // traversal used by parity checks and for the two-child order.
 struct DevScene {
-  const float4 *__restrict__ node;    // device BVH layout
+  const float4 *__restrict__ node;      // nodes that the fast loops walk
+  const float4 *__restrict__ node_own;  // width 4 and 8: the layout's own nodes (the same array for 4)
   const float4 *__restrict__ tri;
   const float4 *__restrict__ shade;
   int32_t num_nodes, num_tris;

@@ -39,6 +39,33 @@ constexpr int kCntTies = kCntFetchS + kMaxDepth + 1;  // [2 * (kMaxDepth+1)] tie
 constexpr int kCntTotal = kCntTies + 2 * (kMaxDepth + 1);
 static_assert(kCntTotal <= 8192, "WaveBuffers::counts");
 
+// ---- dependent launches
+// The stages of a depth-synchronous pass are launched with programmatic stream
+// serialisation: a stage's blocks come up while the one before drains, and every
+// thread waits for that one's end before it reads or writes anything.  Every
+// block of a stage waits, also one without work, so a stage's end implies the
+// ends of all before it.  A 64^2 pass of 18 launches takes 500 us without, 474 us so;
+// 25 passes at 256^2 19.4 and 18.5 ms.
+__device__ __forceinline__ void stage_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... Params, class... Args>
+void launch_stage(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, Params(args)...);  // the caller looks at cudaGetLastError
+}
+
 // ---- work fetching
 // The blocks of k_shade* and trace_groups are all resident (resident_grid: what the
 // kernel's registers allow), so every warp has its first items without asking:
@@ -271,7 +298,7 @@ constexpr int kPhases = 4;      // 1: 5 % slower, 8: the same
 constexpr int kIdleLanes = 16;  // 4 / 8 / 12: 11 / 5 / 1 % slower, 20: 3 % slower on the volume
 
 // A tied item goes to a list (k_trace_ties): a call to trace_plain() in this
-// kernel, wherever it stood, cost the two-child layout 16 to 20 %.
+// kernel, wherever it stood, cost the stage 16 to 20 %.
 template <int W, class Src>
 __device__ __forceinline__ void trace_lanes(const Src &src, const WaveBuffers &w, const TraceItems &it,
                                             uint32_t &eb) {
@@ -319,7 +346,7 @@ template <int W, class Src>
 __device__ __forceinline__ void trace_groups(const Src &src, const WaveBuffers &w, const TraceItems &it, int2 *stacks,
                                              uint32_t &eb) {
   constexpr unsigned kFull = 0xffffffffu;
-  constexpr int G = W == 8 ? 8 : 4;
+  constexpr int G = kGroupLanes;
   const int lane = threadIdx.x & 31, sub = lane & (G - 1), shift = lane & ~(G - 1);
   const int stride = blockDim.x / G;
   int2 *stack = stacks + threadIdx.x / G;
@@ -404,6 +431,7 @@ __global__ void __launch_bounds__(kMaxBlock, (kGroups ? kWideThreads : kStageThr
                                                      int shadow_sorted, WaveLoop *L) {
   extern __shared__ int2 group_stacks[];  // kGroups: [kGroupStack][groups of the block]
   uint32_t eb = 0;
+  if (!kLoop) stage_begin();
   const TraceItems it = trace_items<kLoop>(c, depth, w, ext_sorted, shadow_sorted, L);
   if (it.total <= 0) return;
   const OneScene src{s, c, f, kLoop && L->shared != 0};
@@ -412,18 +440,19 @@ __global__ void __launch_bounds__(kMaxBlock, (kGroups ? kWideThreads : kStageThr
   if (eb) atomicOr(err, eb);
 }
 
-// the items that trace_lanes left open (two-child layout)
-template <bool kLoop>
+// the items that trace_lanes left open
+template <int W, bool kLoop>
 __global__ void __launch_bounds__(128) k_trace_ties(const __grid_constant__ DevScene s,
                                                     const __grid_constant__ DevConfig c, int depth,
                                                     const __grid_constant__ Film f,
                                                     const __grid_constant__ WaveBuffers w, uint32_t *__restrict__ err,
                                                     WaveLoop *L) {
+  if (!kLoop) stage_begin();
   const int *n = kLoop ? L->ties : w.counts + kCntTies + 2 * depth;
   const int nsh = n[0], total = nsh + n[1];
   uint32_t eb = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x)
-    item_plain<2>(s, c, f, w, i < nsh ? w.shadow_queue[i] : w.sorted[i - nsh], i < nsh, kLoop && L->shared != 0, eb);
+    item_plain<W>(s, c, f, w, i < nsh ? w.shadow_queue[i] : w.sorted[i - nsh], i < nsh, kLoop && L->shared != 0, eb);
   if (eb) atomicOr(err, eb);
 }
 
@@ -436,19 +465,29 @@ __global__ void __launch_bounds__(128) k_trace_ties(const __grid_constant__ DevS
 // 512^2 10.4 / 10.9.
 constexpr int kGroupPaths = 148 * 1024 * 3 / 2;
 
+// a stage of a pass, or of the loop (plainly: it is captured as the body of a while node)
+template <bool kLoop, class... Params, class... Args>
+void trace_launch(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
+  if (kLoop) kernel<<<grid, block, smem, st>>>(args...);
+  else launch_stage(kernel, grid, block, smem, st, args...);
+}
+
 template <int W, bool kLoop>
 void launch_trace_w(const DevScene &s, const DevConfig &c, int depth, Film f, const WaveBuffers &w, uint32_t *err,
                     int grid, int block, cudaStream_t st, int ext_sorted, int shadow_sorted, WaveLoop *L,
                     int paths) {
   if constexpr (W != 5 && W != 9) {
     if (paths <= kGroupPaths) {
-      const size_t smem = (size_t)(block / (W == 8 ? 8 : 4)) * kGroupStack * sizeof(int2);
-      k_trace<W, kLoop, true><<<resident_grid(grid, block, kWideThreads), block, smem, st>>>(s, c, depth, f, w, err, ext_sorted, shadow_sorted, L);
+      const size_t smem = (size_t)(block / kGroupLanes) * kGroupStack * sizeof(int2);
+      trace_launch<kLoop>(k_trace<W, kLoop, true>, resident_grid(grid, block, kWideThreads), block, smem, st, s, c, depth,
+                          f, w, err, ext_sorted, shadow_sorted, L);
       return;
     }
   }
-  k_trace<W, kLoop, false><<<grid, block, 0, st>>>(s, c, depth, f, w, err, ext_sorted, shadow_sorted, L);
-  if (W == 2) k_trace_ties<kLoop><<<kSMs, 128, 0, st>>>(s, c, depth, f, w, err, L);
+  trace_launch<kLoop>(k_trace<W, kLoop, false>, grid, block, (size_t)0, st, s, c, depth, f, w, err, ext_sorted,
+                      shadow_sorted, L);
+  if constexpr (kWalkedAsFour<W>)
+    trace_launch<kLoop>(k_trace_ties<W, kLoop>, kSMs, 128, (size_t)0, st, s, c, depth, f, w, err, L);
 }
 
 // paths: path slots in use, the most extension rays (and shadow queries) the stage can have
@@ -650,6 +689,7 @@ __device__ __forceinline__ void append_ext(int *count, int *q, int pid, bool wan
 
 __global__ void __launch_bounds__(kMaxBlock, kWideThreads / kMaxBlock) k_shade(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass, int band, int depth,
                                                Film f, WaveBuffers w, int use_sorted, uint32_t *err) {
+  stage_begin();
   const int n = w.counts[kCntExt + depth];
   const int *q = use_sorted ? w.sorted : w.queue[depth & 1];
   int *qn = w.queue[(depth + 1) & 1];
@@ -837,7 +877,8 @@ cudaError_t launch_wave_chunk(const DevScene &s, const DevConfig &c, uint32_t pa
     if (sh_sorted) launch_sort(s, d - 1, w, kSortShadow, kShadowKeys, w.shadow_order, sort_grid, st);
     launch_trace(s, c, d, f, w, err, grid, block, st, n, ext_sorted, sh_sorted);
     if (sort_keys & 1) launch_sort(s, d, w, kSortShade, nmat, w.sorted, sort_grid, st);
-    k_shade<<<resident_grid(grid, block, kWideThreads), block, 0, st>>>(s, c, pass, band, d, f, w, (sort_keys & 1) ? 1 : 0, err);
+    launch_stage(k_shade, resident_grid(grid, block, kWideThreads), block, 0, st, s, c, pass, band, d, f, w,
+                 (sort_keys & 1) ? 1 : 0, err);
   }
   // the last depth's shadow queries
   if (c.max_depth > 0) {
@@ -1058,6 +1099,7 @@ __global__ void __launch_bounds__(kMaxBlock, kStageThreads / kMaxBlock) k_trace_
   if (eb) atomicOr(err, eb);
 }
 
+template <int W>
 __global__ void __launch_bounds__(128) k_trace_ties_bloop(const BatchSlot *__restrict__ slots,
                                                           const __grid_constant__ WaveBuffers w,
                                                           uint32_t *__restrict__ err, const WaveLoop *L) {
@@ -1066,7 +1108,7 @@ __global__ void __launch_bounds__(128) k_trace_ties_bloop(const BatchSlot *__res
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const int id = i < nsh ? w.shadow_queue[i] : w.sorted[i - nsh];
     const BatchSlot &sl = slots[i < nsh ? w.sq_view[id] : w.view[id]];
-    item_plain<2>(sl.s, sl.c, sl.f, w, id, i < nsh, slot_shared(sl), eb);
+    item_plain<W>(sl.s, sl.c, sl.f, w, id, i < nsh, slot_shared(sl), eb);
   }
   if (eb) atomicOr(err, eb);
 }
@@ -1137,11 +1179,14 @@ cudaError_t launch_trace_bloop(const BatchSlot *slots, const WaveBuffers &w, uin
                                int block, cudaStream_t st) {
   if (width == 9) k_trace_bloop<9><<<grid, block, 0, st>>>(slots, w, err, w.loop);
   else if (width == 5) k_trace_bloop<5><<<grid, block, 0, st>>>(slots, w, err, w.loop);
-  else if (width == 8) k_trace_bloop<8><<<grid, block, 0, st>>>(slots, w, err, w.loop);
+  else if (width == 8) {
+    k_trace_bloop<8><<<grid, block, 0, st>>>(slots, w, err, w.loop);
+    k_trace_ties_bloop<8><<<kSMs, 128, 0, st>>>(slots, w, err, w.loop);
+  }
   else if (width == 4) k_trace_bloop<4><<<grid, block, 0, st>>>(slots, w, err, w.loop);
   else {
     k_trace_bloop<2><<<grid, block, 0, st>>>(slots, w, err, w.loop);
-    k_trace_ties_bloop<<<kSMs, 128, 0, st>>>(slots, w, err, w.loop);
+    k_trace_ties_bloop<2><<<kSMs, 128, 0, st>>>(slots, w, err, w.loop);
   }
   return cudaGetLastError();
 }
@@ -1383,7 +1428,7 @@ cudaError_t launch_wave_tile_noalloc(const DevScene &s, const DevConfig &c, uint
   k_generate_tile<<<(n + 255) / 256, 256, 0, st>>>(s, c, pass, band, w, x0, y0, tw, th);
   for (int d = 0; d < c.max_depth; ++d) {
     launch_trace(s, c, d, f, w, err, grid, block, st, n);
-    k_shade<<<resident_grid(grid, block, kWideThreads), block, 0, st>>>(s, c, pass, band, d, f, w, 0, err);
+    launch_stage(k_shade, resident_grid(grid, block, kWideThreads), block, 0, st, s, c, pass, band, d, f, w, 0, err);
   }
   if (c.max_depth > 0) launch_trace(s, c, c.max_depth, f, w, err, grid, block, st, n);
   return cudaGetLastError();

@@ -253,7 +253,7 @@ TS_D int node_children_q(const DevScene &s, const Traversal &t, float *key, int 
 
 // The children of a wide node that the ray enters, as sorted (entry distance,
 // link) pairs; returns how many.
-// W: 4 or 8, 5 and 9 for quantized nodes.
+// W: 4; 5 and 9 for quantized nodes.
 template <int W>
 TS_D int node_children(const DevScene &s, const Traversal &t, float *key, int *ref) {
   if (W == 5 || W == 9) return node_children_q<W>(s, t, key, ref);
@@ -451,14 +451,14 @@ TS_D Hit trace_wide_plain(const DevScene &s, float3 o, float3 d, float eps, uint
   h.t = 1e9f;
   h.u = h.v = 0.f;
   h.slot = -1;
-  if (s.num_nodes <= 0) return h;
+  if (s.num_tris <= 0) return h;
   const float3 inv = f3(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z));
   float tcull = cull_bound(fminf(bound, 1e9f));
   int2 stack[kWideStack];
   int sp = 0, node = 0;
   for (;;) {
     if (node >= 0) {
-      const float *n = reinterpret_cast<const float *>(s.node) + (size_t)(W == 4 ? 32 : 64) * node;
+      const float *n = reinterpret_cast<const float *>(s.node_own) + (size_t)(8 * W) * node;
       if (kCount) tc->nodes++;
       float key[W];
       int ref[W];
@@ -523,11 +523,14 @@ __device__ __noinline__ Hit trace_plain(const DevScene &s, float3 o, float3 d, f
 }
 
 // ---- layouts ----------------------------------------------------------------
-// A compile-time choice of each kernel instance.  W = 2: two-child layout, which
-// the fast loop walks as four-child nodes collapsed from the same tree (half the
-// steps of a ray); its box tests accept the same leaves, so only a ray that meets
-// two triangles at exactly the same distance can differ, and that ray is traced
-// again in the two-child order.  W = 4 / 8: wide nodes; W = 5 / 9: quantized.
+// A compile-time choice of each kernel instance.  W = 2 and 8: the fast loops walk
+// the four-child nodes collapsed from the same tree (against two children half the
+// steps of a ray; against eight a quarter of the sorting network: 17 % less time
+// for the terrain's bundles); their box tests accept the same leaves, so only a ray
+// that meets two triangles at exactly the same distance can differ, and that ray
+// is traced again in the layout's own order.  W = 4; W = 5 / 9: quantized.
+template <int W>
+constexpr bool kWalkedAsFour = W == 2 || W == 8;
 
 // bound: distance beyond which hits do not matter to the caller.  Boxes past
 // it are skipped; a hit beyond it may still be returned (callers treat such a
@@ -548,22 +551,23 @@ TS_D void trav_begin(const DevScene &s, Traversal &t, float3 o, float3 d, float 
   t.tcull = cull_bound(fminf(bound, 1e9f));
   t.node = s.num_nodes > 0 ? 0 : kTravDone;
   t.sp = 0;
-  t.tie = W == 2 && s.num_nodes <= 0;  // a two-child tree too deep for the wide stack has no wide nodes
+  t.tie = kWalkedAsFour<W> && s.num_nodes <= 0;  // a tree too deep for the wide stack has no four-child nodes
 }
 
 // a finished traversal's hit does not stand: trace_plain() has to decide a tie
 template <int W>
 TS_D bool trav_tied(const Traversal &t) {
-  return W == 2 && t.tie;
+  return kWalkedAsFour<W> && t.tie;
 }
 
 // the node layout behind a layout id
 template <int W>
 struct Nodes {
-  static constexpr int value = W == 2 ? 4 : W;
+  static constexpr int value = W == 2 || W == 8 ? 4 : W;
 };
 
-// Fast closest hit in one go (local-memory stack).  errbits gets
+// Fast closest hit in one go (local-memory stack); slot kTiedSlot: a tie that
+// trace_plain() decides.  errbits gets
 // kErrStackOverflow if the tree is deeper than the stack (the builder bounds
 // the depth below it, so this is a guard only).
 // Not inlined: one copy of the traversal per kernel instead of one per call
@@ -573,9 +577,11 @@ struct Nodes {
 // kTogether: the lanes that arrive together step together (warp_phase): 9 % less
 // time for the adjoint's replays and the batch kernel, 15 % for ray queries; a
 // single pass of few paths waits more than it gains.
-template <int W, bool kCount = false, bool kTogether = true>
-__device__ __noinline__ Hit trace_closest(const DevScene &s, float3 o, float3 d, float eps, uint32_t &errbits,
-                                          TraceCount *tc = nullptr, float bound = 1e9f) {
+constexpr int kTiedSlot = -2;
+
+template <int W, bool kCount, bool kTogether>
+__device__ __noinline__ Hit trace_fast(const DevScene &s, float3 o, float3 d, float eps, uint32_t &errbits,
+                                       TraceCount *tc, float bound) {
   if (kCount && W == 2) return trace_two_child<true>(s, o, d, eps, errbits, tc, bound);
   if (kCount && (W == 4 || W == 8)) return trace_wide_plain<W == 8 ? 8 : 4, true>(s, o, d, eps, errbits, tc, bound);
   Traversal t;
@@ -587,17 +593,26 @@ __device__ __noinline__ Hit trace_closest(const DevScene &s, float3 o, float3 d,
     const unsigned mask = __activemask();
     while (warp_phase<Nodes<W>::value>(s, t, stack, eps, errbits, mask)) {}
   }
-  if (trav_tied<W>(t)) return trace_plain<W>(s, o, d, eps, errbits, bound);
+  if (trav_tied<W>(t)) t.h.slot = kTiedSlot;
   return t.h;
 }
 
+template <int W, bool kCount = false, bool kTogether = true>
+TS_D Hit trace_closest(const DevScene &s, float3 o, float3 d, float eps, uint32_t &errbits, TraceCount *tc = nullptr,
+                       float bound = 1e9f) {
+  Hit h = trace_fast<W, kCount, kTogether>(s, o, d, eps, errbits, tc, bound);
+  if (kWalkedAsFour<W> && h.slot == kTiedSlot) h = trace_plain<W>(s, o, d, eps, errbits, bound);
+  return h;
+}
+
 // ---- group traversal ---------------------------------------------------------
-// G lanes (the node width, 4 or 8) walk one ray: lane k tests child k of a node
+// Four lanes (kGroupLanes, G below) walk one ray: lane k tests child k of a node
 // and triangles k, k + G, ... of a leaf.  Against a ray per lane a step is a
 // third of the instructions (one box, no sorting network, one triangle) and a
 // node costs one or two contiguous loads of the warp instead of eight scattered
 // ones per lane, and a warp serialises G times fewer rays.  All lanes of a warp run
 // the same loop: its votes and shuffles take the whole warp.
+constexpr int kGroupLanes = 4;
 constexpr int kGroupStack = 32;  // entries per ray, in shared memory; a ray that needs more goes to trace_plain()
 
 template <int G>
