@@ -621,6 +621,16 @@ ts_status ts_record_paths(ts_ctx *c, uint32_t first_pass, int32_t num_passes) {
   return TS_OK;
 }
 
+// A wavefront pass of few paths is one launch of the path kernel: each of its
+// 2 * depth + 1 stages would last as long as its longest ray, and its code comes
+// to cold instruction caches.  us per pass, stages / one kernel: box 64^2 450 / 314,
+// 256^2 702 / 682, 400^2 1019 / 870; terrain (647k triangles) 64^2 336 / 234, 448^2
+// 976 / 704; volume 64^2 2274 / 1990, 448^2 8681 / 8771, 512^2 8987 / 10831.
+static bool pass_in_one_kernel(const ts_ctx *c) {
+  return c->cfg.queue_capacity == 0 && c->cfg.sort_keys == 0 &&
+         (int64_t)c->cfg.width * c->cfg.height <= 148 * 1024 * 3 / 2;
+}
+
 ts_status ts_render_pass(ts_ctx *c, uint32_t pass_idx, int32_t band, void *stream) {
   if (!c) return fail(nullptr, TS_ERR_INVALID_ARG, "ts_render_pass: null context");
   if (!c->has_scene) return fail(c, TS_ERR_NO_SCENE, "ts_render_pass: no scene uploaded");
@@ -629,11 +639,13 @@ ts_status ts_render_pass(ts_ctx *c, uint32_t pass_idx, int32_t band, void *strea
   const cudaStream_t st = as_stream(stream);
   const int bs = c->cfg.block_size;
   if (float *rec = rec_slot(c, pass_idx, 1)) return render_recorded(c, pass_idx, 1, band, rec, st, "render pass");
-  if (c->cfg.kernel == TS_KERNEL_MEGA) {
+  if (c->cfg.kernel == TS_KERNEL_MEGA || pass_in_one_kernel(c)) {
     int per_sm = c->cfg.blocks_per_sm;
     if (per_sm <= 0) per_sm = std::max(1, 2048 / bs);
     const int grid = c->num_sms * per_sm;
-    TS_CUDA(c, ts::launch_render_mega(c->ds, c->dc, pass_idx, band, film_of(c), c->d_counter, c->d_err, grid, bs, st,
+    ts::Film f = film_of(c);
+    f.each_vertex = c->cfg.kernel != TS_KERNEL_MEGA;
+    TS_CUDA(c, ts::launch_render_mega(c->ds, c->dc, pass_idx, band, f, c->d_counter, c->d_err, grid, bs, st,
                                       nullptr, 1, c->cfg.occupancy),
             "render pass");
   } else {

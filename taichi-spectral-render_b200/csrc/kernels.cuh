@@ -18,6 +18,9 @@ struct Film {
   // item of the launch the path's total deposit, or -1 where volume
   // fluorescence moved the path to another band
   float *rec = nullptr;
+  // megakernel: deposit each vertex as the wavefront stages do, not each path's sum
+  // (without records); the film then has the stages' order of additions
+  bool each_vertex = false;
 };
 
 // largest scene whose vertices a block's warps take together (mega_path.cuh)

@@ -146,6 +146,10 @@ __device__ __forceinline__ void mega_vertex(const DevScene &s, const DevConfig &
     // A path whose throughput is exactly zero deposits exact zeros from
     // here on (every later term is a product with it), so it ends early.
     if (++L.k >= c.max_depth || p.thr == 0.f) done = true;
+    if (f.each_vertex) {
+      mega_flush(f, L.pix, p.active_px, L.dep, shared);
+      L.dep = 0.0;
+    }
   }
   if (done) {
     if (kCount) cnt.dep += L.dep != 0.0;

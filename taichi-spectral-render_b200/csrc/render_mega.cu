@@ -31,7 +31,11 @@ __global__ void __launch_bounds__(128, kMinBlocks) k_render_mega(const __grid_co
   const int npix = c.W * c.H;
   const int total = npix * npass;
   uint32_t errbits = 0;
-  bool exhausted = false;
+  // Few paths: fewer lanes of each warp rather than fewer warps, whose lanes'
+  // branches run one after the other.  us per pass, full warps / so: box 32^2
+  // 513 / 193, 64^2 506 / 316; terrain 64^2 391 / 241; volume 32^2 3141 / 1081.
+  const int warps = (int)min((int64_t)gridDim.x * (blockDim.x >> 5), (int64_t)148 * kMinBlocks * 4);  // what the device holds
+  bool exhausted = lane >= max(1, (total - 1) / warps + 1);
   MegaLane L;
   L.pix = -1;
   for (;;) {
@@ -74,11 +78,11 @@ template <int W>
 void launch_w(const DevScene &s, const DevConfig &c, uint32_t pass0, int npass, int band0, Film f, int *counter,
               uint32_t *err, int grid, int block, cudaStream_t st, unsigned long long *work, int occupancy) {
   // Together where shading, not the length of single traversals, takes the time:
-  // small trees and enough paths.  ms per pass apart / together: box (2,062
-  // triangles) 64^2 0.50 / 0.55, 128^2 0.55 / 0.59, 256^2 0.77 / 0.67, 512^2 1.57 / 1.20,
-  // bundles of 25 passes at 512^2 1.23 / 0.92; volume (20,014) 256^2 4.87 / 4.74,
-  // bundle 2.57 / 2.52; terrain (647,258) 256^2 0.57 / 0.59, 512^2 0.76 / 0.83.
-  const bool together = s.num_tris <= kTogetherTris && (int64_t)c.W * c.H * npass >= 65536;
+  // small trees and enough paths.  us per pass apart / together: box (2,062
+  // triangles) 64^2 306 / 316, 128^2 565 / 468, 192^2 737 / 584, 512^2 1570 / 1217,
+  // volume (20,014) 128^2 3373 / 2640, 192^2 4183 / 3535, bundles of 25 at 256^2
+  // 63 / 63 ms; terrain (647,258) 256^2 568 / 594, 512^2 762 / 829.
+  const bool together = s.num_tris <= kTogetherTris && (int64_t)c.W * c.H * npass >= 16384;
   const auto k = work          ? k_render_mega<W, true>
                  : occupancy >= 8 ? (together ? k_render_mega<W, false, 8, true> : k_render_mega<W, false, 8>)
                                   : (together ? k_render_mega<W, false, 5, true> : k_render_mega<W, false>);

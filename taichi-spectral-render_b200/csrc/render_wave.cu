@@ -340,7 +340,7 @@ __device__ __forceinline__ void trace_lanes(const Src &src, const WaveBuffers &w
 
 // A group of lanes per ray (full-precision nodes), looking for finished groups
 // every kGroupSteps steps and stopping for kGroupIdle of them.
-constexpr int kGroupSteps = 2, kGroupIdle = 2;
+constexpr int kGroupSteps = 4, kGroupIdle = 3;
 
 template <int W, class Src>
 __device__ __forceinline__ void trace_groups(const Src &src, const WaveBuffers &w, const TraceItems &it, int2 *stacks,
@@ -351,7 +351,7 @@ __device__ __forceinline__ void trace_groups(const Src &src, const WaveBuffers &
   const int stride = blockDim.x / G;
   int2 *stack = stacks + threadIdx.x / G;
   const int rays = warp_share(it.total, 32 / G);
-  const int stop = rays > 3 ? kGroupIdle * G : G;
+  const int stop = rays > 4 ? kGroupIdle * G : G;
   bool exhausted = lane / G >= rays, first = true;
   do {
     TraceItem im;
