@@ -62,8 +62,9 @@ typedef struct {
                                     2 extension rays by direction octant, 4 shadow rays by light (0 = off) */
   int32_t trace_budget;          /* wavefront: accepted, without effect (idle lanes are refilled as they gather) */
   int32_t traversal;             /* TS_TRAVERSAL_DEFAULT or TS_TRAVERSAL_SPECULATIVE; both run the same loop */
-  int32_t occupancy;             /* megakernel register budget: 0 = 5 resident blocks of 128 per SM (96 registers),
-                                    8 = 8 blocks (64 registers, spills; more latency hiding on large frames) */
+  int32_t occupancy;             /* megakernel register budget: 5 = 5 resident blocks of 128 per SM (96 registers),
+                                    8 = 8 blocks (64 registers, spills; more latency hiding on large frames),
+                                    0 = 8 for launches of 2^19 paths or more, else 5 */
   int32_t queue_capacity;        /* wavefront path slots (0 = one per pixel; at most 2^25).  With sort_keys == 0,
                                     ts_render_passes, and ts_render_pass when queue_capacity > 0, run the
                                     regenerating loop: a slot whose path has ended starts the next pixel (of

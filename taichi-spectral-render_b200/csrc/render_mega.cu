@@ -83,9 +83,17 @@ void launch_w(const DevScene &s, const DevConfig &c, uint32_t pass0, int npass, 
   // volume (20,014) 128^2 3373 / 2640, 192^2 4183 / 3535, bundles of 25 at 256^2
   // 63 / 63 ms; terrain (647,258) 256^2 568 / 594, 512^2 762 / 829.
   const bool together = s.num_tris <= kTogetherTris && (int64_t)c.W * c.H * npass >= 16384;
-  const auto k = work          ? k_render_mega<W, true>
-                 : occupancy >= 8 ? (together ? k_render_mega<W, false, 8, true> : k_render_mega<W, false, 8>)
-                                  : (together ? k_render_mega<W, false, 5, true> : k_render_mega<W, false>);
+  // Unless the caller chose, 64 registers where there are paths for the 8 blocks of
+  // an SM that they allow, several for each lane; with fewer paths the spills cost
+  // more than the warps hide.  us at 96 / 64 registers: bundles of 25 at 128^2
+  // (409,600 paths) box 1857 / 1889, volume 17507 / 15320, terrain (20,000) 910 /
+  // 835, (647,258) 1283 / 1263; at 256^2 (1.6M) 6131 / 5738, 64199 / 52926, 2745 /
+  // 2349, 3957 / 3616; a pass at 512^2 (262,144) 1223 / 1245, 10952 / 9951, 540 / 572,
+  // 797 / 890; at 256^2 (65,536) 669 / 845, 4433 / 5140, 365 / 375, 547 / 548.
+  const bool narrow = occupancy >= 8 || (occupancy == 0 && (int64_t)c.W * c.H * npass >= (1 << 19));
+  const auto k = work     ? k_render_mega<W, true>
+                 : narrow ? (together ? k_render_mega<W, false, 8, true> : k_render_mega<W, false, 8>)
+                          : (together ? k_render_mega<W, false, 5, true> : k_render_mega<W, false>);
   k<<<grid, block, 0, st>>>(s, c, pass0, npass, band0, f, counter, err, work);
 }
 

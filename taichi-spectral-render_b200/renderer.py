@@ -56,7 +56,7 @@ class RenderConfig:
     sort_keys: int = 0
     trace_budget: int = 0           # accepted, without effect (idle lanes are refilled as they gather)
     traversal: str = "default"      # "default" or "speculative": accepted, both run the same loop
-    occupancy: int = 0              # megakernel: 0 = 5 blocks/SM (96 registers), 8 = 8 blocks/SM (64 registers)
+    occupancy: int = 0              # megakernel: 5 blocks/SM (96 registers) or 8 (64 registers), 0 = by the paths of a launch
     queue_capacity: int = 0         # wavefront path slots (0 = one per pixel); see ts_config
     loop_host: int = 0              # wavefront loop iterations launched by the host (profiling)
     defer_passes: bool = False      # cast_rays queues passes; runs of consecutive passes launch as bundles
