@@ -898,8 +898,11 @@ def bench_ours(args):
                 for b in range(B):
                     r.cast_rays(b, pass_idx=timed_first + k * B + b)
                     iters.append(r.wave_loop_iterations())
-        # a loop launch: the init kernel, then trace + shade + control per iteration
-        gpu_launches = sum(1 + 3 * it for it in iters)
+        # a loop launch: the init kernel, then trace + shade + control per iteration, and where the
+        # layout is walked as four-child nodes by a ray per lane, the kernel that decides ties
+        ties = info["node_width"] in (2, 8) and not info["node_quantized"] and min(
+            r.config.queue_capacity, (B if use_bundles else 1) * npix) > 227328
+        gpu_launches = sum(1 + (4 if ties else 3) * it for it in iters)
         launches = ("one regenerating wavefront loop per %s (init kernel, then a CUDA-graph while-loop of trace, "
                     "shade, control; %.1f iterations per launch)" % ("step (25-pass bundle)" if use_bundles
                                                                      else "pass", sum(iters) / len(iters)))
@@ -907,8 +910,12 @@ def bench_ours(args):
         gpu_launches = args.steps * (1 if use_bundles else B)
         launches = "one megakernel launch per " + ("step (25-pass bundle)" if use_bundles else "pass")
     else:
-        gpu_launches = args.steps * B * (2 + 2 * cfg.max_path_length)
-        launches = "depth-synchronous wavefront: generate, then trace + shade per depth, per pass"
+        if npix <= 227328 and not r.config.sort_keys:
+            gpu_launches = args.steps * B
+            launches = "one path-kernel launch per pass"
+        else:
+            gpu_launches = args.steps * B * (2 + 2 * cfg.max_path_length)
+            launches = "depth-synchronous wavefront: generate, then trace + shade per depth, per pass"
     torch.cuda.synchronize()
 
     # ---- end to end through the public API with host buffers, at the

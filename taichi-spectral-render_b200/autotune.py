@@ -7,10 +7,8 @@ only its cost.  Knobs:
   * BVH node width 2 / 4 / 8, and for 4 / 8 full-precision or quantized
     child boxes (the scene is re-uploaded per layout; the host builder's tree
     is reused),
-  * traversal loop of two-child nodes (default if-if / speculative while-while),
   * kernel: the persistent megakernel or the wavefront stages, and for the
-    wavefront its queue sorting (sort_keys bit mask), the traversal steps
-    between lane refills (trace_budget) and, for wavelength bundles, the
+    wavefront its queue sorting (sort_keys bit mask) and, for wavelength bundles, the
     queue capacity of the regenerating loop (path slots: how many passes'
     paths are in flight at once),
   * threads per block and resident blocks per SM of the persistent grid, and
