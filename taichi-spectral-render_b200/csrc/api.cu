@@ -626,8 +626,9 @@ ts_status ts_record_paths(ts_ctx *c, uint32_t first_pass, int32_t num_passes) {
 // to cold instruction caches.  us per pass, stages / one kernel: box 64^2 450 / 314,
 // 256^2 702 / 682, 400^2 1019 / 870; terrain (647k triangles) 64^2 336 / 234, 448^2
 // 976 / 704; volume 64^2 2274 / 1990, 448^2 8681 / 8771, 512^2 8987 / 10831.
+// Paths of no vertex have no stage, while the path kernel takes one vertex before it looks.
 static bool pass_in_one_kernel(const ts_ctx *c) {
-  return c->cfg.queue_capacity == 0 && c->cfg.sort_keys == 0 &&
+  return c->cfg.queue_capacity == 0 && c->cfg.sort_keys == 0 && c->cfg.max_path_length > 0 &&
          (int64_t)c->cfg.width * c->cfg.height <= 148 * 1024 * 3 / 2;
 }
 
