@@ -440,7 +440,7 @@ ts_status ts_upload_scene(ts_ctx *c, const ts_scene_desc *sd) {
   c->info.num_nodes = bvh.width == 2            ? bvh.two_child_nodes
                       : !bvh.node_own.empty() ? (int)(bvh.node_own.size() / ts::node_float4s(8))
                                               : ds.num_nodes;
-  c->info.num_ref_nodes = ds.num_ref_nodes;
+  c->info.num_ref_nodes = bvh.num_ref_nodes;
   c->info.max_depth = bvh.max_depth;
   c->info.leaves = bvh.leaves;
   c->info.sah_cost = bvh.sah_cost;
@@ -511,7 +511,7 @@ ts_status ts_build_bvh_host(int32_t T, const float *v0, const float *v1, const f
   ts::BvhOut b;
   std::string err;
   if (!ts::build_bvh_binned(T, v0, v1, v2, p, b, err)) return fail(nullptr, TS_ERR_INVALID_ARG, "ts_build_bvh_host: " + err);
-  const int N = (int)b.ref_link.size();
+  const int N = b.num_ref_nodes;
   *num_nodes_out = N;
   if (N > max_nodes || (N > 0 && (!nmin || !nmax || !left || !right || !ntris || !tstart)))
     return fail(nullptr, TS_ERR_CAPACITY, "ts_build_bvh_host: output arrays hold " + std::to_string(max_nodes) +

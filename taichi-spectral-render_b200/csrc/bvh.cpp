@@ -464,6 +464,23 @@ bool flatten_tree(std::vector<BNode> &&tree, const std::vector<Prim> &prims, con
   // where the wide traversal stack could overflow
   if (!flatten_wide(tree, 4, out)) out.node2.clear();
   out.width = 2;
+  // Leaves that were split: the two-child order visits their halves, nearest
+  // first, while the reference takes such a leaf's triangles in one go.  The
+  // table holds both: the leaf keeps its triangles and gets the links of its
+  // halves, which follow the tree's own nodes.
+  for (int i = 0; i < N; ++i) {
+    const BNode &b = tree[i];
+    if (i < out.num_ref_nodes) {
+      if (out.ref_link[i].z > 0 && b.left >= 0) {
+        out.ref_link[i].x = b.left;
+        out.ref_link[i].y = b.right;
+      }
+      continue;
+    }
+    out.ref_min.insert(out.ref_min.end(), b.lo, b.lo + 3);
+    out.ref_max.insert(out.ref_max.end(), b.hi, b.hi + 3);
+    out.ref_link.push_back(b.left >= 0 ? make_int4(b.left, b.right, 0, 0) : make_int4(-1, -1, b.count, b.first));
+  }
   return true;
 }
 
@@ -506,6 +523,7 @@ bool build_bvh_binned(int T, const float *v0, const float *v1, const float *v2, 
   out.ref_min.resize(3 * (size_t)N);
   out.ref_max.resize(3 * (size_t)N);
   out.ref_link.resize(N);
+  out.num_ref_nodes = N;
   double cost = 0.0;
   const double root_area = half_area(tree[0].lo, tree[0].hi);
   for (int i = 0; i < N; ++i) {
@@ -553,6 +571,7 @@ bool bvh_from_reference(int T, const float *v0, const float *v1, const float *v2
   out.ref_min.assign(nmin, nmin + 3 * (size_t)N);
   out.ref_max.assign(nmax, nmax + 3 * (size_t)N);
   out.ref_link.resize(N);
+  out.num_ref_nodes = N;
   for (int i = 0; i < N; ++i) {
     BNode &b = tree[i];
     for (int a = 0; a < 3; ++a) {

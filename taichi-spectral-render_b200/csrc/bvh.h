@@ -52,7 +52,8 @@ struct BvhOut {
   bool quantized = false;      // node2 holds quantized wide nodes
   int stack_need = 0;          // deepest traversal stack the device layout can require
   std::vector<float> ref_min, ref_max;  // reference layout, [N][3]
-  std::vector<int4> ref_link;           // (left, right, num_tris, tri_start)
+  std::vector<int4> ref_link;           // (left, right, num_tris, tri_start); leaf: left = right = -1, or its halves
+  int num_ref_nodes = 0;                // nodes of the tree; the halves of big leaves follow them (two-child layout)
   int max_depth = 0;
   int leaves = 0;
   double sah_cost = 0.0;

@@ -54,7 +54,7 @@ struct DevScene {
   int32_t node_width;                 // 2, 4 or 8
   const float *__restrict__ ref_min;
   const float *__restrict__ ref_max;
-  const int4 *__restrict__ ref_link;  // (left, right, num_tris, tri_start)
+  const int4 *__restrict__ ref_link;  // (left, right, num_tris, tri_start); a split leaf has both triangles and children
   int32_t num_ref_nodes;
   const float4 *__restrict__ mat;     // [(m*B+band)*2 + 0/1]: (n,k,rough,sigma_s), (emission,g,is_vol,surf_emis)
   const int32_t *__restrict__ mat_eem;

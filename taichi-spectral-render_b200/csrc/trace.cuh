@@ -372,7 +372,8 @@ TS_D bool warp_phase(const DevScene &s, Traversal &t, int2 *stack, float eps, ui
 // run for the rays that the fast loops hand over -- a tie, where those loops
 // visit in another order -- and for the counting pass.
 
-// two children per node, nearest first, over the reference-layout table
+// two children per node, nearest first, over the reference-layout table; a leaf
+// of more than kLeafMax triangles has two halves as its children
 template <bool kCount = false>
 TS_D Hit trace_two_child(const DevScene &s, float3 o, float3 d, float eps, uint32_t &errbits, TraceCount *tc,
                          float bound) {
@@ -394,14 +395,14 @@ TS_D Hit trace_two_child(const DevScene &s, float3 o, float3 d, float eps, uint3
   int ni = 0;
   int4 l = __ldg(s.ref_link);
   bool go = true;
-  if (l.z > 0) {  // the root is a leaf: a node with one child
+  if (l.z > 0 && l.x < 0) {  // the root is a leaf: a node with one child
     float te;
     if (kCount) tc->nodes++;
     go = entry(0, te);
   }
   while (go) {
     bool down = false;
-    if (l.z <= 0) {
+    if (l.z <= 0 || l.x >= 0) {
       float e0, e1;
       if (kCount) tc->nodes++;
       const bool h0 = entry(l.x, e0), h1 = entry(l.y, e1);
