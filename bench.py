@@ -51,7 +51,8 @@ def parse():
     p.add_argument("--traversal", default="default", choices=["default", "speculative"])
     p.add_argument("--leaf-max", type=int, default=0, help="largest BVH leaf the SAH may choose, 1..16 (--no-tune; 0 = 8)")
     p.add_argument("--cost-trav", type=float, default=0.0, help="SAH node-visit cost per triangle test (--no-tune; 0 = 1)")
-    p.add_argument("--occupancy", type=int, default=0, choices=[0, 8], help="megakernel register budget (--no-tune)")
+    p.add_argument("--occupancy", type=int, default=0, choices=[0, 5, 8],
+                   help="megakernel register budget: blocks per SM, 0 = by the paths of a launch (--no-tune)")
     p.add_argument("--launch", default="bundle", choices=["bundle", "pass"],
                    help="render each step's 25 passes in one launch (a wavelength bundle) or one launch per pass")
     p.add_argument("--budget", type=int, default=0, help="wavefront traversal steps between refills")

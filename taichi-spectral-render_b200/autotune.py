@@ -12,7 +12,7 @@ only its cost.  Knobs:
     queue capacity of the regenerating loop (path slots: how many passes'
     paths are in flight at once),
   * threads per block and resident blocks per SM of the persistent grid, and
-    the megakernel's register budget (5 blocks/SM without spills, or 8 with).
+    the megakernel's register budget (for 5 or 8 blocks/SM).
 
 Each candidate renders ``passes`` passes after ``warmup`` (CUDA events on the
 current stream); the fastest wins.  Results are cached in a JSON file keyed by
@@ -59,14 +59,22 @@ class Candidate:
 
 
 def default_candidates(quick=False):
-    out = [Candidate(w, "default", "mega", bs, bpsm) for w in (2, 4, 8) for bs in (64, 128) for bpsm in (0, 5)]
+    # both register budgets by name: 0 leaves the choice to the number of paths of a launch
+    out = [Candidate(w, "default", "mega", bs, bpsm, occupancy=5)
+           for w in (2, 4, 8) for bs in (64, 128) for bpsm in (0, 5)]
     out += [Candidate(w, "default", "mega", 128, 0, occupancy=8) for w in (2, 4, 8)]
-    out += [Candidate(w, "default", "mega", 128, 0, occupancy=o, quantize=True) for w in (4, 8) for o in (0, 8)]
-    out += [Candidate(2, "speculative", "mega", 128, 0), Candidate(2, "speculative", "mega", 128, 0, occupancy=8)]
+    out += [Candidate(w, "default", "mega", 128, 0, occupancy=o, quantize=True) for w in (4, 8) for o in (5, 8)]
+    out += [Candidate(2, "speculative", "mega", 128, 0, occupancy=o) for o in (5, 8)]
     if not quick:
         out += [Candidate(w, "default", "wavefront", 128, 0, sk, tb)
                 for w in (2, 4) for sk in (0, 1) for tb in (16, 32, 64)]
     return out
+
+
+def same_kernels(cand):
+    """The candidate without the knobs that select no kernel (two-child traversal
+    loop, traversal steps between refills): equal results launch the same kernels."""
+    return dataclasses.replace(cand, traversal="default", trace_budget=0)
 
 
 MAX_QUEUE_CAPACITY = 1 << 25
@@ -75,10 +83,9 @@ MAX_QUEUE_CAPACITY = 1 << 25
 def bundle_wavefront_candidates(npix, bands, widths=(2, 4, (4, True), (8, True)), multiples=(2, 4, 8, 16, 32),
                                 budgets=(16, 8)):
     """Regenerating-loop wavefront candidates for wavelength bundles: queue
-    capacities of several frames' worth of path slots (passes in flight),
-    up to the whole bundle, and traversal steps between lane refills (8 is
-    faster on shallow BVHs and deep volume paths, 16 on the 2.6M-triangle
-    terrain)."""
+    capacities of several frames' worth of path slots (passes in flight), up to
+    the whole bundle.  ``budgets`` (trace_budget) selects no kernel: ``tune``
+    times such copies once."""
     caps = sorted({min(m * npix, bands * npix, MAX_QUEUE_CAPACITY) for m in multiples})
     lay = [w if isinstance(w, tuple) else (w, False) for w in widths]
     return [Candidate(w, "default", "wavefront", 256, 0, 0, tb, queue_capacity=qc, quantize=q)
@@ -148,7 +155,11 @@ def tune(scene_dict, cfg, eems=None, cmf=None, candidates=None, passes=6, warmup
         group = [c for c in candidates if (c.width, c.quantize) == layout]
         with Renderer(scene_dict, group[0].apply(cfg), eems=eems, cmf=cmf, bvh=bvh,
                       bvh_params=group[0].bvh_params()) as r:
+            timed = {}
             for cand in group:
+                if same_kernels(cand) in timed:
+                    table.append((cand, timed[same_kernels(cand)]))
+                    continue
                 r.set_launch_config(kernel=cand.kernel, traversal=cand.traversal, block_size=cand.block_size,
                                     blocks_per_sm=cand.blocks_per_sm, sort_keys=cand.sort_keys,
                                     trace_budget=cand.trace_budget, occupancy=cand.occupancy,
@@ -156,6 +167,7 @@ def tune(scene_dict, cfg, eems=None, cmf=None, candidates=None, passes=6, warmup
                 ms = _time_passes(r, passes, warmup, first_pass, bundles)
                 if r.check_device() != 0:
                     ms = float("inf")
+                timed[same_kernels(cand)] = ms
                 table.append((cand, ms))
     best = min(table, key=lambda t: t[1])[0]
     if cache:
