@@ -38,8 +38,10 @@ struct ts_ctx {
   double *d_film[3] = {nullptr, nullptr, nullptr};
   int *d_counter = nullptr;
   uint32_t *d_err = nullptr;
-  float *d_xyz = nullptr;
-  float *d_frame_rgb = nullptr;  // ts_resolve_rgb's image at render resolution
+  // An image at render resolution, which ts_resolve_xyz_host and ts_resolve_rgb pass
+  // through; image_read: its last use, which the next one waits for on its own stream.
+  float *d_image = nullptr;
+  cudaEvent_t image_read = nullptr;
   float4 *d_mat = nullptr;  // packed material table (scene allocation), rewritten by ts_update_materials
   float *d_eem = nullptr, *d_qy = nullptr, *d_cdf = nullptr;
   float *d_adj_weight = nullptr;  // adjoint scratch: per-path weighted totals
@@ -190,8 +192,8 @@ ts_status ts_create(const ts_config *cfg, ts_ctx **out) {
   c->film_bytes = 3 * cells * sizeof(double);
   e = cudaMalloc((void **)&c->d_counter, 64 * sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_err, sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xyz, (size_t)k.width * k.height * 3 * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_frame_rgb, (size_t)k.width * k.height * 3 * sizeof(float));
+  if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_image, (size_t)k.width * k.height * 3 * sizeof(float));
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->image_read, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, sizeof(uint32_t));
   if (e != cudaSuccess) {
     ts_destroy(c);
@@ -237,8 +239,8 @@ ts_status ts_destroy(ts_ctx *c) {
   for (double *p : c->d_film) cudaFree(p);
   cudaFree(c->d_counter);
   cudaFree(c->d_err);
-  cudaFree(c->d_xyz);
-  cudaFree(c->d_frame_rgb);
+  cudaFree(c->d_image);
+  if (c->image_read) cudaEventDestroy(c->image_read);
   cudaFree(c->d_adj_weight);
   cudaFree(c->d_rec);
   delete c;
@@ -812,10 +814,12 @@ ts_status ts_resolve_xyz(ts_ctx *c, double scale, float *xyz_dev, void *stream) 
 
 ts_status ts_resolve_xyz_host(ts_ctx *c, double scale, float *xyz_host, void *stream) {
   if (!c || !xyz_host) return fail(c, TS_ERR_INVALID_ARG, "ts_resolve_xyz_host: bad argument");
-  ts_status s = ts_resolve_xyz(c, scale, c->d_xyz, stream);
+  cudaSetDevice(c->cfg.device);
+  TS_CUDA(c, cudaStreamWaitEvent(as_stream(stream), c->image_read, 0), "resolve xyz");
+  ts_status s = ts_resolve_xyz(c, scale, c->d_image, stream);
   if (s != TS_OK) return s;
   const size_t n = (size_t)c->cfg.width * c->cfg.height * 3;
-  TS_CUDA(c, cudaMemcpyAsync(xyz_host, c->d_xyz, n * sizeof(float), cudaMemcpyDeviceToHost, as_stream(stream)),
+  TS_CUDA(c, cudaMemcpyAsync(xyz_host, c->d_image, n * sizeof(float), cudaMemcpyDeviceToHost, as_stream(stream)),
           "resolve xyz copy");
   TS_CUDA(c, cudaStreamSynchronize(as_stream(stream)), "resolve xyz sync");
   return TS_OK;
@@ -828,9 +832,18 @@ ts_status ts_resolve_rgb(ts_ctx *c, double scale, const float M[9], float exposu
   cudaSetDevice(c->cfg.device);
   ts::ColorMatrix m;
   std::copy(M, M + 9, m.m);
-  TS_CUDA(c, ts::launch_resolve_rgb(film_of(c), c->d_cmf, scale, c->d_frame_rgb, m, exposure, gamma, iw, ih, rgb_dev,
-                                    as_stream(stream)),
+  const cudaStream_t st = as_stream(stream);
+  // The buffer's uses are ordered by an event, so calls on several streams do not
+  // write into one another's image.  A captured call can be replayed at any time,
+  // beside any other: it does without the buffer.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  TS_CUDA(c, cudaStreamIsCapturing(st, &capture), "resolve rgb");
+  const bool by_frame = ts::resolve_rgb_by_frame(film_of(c), iw, ih) && capture == cudaStreamCaptureStatusNone;
+  if (by_frame) TS_CUDA(c, cudaStreamWaitEvent(st, c->image_read, 0), "resolve rgb");
+  TS_CUDA(c, ts::launch_resolve_rgb(film_of(c), c->d_cmf, scale, by_frame ? c->d_image : nullptr, m, exposure, gamma,
+                                    iw, ih, rgb_dev, st),
           "resolve rgb");
+  if (by_frame) TS_CUDA(c, cudaEventRecord(c->image_read, st), "resolve rgb");
   return TS_OK;
 }
 

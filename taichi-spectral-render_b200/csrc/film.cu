@@ -101,8 +101,8 @@ __device__ __forceinline__ int source_of(int i, int n, int size) {
   return (int)((float)i / (float)n * (float)size);
 }
 
-// Whole color_rays (main.py:1609-1629) of an image with fewer pixels than the
-// frame: nearest-neighbour, XYZ -> RGB, tone mapping.  Output [j][i][3].
+// Whole color_rays (main.py:1609-1629), every image pixel by itself:
+// nearest-neighbour, XYZ -> RGB, tone mapping.  Output [j][i][3].
 __global__ void k_resolve_rgb(const Film f, const float *__restrict__ cmf, double scale, const __grid_constant__ ColorMatrix M,
                               float exposure, float gamma, int iw, int ih, float *__restrict__ rgb) {
   __shared__ double cmf64[3 * kMaxBands];
@@ -303,13 +303,17 @@ cudaError_t launch_resolve_xyz(Film f, const float *cmf, double scale, float *xy
   k_resolve_xyz<<<grid_for((size_t)f.W * f.H), kThreads, 0, st>>>(f, cmf, scale, xyz);
   return cudaGetLastError();
 }
-cudaError_t launch_resolve_rgb(Film f, const float *cmf, double scale, float *frame_rgb, ColorMatrix M, float exposure,
-                               float gamma, int iw, int ih, float *rgb, cudaStream_t st) {
+bool resolve_rgb_by_frame(const Film &f, int iw, int ih) {
   // An image of at least the frame's pixels repeats them: each is resolved and
   // tone-mapped once, then copied.  1024^2 frame, 1600^2 image: 135 us when every
-  // image pixel read the film and took its own powers, 59 us so.  Small images
-  // are shorter than the second launch.
-  if ((int64_t)iw * ih >= (int64_t)f.W * f.H && (int64_t)iw * ih > (1 << 18)) {
+  // image pixel read the film and took its own powers, 59 us so; in one kernel, whose
+  // blocks kept the colours under a tile of the image in shared memory, 112 us.
+  // Small images are shorter than the second launch.
+  return (int64_t)iw * ih >= (int64_t)f.W * f.H && (int64_t)iw * ih > (1 << 18);
+}
+cudaError_t launch_resolve_rgb(Film f, const float *cmf, double scale, float *frame_rgb, ColorMatrix M, float exposure,
+                               float gamma, int iw, int ih, float *rgb, cudaStream_t st) {
+  if (frame_rgb) {
     k_frame_rgb<<<grid_for((size_t)f.W * f.H), kThreads, 0, st>>>(f, cmf, scale, M, exposure, gamma, frame_rgb);
     const dim3 grid((unsigned)((iw - 1) / kThreads + 1), (unsigned)std::min(ih, 65535));
     k_upscale<<<grid, kThreads, 0, st>>>(frame_rgb, f.W, f.H, iw, ih, rgb);

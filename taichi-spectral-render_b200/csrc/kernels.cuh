@@ -43,7 +43,9 @@ cudaError_t launch_resolve_xyz(Film f, const float *cmf, double scale, float *xy
 struct ColorMatrix {
   float m[9];  // XYZ -> RGB, row-major
 };
-// frame_rgb: [H][W][3] scratch
+// whether an image of this size is faster by way of the frame's colours
+bool resolve_rgb_by_frame(const Film &f, int img_w, int img_h);
+// frame_rgb: [H][W][3] scratch for the frame's colours; nullptr: without
 cudaError_t launch_resolve_rgb(Film f, const float *cmf, double scale, float *frame_rgb, ColorMatrix xyz_to_rgb,
                                float exposure, float gamma, int img_w, int img_h, float *rgb, cudaStream_t st);
 cudaError_t launch_render_normals(const DevScene &s, const DevConfig &c, float *out, uint32_t *err,
