@@ -465,6 +465,11 @@ __global__ void __launch_bounds__(128) k_trace_ties(const __grid_constant__ DevS
 // 512^2 10.4 / 10.9.
 constexpr int kGroupPaths = 148 * 1024 * 3 / 2;
 
+// full-precision nodes: a quantized node's children have no record per lane
+inline bool in_groups(const DevScene &s, int paths) {
+  return s.node_width != 5 && s.node_width != 9 && paths <= kGroupPaths;
+}
+
 // a stage of a pass, or of the loop (plainly: it is captured as the body of a while node)
 template <bool kLoop, class... Params, class... Args>
 void trace_launch(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
@@ -477,7 +482,7 @@ void launch_trace_w(const DevScene &s, const DevConfig &c, int depth, Film f, co
                     int grid, int block, cudaStream_t st, int ext_sorted, int shadow_sorted, WaveLoop *L,
                     int paths) {
   if constexpr (W != 5 && W != 9) {
-    if (paths <= kGroupPaths) {
+    if (in_groups(s, paths)) {
       const size_t smem = (size_t)(block / kGroupLanes) * kGroupStack * sizeof(int2);
       trace_launch<kLoop>(k_trace<W, kLoop, true>, resident_grid(grid, block, kWideThreads), block, smem, st, s, c, depth,
                           f, w, err, ext_sorted, shadow_sorted, L);
@@ -890,30 +895,36 @@ cudaError_t launch_wave_chunk(const DevScene &s, const DevConfig &c, uint32_t pa
 }
 
 struct WaveLoopGraph {
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  // the two trace stages: launches of one scene and launch configuration that
+  // differ only in their paths take one or the other
+  struct Loop {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    std::vector<unsigned char> key;  // the captured kernel arguments
+  } loop[2];                         // [a group of lanes per ray]
   cudaStream_t capture = nullptr;
-  std::vector<unsigned char> key;  // the captured kernel arguments
 };
 
 void free_wave_loop(WaveLoopGraph *g) {
   if (!g) return;
-  if (g->exec) cudaGraphExecDestroy(g->exec);
-  if (g->graph) cudaGraphDestroy(g->graph);
+  for (WaveLoopGraph::Loop &l : g->loop) {
+    if (l.exec) cudaGraphExecDestroy(l.exec);
+    if (l.graph) cudaGraphDestroy(l.graph);
+  }
   if (g->capture) cudaStreamDestroy(g->capture);
   delete g;
 }
 
 namespace {
 
-cudaError_t build_wave_loop(WaveLoopGraph &G, const DevScene &s, const DevConfig &c, Film f, const WaveBuffers &w,
-                            uint32_t *err, int grid, int block, int paths) {
+cudaError_t build_wave_loop(WaveLoopGraph::Loop &G, cudaStream_t &capture, const DevScene &s, const DevConfig &c, Film f,
+                            const WaveBuffers &w, uint32_t *err, int grid, int block, int paths) {
   if (G.exec) cudaGraphExecDestroy(G.exec);
   if (G.graph) cudaGraphDestroy(G.graph);
   G.exec = nullptr;
   G.graph = nullptr;
   cudaError_t e;
-  if (!G.capture && (e = cudaStreamCreateWithFlags(&G.capture, cudaStreamNonBlocking)) != cudaSuccess) return e;
+  if (!capture && (e = cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking)) != cudaSuccess) return e;
   if ((e = cudaGraphCreate(&G.graph, 0)) != cudaSuccess) return e;
   cudaGraphConditionalHandle h;
   if ((e = cudaGraphConditionalHandleCreate(&h, G.graph, 1, cudaGraphCondAssignDefault)) != cudaSuccess) return e;
@@ -925,15 +936,15 @@ cudaError_t build_wave_loop(WaveLoopGraph &G, const DevScene &s, const DevConfig
   cudaGraphNode_t node;
   if ((e = cudaGraphAddNode(&node, G.graph, nullptr, 0, &cp)) != cudaSuccess) return e;
   cudaGraph_t body = cp.conditional.phGraph_out[0];
-  if ((e = cudaStreamBeginCaptureToGraph(G.capture, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
+  if ((e = cudaStreamBeginCaptureToGraph(capture, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
       cudaSuccess)
     return e;
-  launch_trace<true>(s, c, 0, f, w, err, grid, block, G.capture, paths, 0, 0, w.loop);
-  k_shade_loop<<<resident_grid(grid, block, kStageThreads), block, 0, G.capture>>>(s, c, f, w, w.loop, err);
-  k_loop_control<<<1, 32, 0, G.capture>>>(w.loop, h, 1, err);
+  launch_trace<true>(s, c, 0, f, w, err, grid, block, capture, paths, 0, 0, w.loop);
+  k_shade_loop<<<resident_grid(grid, block, kStageThreads), block, 0, capture>>>(s, c, f, w, w.loop, err);
+  k_loop_control<<<1, 32, 0, capture>>>(w.loop, h, 1, err);
   const cudaError_t le = cudaGetLastError();
   cudaGraph_t captured = nullptr;
-  e = cudaStreamEndCapture(G.capture, &captured);
+  e = cudaStreamEndCapture(capture, &captured);
   if (le != cudaSuccess) return le;
   if (e != cudaSuccess) return e;
   return cudaGraphInstantiate(&G.exec, G.graph, 0);
@@ -963,7 +974,7 @@ cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pas
     Film f;
     WaveBuffers w;
     uint32_t *err;
-    int grid, block, paths;
+    int grid, block;
   } k;
   memset(&k, 0, sizeof k);
   memcpy(&k.s, &s, sizeof s);
@@ -978,7 +989,6 @@ cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pas
   k.err = err;
   k.grid = grid;
   k.block = block;
-  k.paths = n0;
   const unsigned char *kb = reinterpret_cast<const unsigned char *>(&k);
   if (host_driven) {
     const int init_grid = (int)((n0 + 255) / 256 < 4096 ? (n0 + 255) / 256 : 4096);
@@ -996,10 +1006,10 @@ cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pas
     return cudaGetLastError();
   }
   if (!*graph) *graph = new WaveLoopGraph;
-  WaveLoopGraph &G = **graph;
+  WaveLoopGraph::Loop &G = (*graph)->loop[in_groups(s, n0) ? 1 : 0];
   if (!G.exec || G.key.size() != sizeof k || memcmp(G.key.data(), kb, sizeof k) != 0) {
     G.key.clear();
-    const cudaError_t e = build_wave_loop(G, s, c, f, w, err, grid, block, n0);
+    const cudaError_t e = build_wave_loop(G, (*graph)->capture, s, c, f, w, err, grid, block, n0);
     if (e != cudaSuccess) return e;
     G.key.assign(kb, kb + sizeof k);
   }
