@@ -26,6 +26,12 @@ struct Film {
 // largest scene whose vertices a block's warps take together (mega_path.cuh)
 constexpr int kTogetherTris = 32768;
 
+// Passes of few paths, by what runs them: a group of lanes per ray up to kFewPaths
+// (the trace stages, trace_way()), the path kernel in place of the stages up to
+// kPassPaths, or kFewPaths where a medium scatters (pass_in_one_kernel()).
+constexpr int kFewPaths = 148 * 768;
+constexpr int kPassPaths = 148 * 1536;
+
 // npass consecutive sample passes (cast_rays) from pass / band, band wrapping
 // mod B (npass <= B): persistent megakernel with per-lane path regeneration.
 // work != nullptr selects the counting variant (work[8], accumulated)

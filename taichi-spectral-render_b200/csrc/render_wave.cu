@@ -148,9 +148,11 @@ __global__ void k_generate(const __grid_constant__ DevScene s, const __grid_cons
 
 // ---- the trace stage ---------------------------------------------------------
 // Work items are shadow queries (a query's whole chain of segments) and extension
-// rays.  Two ways to run them, for the same results: a ray per lane, the lanes of
-// a warp stepping together (trace_lanes), and a group of lanes per ray
-// (trace_groups).  launch_trace() says which when.
+// rays.  Three ways to run them, for the same results: a ray per lane, the lanes of
+// a warp stepping together or each at its own pace (trace_lanes), and a group of
+// lanes per ray (trace_groups).  trace_way() says which when.
+enum class Way { kTogether, kOwnPace, kGroups };
+
 struct TraceItems {
   int nsh, total;           // shadow queries [0, nsh), then extension rays
   const int *q;             // path slots of the extension rays
@@ -290,16 +292,22 @@ __device__ __noinline__ void item_plain(const DevScene &s, const DevConfig &c, c
   if (ss.total > 1e-6f) deposit(f, pixel, dep_band, q.contrib * ss.total, shared);
 }
 
-// A ray per lane.  A warp looks every kPhases phases for lanes that have
-// finished, and ends their items and starts others once kIdleLanes of them wait:
-// the end of a shadow segment is as long as three node tests, and when every
-// finished lane had its own, it ran with two lanes of 32.
+// A ray per lane.
+// Together: a warp looks every kPhases phases for lanes that have finished, and
+// ends their items and starts others once kIdleLanes of them wait: the end of a
+// shadow segment is as long as three node tests, and when every finished lane had
+// its own, it ran with two lanes of 32.
+// Own pace: kSteps steps of each lane between looks, and few items are spread over
+// the lanes of all warps.  More instructions, and a ray waits for no other: where
+// the schedulers are not full, a ray's own chain of loads is the time.
 constexpr int kPhases = 4;      // 1: 5 % slower, 8: the same
 constexpr int kIdleLanes = 16;  // 4 / 8 / 12: 11 / 5 / 1 % slower, 20: 3 % slower on the volume
+constexpr int kSteps = 16;      // 8: 1-2 % slower with full-precision nodes, up to 4 % faster with quantized ones
+constexpr int kIdlePaced = 8;   // 1: up to 2 % slower
 
 // A tied item goes to a list (k_trace_ties): a call to trace_plain() in this
 // kernel, wherever it stood, cost the stage 16 to 20 %.
-template <int W, class Src>
+template <int W, bool kTogether, class Src>
 __device__ __forceinline__ void trace_lanes(const Src &src, const WaveBuffers &w, const TraceItems &it,
                                             uint32_t &eb) {
   constexpr unsigned kFull = 0xffffffffu;
@@ -308,12 +316,12 @@ __device__ __forceinline__ void trace_lanes(const Src &src, const WaveBuffers &w
   t.node = kTravDone;
   t.tie = 0;
   int2 stack[kWideStack];
-  bool exhausted = false;
+  bool exhausted = kTogether ? false : (int)(threadIdx.x & 31) >= warp_share(it.total, 32);
   const auto begin = [&](const DevScene &s, float3 o, float3 d, float bound) { trav_begin<W>(s, t, o, d, bound); };
   for (;;) {
     const bool done = t.node == kTravDone;
     const unsigned idle = __ballot_sync(kFull, done && !(exhausted && im.id < 0));
-    if (__popc(idle) >= kIdleLanes || __ballot_sync(kFull, !done) == 0) {
+    if (__popc(idle) >= (kTogether ? kIdleLanes : kIdlePaced) || __ballot_sync(kFull, !done) == 0) {
       if (done && im.id >= 0) {
         if (trav_tied<W>(t)) {
           (im.shadow ? w.shadow_queue : w.sorted)[atomicAdd(it.ties + (im.shadow ? 0 : 1), 1)] = im.id;
@@ -332,9 +340,15 @@ __device__ __forceinline__ void trace_lanes(const Src &src, const WaveBuffers &w
     }
     const DevScene &s = src.scene(im.view);
     const float eps = src.config(im.view).eps;
+    if constexpr (kTogether) {
 #pragma unroll 1
-    for (int i = 0; i < kPhases; ++i)
-      if (!warp_phase<Nodes<W>::value>(s, t, stack, eps, eb)) break;
+      for (int i = 0; i < kPhases; ++i)
+        if (!warp_phase<Nodes<W>::value>(s, t, stack, eps, eb)) break;
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < kSteps && t.node != kTravDone; ++i) trav_step<Nodes<W>::value>(s, t, stack, eps, eb);
+      __syncwarp();
+    }
   }
 }
 
@@ -422,21 +436,21 @@ __device__ __forceinline__ TraceItems trace_items(const DevConfig &c, int depth,
   return it;
 }
 
-template <int W, bool kLoop, bool kGroups>
-__global__ void __launch_bounds__(kMaxBlock, (kGroups ? kWideThreads : kStageThreads) / kMaxBlock) k_trace(const __grid_constant__ DevScene s,
+template <int W, bool kLoop, Way kWay>
+__global__ void __launch_bounds__(kMaxBlock, (kWay == Way::kGroups ? kWideThreads : kStageThreads) / kMaxBlock) k_trace(const __grid_constant__ DevScene s,
                                                      const __grid_constant__ DevConfig c, int depth,
                                                      const __grid_constant__ Film f,
                                                      const __grid_constant__ WaveBuffers w,
                                                      uint32_t *__restrict__ err, int ext_sorted,
                                                      int shadow_sorted, WaveLoop *L) {
-  extern __shared__ int2 group_stacks[];  // kGroups: [kGroupStack][groups of the block]
+  extern __shared__ int2 group_stacks[];  // groups: [kGroupStack][groups of the block]
   uint32_t eb = 0;
   if (!kLoop) stage_begin();
   const TraceItems it = trace_items<kLoop>(c, depth, w, ext_sorted, shadow_sorted, L);
   if (it.total <= 0) return;
   const OneScene src{s, c, f, kLoop && L->shared != 0};
-  if constexpr (kGroups) trace_groups<W>(src, w, it, group_stacks, eb);
-  else trace_lanes<W>(src, w, it, eb);
+  if constexpr (kWay == Way::kGroups) trace_groups<W>(src, w, it, group_stacks, eb);
+  else trace_lanes<W, kWay == Way::kTogether>(src, w, it, eb);
   if (eb) atomicOr(err, eb);
 }
 
@@ -456,18 +470,33 @@ __global__ void __launch_bounds__(128) k_trace_ties(const __grid_constant__ DevS
   if (eb) atomicOr(err, eb);
 }
 
-// Groups of lanes up to this many path slots, a ray per lane above.  A ray per
-// lane costs half the instructions of a group per step once the schedulers are
-// full; below that the length of a warp's step counts, where a group's is a
-// third.  Measured per pass (ms, lanes / groups): box 256^2 1.10 / 0.88, 384^2
-// 1.23 / 1.15, 512^2 1.44 / 1.56; terrain (647k triangles) 256^2 1.36 / 0.89,
-// 512^2 1.72 / 1.38, 1024^2 2.76 / 3.21; volume 256^2 7.6 / 5.1, 384^2 8.7 / 7.4,
-// 512^2 10.4 / 10.9.
-constexpr int kGroupPaths = 148 * 1024 * 3 / 2;
+// The way by the paths under way (slots of the loop, pixels of a pass) and the tree.
+// A group of lanes makes a ray's step a third as long and costs twice the
+// instructions, so it wins while the schedulers are mostly empty; stepping together
+// saves a quarter of the instructions and wins once they are full.  A pass has its
+// last stages to run with few paths, and a large tree waits longer for its loads:
+// both move the lines up.
+// Loop of one frame's slots, 25 passes, ms, groups / own pace / together: box 192^2
+// 10.5 / 10.6 / 11.8, 256^2 13.2 / 12.3 / 13.1, 384^2 19.8 / 14.9 / 15.3, 448^2 26.1 /
+// 18.0 / 17.9, 512^2 32.6 / 20.6 / 20.1; volume 192^2 75 / 85 / 99, 256^2 101 / 103 /
+// 114, 384^2 175 / 125 / 131, 512^2 295 / 174 / 171; terrain (647k triangles) 192^2
+// 5.8 / 6.4 / 7.9, 256^2 7.8 / 7.6 / 8.9, 512^2 20.7 / 13.2 / 14.1, (2.6M, 8 passes)
+// 724^2 - / 8.2 / 8.7, 1024^2 - / 13.2 / 13.3, 1448^2 - / 22.7 / 21.9.
+// One pass, us: box 256^2 716 / 759 / 988, 384^2 987 / 935 / 1089, 640^2 - / 1406 /
+// 1579, 1024^2 - / 2541 / 2541, 1600^2 - / 5315 / 4940; volume 256^2 4311 / 4834 /
+// 6896, 640^2 - / 10340 / 11113, 1024^2 - / 21135 / 20269; terrain (2.6M) 640^2 - /
+// 1475 / 2198, 1024^2 - / 2297 / 3109, 1600^2 - / 3954 / 4682.
+constexpr int kGroupSlots = 148 * 384;
+constexpr int kPacedSlots = 148 * 1536, kPacedSlotsLargeTree = 148 * 7168;   // of the loop
+constexpr int kPacedPaths = 148 * 4096, kPacedPathsLargeTree = 148 * 16384;  // of a pass
 
-// full-precision nodes: a quantized node's children have no record per lane
-inline bool in_groups(const DevScene &s, int paths) {
-  return s.node_width != 5 && s.node_width != 9 && paths <= kGroupPaths;
+template <bool kLoop>
+inline Way trace_way(const DevScene &s, int paths) {
+  const bool records = s.node_width != 5 && s.node_width != 9;  // a quantized node's children have no record per lane
+  if (records && paths <= (kLoop ? kGroupSlots : kFewPaths)) return Way::kGroups;
+  const bool large = s.num_tris > kTogetherTris;
+  const int paced = kLoop ? (large ? kPacedSlotsLargeTree : kPacedSlots) : (large ? kPacedPathsLargeTree : kPacedPaths);
+  return paths <= paced ? Way::kOwnPace : Way::kTogether;
 }
 
 // a stage of a pass, or of the loop (plainly: it is captured as the body of a while node)
@@ -481,16 +510,21 @@ template <int W, bool kLoop>
 void launch_trace_w(const DevScene &s, const DevConfig &c, int depth, Film f, const WaveBuffers &w, uint32_t *err,
                     int grid, int block, cudaStream_t st, int ext_sorted, int shadow_sorted, WaveLoop *L,
                     int paths) {
+  const Way way = trace_way<kLoop>(s, paths);
   if constexpr (W != 5 && W != 9) {
-    if (in_groups(s, paths)) {
+    if (way == Way::kGroups) {
       const size_t smem = (size_t)(block / kGroupLanes) * kGroupStack * sizeof(int2);
-      trace_launch<kLoop>(k_trace<W, kLoop, true>, resident_grid(grid, block, kWideThreads), block, smem, st, s, c, depth,
-                          f, w, err, ext_sorted, shadow_sorted, L);
+      trace_launch<kLoop>(k_trace<W, kLoop, Way::kGroups>, resident_grid(grid, block, kWideThreads), block, smem, st, s, c,
+                          depth, f, w, err, ext_sorted, shadow_sorted, L);
       return;
     }
   }
-  trace_launch<kLoop>(k_trace<W, kLoop, false>, grid, block, (size_t)0, st, s, c, depth, f, w, err, ext_sorted,
-                      shadow_sorted, L);
+  if (way == Way::kTogether)
+    trace_launch<kLoop>(k_trace<W, kLoop, Way::kTogether>, grid, block, (size_t)0, st, s, c, depth, f, w, err, ext_sorted,
+                        shadow_sorted, L);
+  else
+    trace_launch<kLoop>(k_trace<W, kLoop, Way::kOwnPace>, resident_grid(grid, block, kStageThreads), block, (size_t)0, st, s,
+                        c, depth, f, w, err, ext_sorted, shadow_sorted, L);
   if constexpr (kWalkedAsFour<W>)
     trace_launch<kLoop>(k_trace_ties<W, kLoop>, kSMs, 128, (size_t)0, st, s, c, depth, f, w, err, L);
 }
@@ -895,13 +929,13 @@ cudaError_t launch_wave_chunk(const DevScene &s, const DevConfig &c, uint32_t pa
 }
 
 struct WaveLoopGraph {
-  // the two trace stages: launches of one scene and launch configuration that
-  // differ only in their paths take one or the other
+  // the ways to trace: launches of one scene and launch configuration that differ
+  // only in their paths take one or another
   struct Loop {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     std::vector<unsigned char> key;  // the captured kernel arguments
-  } loop[2];                         // [a group of lanes per ray]
+  } loop[3];                         // by trace_way()
   cudaStream_t capture = nullptr;
 };
 
@@ -1006,7 +1040,7 @@ cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pas
     return cudaGetLastError();
   }
   if (!*graph) *graph = new WaveLoopGraph;
-  WaveLoopGraph::Loop &G = (*graph)->loop[in_groups(s, n0) ? 1 : 0];
+  WaveLoopGraph::Loop &G = (*graph)->loop[(int)trace_way<true>(s, n0)];
   if (!G.exec || G.key.size() != sizeof k || memcmp(G.key.data(), kb, sizeof k) != 0) {
     G.key.clear();
     const cudaError_t e = build_wave_loop(G, (*graph)->capture, s, c, f, w, err, grid, block, n0);
@@ -1097,7 +1131,7 @@ struct BatchScenes {
   __device__ __forceinline__ bool shared(int v) const { return slot_shared(slots[v]); }
 };
 
-template <int W>
+template <int W, bool kTogether>
 __global__ void __launch_bounds__(kMaxBlock, kStageThreads / kMaxBlock) k_trace_bloop(const BatchSlot *__restrict__ slots,
                                                            const __grid_constant__ WaveBuffers w,
                                                            uint32_t *__restrict__ err, WaveLoop *L) {
@@ -1105,7 +1139,7 @@ __global__ void __launch_bounds__(kMaxBlock, kStageThreads / kMaxBlock) k_trace_
   const int a = L->iter & 1;
   const int nsh = L->sh[a ^ 1];
   const TraceItems it{nsh, nsh + L->ext[a], w.queue[a], nullptr, L->fetch + 0, L->ties};
-  trace_lanes<W>(BatchScenes{slots}, w, it, eb);
+  trace_lanes<W, kTogether>(BatchScenes{slots}, w, it, eb);
   if (eb) atomicOr(err, eb);
 }
 
@@ -1185,19 +1219,23 @@ void free_batch_loop(BatchLoopGraph *g) {
 
 namespace {
 
+template <int W>
+void launch_trace_bloop_w(const BatchSlot *slots, const WaveBuffers &w, uint32_t *err, int grid, int block, cudaStream_t st) {
+  if (w.capacity <= kPacedSlots)
+    k_trace_bloop<W, false><<<resident_grid(grid, block, kStageThreads), block, 0, st>>>(slots, w, err, w.loop);
+  else
+    k_trace_bloop<W, true><<<grid, block, 0, st>>>(slots, w, err, w.loop);
+  if constexpr (kWalkedAsFour<W>) k_trace_ties_bloop<W><<<kSMs, 128, 0, st>>>(slots, w, err, w.loop);
+}
+
 cudaError_t launch_trace_bloop(const BatchSlot *slots, const WaveBuffers &w, uint32_t *err, int width, int grid,
                                int block, cudaStream_t st) {
-  if (width == 9) k_trace_bloop<9><<<grid, block, 0, st>>>(slots, w, err, w.loop);
-  else if (width == 5) k_trace_bloop<5><<<grid, block, 0, st>>>(slots, w, err, w.loop);
-  else if (width == 8) {
-    k_trace_bloop<8><<<grid, block, 0, st>>>(slots, w, err, w.loop);
-    k_trace_ties_bloop<8><<<kSMs, 128, 0, st>>>(slots, w, err, w.loop);
-  }
-  else if (width == 4) k_trace_bloop<4><<<grid, block, 0, st>>>(slots, w, err, w.loop);
-  else {
-    k_trace_bloop<2><<<grid, block, 0, st>>>(slots, w, err, w.loop);
-    k_trace_ties_bloop<2><<<kSMs, 128, 0, st>>>(slots, w, err, w.loop);
-  }
+  const auto go = width == 9   ? launch_trace_bloop_w<9>
+                  : width == 5 ? launch_trace_bloop_w<5>
+                  : width == 8 ? launch_trace_bloop_w<8>
+                  : width == 4 ? launch_trace_bloop_w<4>
+                               : launch_trace_bloop_w<2>;
+  go(slots, w, err, grid, block, st);
   return cudaGetLastError();
 }
 

@@ -316,22 +316,27 @@ TS_D void trav_inner(const DevScene &s, Traversal &t, int2 *stack, uint32_t &err
   t.node = ref[0];
 }
 
+// One step of a traversal: an inner node, or a leaf and the pop that follows.
+template <int W, bool kCount = false>
+TS_D void trav_step(const DevScene &s, Traversal &t, int2 *stack, float eps, uint32_t &errbits,
+                    TraceCount *tc = nullptr) {
+  if (t.node >= 0) {
+    if (kCount) tc->nodes++;
+    trav_inner<W>(s, t, stack, errbits);
+  } else {
+    const int first = ~t.node >> 4, cnt = (~t.node & 15) + 1;
+    if (kCount) tc->tris += cnt;
+    const float3 o = trav_origin(t);
+    for (int i = 0; i < cnt; ++i) trav_triangle(s, t, o, first + i, eps);
+    trav_pop(t, stack);
+  }
+}
+
 // A traversal by itself, to its end.
 template <int W, bool kCount = false>
 TS_D void trav_run(const DevScene &s, Traversal &t, int2 *stack, float eps, uint32_t &errbits,
                    TraceCount *tc = nullptr) {
-  while (t.node != kTravDone) {
-    if (t.node >= 0) {
-      if (kCount) tc->nodes++;
-      trav_inner<W>(s, t, stack, errbits);
-    } else {
-      const int first = ~t.node >> 4, cnt = (~t.node & 15) + 1;
-      if (kCount) tc->tris += cnt;
-      const float3 o = trav_origin(t);
-      for (int i = 0; i < cnt; ++i) trav_triangle(s, t, o, first + i, eps);
-      trav_pop(t, stack);
-    }
-  }
+  while (t.node != kTravDone) trav_step<W, kCount>(s, t, stack, eps, errbits, tc);
 }
 
 // One phase of a warp whose lanes step together: inner nodes, or one triangle of
