@@ -323,6 +323,7 @@ ts_status ts_upload_scene(ts_ctx *c, const ts_scene_desc *sd) {
   });
   // ---- materials, main.py:545-561
   std::vector<float4> mat((size_t)M * B * 2);
+  bool media = false;
   for (int m = 0; m < M; ++m)
     for (int b = 0; b < B; ++b) {
       const float *f = sd->mat_f32 + (size_t)m * 6 * B;
@@ -332,6 +333,7 @@ ts_status ts_upload_scene(ts_ctx *c, const ts_scene_desc *sd) {
       std::memcpy(&se, &i[1 * B + b], 4);
       mat[((size_t)m * B + b) * 2 + 0] = make_float4(f[0 * B + b], f[1 * B + b], f[2 * B + b], f[3 * B + b]);
       mat[((size_t)m * B + b) * 2 + 1] = make_float4(f[4 * B + b], f[5 * B + b], iv, se);
+      media |= i[0 * B + b] != 0 && f[3 * B + b] > 0.f;
     }
   // ---- EEM tables: row maximum (quantum yield) and running CDF, float32 in
   // the order the reference's kernels accumulate them (main.py:1247-1272)
@@ -412,6 +414,7 @@ ts_status ts_upload_scene(ts_ctx *c, const ts_scene_desc *sd) {
   ds.node_own = d_node_own ? d_node_own : d_node;
   ds.tri = d_tri;
   ds.shade = d_shade;
+  ds.media = media ? 1 : 0;
   ds.node_width = ts::layout_id(bvh.width, bvh.quantized);  // selects the traversal instantiation
   ds.num_nodes = (int)(bvh.node2.size() / ts::node_float4s(bvh.quantized ? bvh.width : 4, bvh.quantized));
   ds.num_tris = T;
@@ -625,13 +628,15 @@ ts_status ts_record_paths(ts_ctx *c, uint32_t first_pass, int32_t num_passes) {
 
 // A wavefront pass of few paths is one launch of the path kernel: each of its
 // 2 * depth + 1 stages would last as long as its longest ray, and its code comes
-// to cold instruction caches.  us per pass, stages / one kernel: box 64^2 450 / 314,
-// 256^2 702 / 682, 400^2 1019 / 870; terrain (647k triangles) 64^2 336 / 234, 448^2
-// 976 / 704; volume 64^2 2274 / 1990, 448^2 8681 / 8771, 512^2 8987 / 10831.
+// to cold instruction caches.  Where media scatter, lanes that take a second path
+// (from 148 * 640 paths on) keep theirs waiting, and the line is lower.  us per pass,
+// stages / one kernel: box 64^2 457 / 327, 256^2 716 / 658, 448^2 1080 / 986, 512^2
+// 1191 / 1243; terrain (647k triangles) 64^2 348 / 258, 448^2 1108 / 749; volume of
+// depth 24 320^2 4565 / 4268, 384^2 5181 / 5908, of depth 16 384^2 3652 / 4828.
 // Paths of no vertex have no stage, while the path kernel takes one vertex before it looks.
 static bool pass_in_one_kernel(const ts_ctx *c) {
   return c->cfg.queue_capacity == 0 && c->cfg.sort_keys == 0 && c->cfg.max_path_length > 0 &&
-         (int64_t)c->cfg.width * c->cfg.height <= 148 * 1024 * 3 / 2;
+         (int64_t)c->cfg.width * c->cfg.height <= (c->ds.media ? ts::kFewPaths : ts::kPassPaths);
 }
 
 ts_status ts_render_pass(ts_ctx *c, uint32_t pass_idx, int32_t band, void *stream) {

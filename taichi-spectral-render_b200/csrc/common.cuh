@@ -52,6 +52,7 @@ struct DevScene {
   const float4 *__restrict__ shade;
   int32_t num_nodes, num_tris;
   int32_t node_width;                 // 2, 4 or 8
+  int32_t media;                      // some medium scattered when the scene was uploaded (choice of kernels only)
   const float *__restrict__ ref_min;
   const float *__restrict__ ref_max;
   const int4 *__restrict__ ref_link;  // (left, right, num_tris, tri_start); a split leaf has both triangles and children
