@@ -13,7 +13,6 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kSMs = 148;
 constexpr int kTied = -2;               // tri_orig of a ray that k_trace_batch_ties decides
-constexpr int kGroupRays = 148 * 1024;  // largest query with a group of lanes per ray
 
 inline int grid_for(size_t n) {
   size_t g = (n + kThreads - 1) / kThreads;
@@ -339,10 +338,17 @@ cudaError_t launch_trace_batch(const DevScene &s, float eps, const float *rays, 
     k_trace_batch<<<grid_for((size_t)n), kThreads, 0, st>>>(s, eps, rays, n, tri_orig, t, u, v, err);
     return cudaGetLastError();
   }
-  // A group of lanes per ray while a ray per lane would leave the schedulers idle.
-  // us, lanes / groups: 2,062 triangles 16k rays 36 / 24, 128k 61 / 58, 256k 81 / 95;
-  // 2.6M triangles 16k 87 / 57, 128k 124 / 104, 256k 181 / 178, 512k 300 / 342.
-  if (n <= kGroupRays && s.node_width != 5 && s.node_width != 9) {
+  // A group of lanes per ray while a ray per lane would leave the schedulers idle, or
+  // wait for a large tree's nodes.  A ray per lane has a second launch for ties in the
+  // two- and eight-child layouts; the eight-child one's groups have more ties to decide.
+  // us, lanes / groups, layouts of two, four and eight children: 2,062 triangles 16k
+  // rays 58 / 43, 52 / 40, 53 / 42; 64k 63 / 56, 54 / 50, 61 / 55; 80k 62 / 59, 58 / 60,
+  // 58 / 64; 100k 65 / 63, 60 / 65, 64 / 70; 125k 68 / 71, 69 / 76, 64 / 79; 647,258
+  // triangles 64k 121 / 104, 110 / 107, 125 / 111; 100k 134 / 128, 125 / 124 (another
+  // 100k 158 / 133), 136 / 152; 150k 151 / 160, 154 / 163, 168 / 180.
+  const bool large = s.num_tris > kTogetherTris;
+  const int most = kSMs * (s.node_width == 8 ? 512 : large ? 1024 : s.node_width == 2 ? 768 : 512);
+  if (n <= most && s.node_width != 5 && s.node_width != 9) {
     const int share = std::min(32 / kGroupLanes, std::max(1, n / (kSMs * 16)));
     const int warps = (n - 1) / share + 1;
     const auto k = s.node_width == 8   ? k_trace_batch_groups<8>
