@@ -1087,7 +1087,7 @@ ts_status ts_batch_create(const ts_batch_config *cfg, ts_ctx *const *ctxs, int32
   if (e == cudaSuccess) e = cudaMemset(b->d_err, 0, sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemcpy(b->d_slots, b->host.data(), sizeof(ts::BatchSlot) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->d_active, b->active.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = ts::batch_set_smem_limit(n);
+  if (e == cudaSuccess) e = ts::batch_set_smem_limit(b->width, b->cfg.occupancy, b->together);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking);
   if (e == cudaSuccess && b->cfg.kernel == TS_KERNEL_WAVEFRONT) {
     // path slots of the loop: the step's work items (all scenes active), at most queue_capacity

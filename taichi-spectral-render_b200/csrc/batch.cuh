@@ -4,7 +4,7 @@
 
 namespace ts {
 
-constexpr int kBatchMaxScenes = 128;  // slots per batch (block-shared copy: ~45 KB at the maximum)
+constexpr int kBatchMaxScenes = 128;  // slots per batch (block-shared copy: 46 KB at the maximum)
 
 // One scene of a batch.  Written by the host at creation and reset; the step
 // kernels keep item0 / items / npass / pass0 / nblocks up to date on the device.
@@ -56,7 +56,8 @@ cudaError_t launch_batch_loop_step(BatchSlot *slots, int n, BatchHeader *h, cons
                                    const WaveBuffers &w, int width, int grid, int block, int capacity,
                                    int limit, int acc_blocks, cudaStream_t st, BatchLoopGraph **graph, bool use_graph);
 void free_batch_loop(BatchLoopGraph *g);
-cudaError_t batch_set_smem_limit(int n);
+// room for the largest batch's slot table in the batch's render kernel
+cudaError_t batch_set_smem_limit(int width, int occupancy, bool together);
 // one step: prepare (item ranges), render (persistent pool), accumulate, advance; together: mega_vertex's
 cudaError_t launch_batch_step(BatchSlot *slots, int n, BatchHeader *h, const int *active, uint32_t *err, int width,
                               int grid, int block, int acc_blocks, cudaStream_t st, int occupancy, bool together);

@@ -151,16 +151,11 @@ cudaError_t launch_batch_finish(BatchSlot *slots, int n, int acc_blocks, cudaStr
   return cudaGetLastError();
 }
 
-cudaError_t batch_set_smem_limit(int n) {
-  const int bytes = (int)batch_smem_bytes(n);
-  for (int width : {2, 4, 5, 8, 9})
-    for (int occupancy : {0, 8})
-      for (bool together : {false, true}) {
-        const cudaError_t e = cudaFuncSetAttribute(batch_kernel(width, occupancy, together),
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) return e;
-      }
-  return cudaSuccess;
+// A function's limit is the process's: every batch sets the same one, so that a
+// small batch does not lower it under a larger one.
+cudaError_t batch_set_smem_limit(int width, int occupancy, bool together) {
+  return cudaFuncSetAttribute(batch_kernel(width, occupancy, together), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)batch_smem_bytes(kBatchMaxScenes));
 }
 
 }  // namespace ts
