@@ -55,7 +55,8 @@ typedef struct {
   uint32_t scene_id;             /* Philox counter word 2 (distinguishes scenes of a batch) */
   int32_t device;                /* CUDA device ordinal */
   int32_t kernel;                /* TS_KERNEL_MEGA or TS_KERNEL_WAVEFRONT (whose passes of up to 227,328 pixels,
-                                    without queue_capacity and sort_keys, are one launch of the path kernel) */
+                                    113,664 where a medium scatters, without queue_capacity and sort_keys, are one
+                                    launch of the path kernel) */
   int32_t block_size;            /* threads per block of the render kernels, 32..256 (0 = 128) */
   int32_t blocks_per_sm;         /* persistent grid = SMs * blocks_per_sm (0 = default) */
   int32_t sort_keys;             /* wavefront queue sorting, bit mask: 1 shading queue by material,

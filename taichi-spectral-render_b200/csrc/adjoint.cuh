@@ -30,11 +30,7 @@ struct Grad {
   double *sh;
   double *gl;
   int pm_shared;  // entries held in shared memory (0 = none)
-#ifdef NI_ADD
-  __device__ __noinline__ void add(int idx, float v) const {
-#else
   TS_D void add(int idx, float v) const {
-#endif
     if (v == 0.f) return;
     if (idx < pm_shared) atomicAdd(sh + idx, (double)v);
     else atomicAdd(gl + idx, (double)v);
@@ -83,12 +79,7 @@ TS_D CD csqrt(CD z) {
   return {re, im};
 }
 // fresnel() with its partials d/dki (.a) and d/dkt (.b)
-#ifdef NI_FD
-__device__ __noinline__
-#else
-TS_D
-#endif
-D2 fresnel_d(float cos_i, float ni, float ki, float nt, float kt) {
+TS_D D2 fresnel_d(float cos_i, float ni, float ki, float nt, float kt) {
   const float ang = acosf(fminf(fmaxf(cos_i, -1.f), 1.f));
   const D2 Ki = {ki, 1.f, 0.f}, Kt = {kt, 0.f, 1.f};
   const D2 Ni = d2c(ni), Nt = d2c(nt);
@@ -136,12 +127,7 @@ TS_D float ggx_g_dr(float3 n, float3 v, float3 l, float r, float &dg) {
 }
 // Oren-Nayar angular term A + B * X and its derivative in the roughness
 // (sigma = roughness * pi / 2, main.py:1068-1088)
-#ifdef NI_ON
-__device__ __noinline__
-#else
-TS_D
-#endif
-float oren_nayar_dr(float3 n, float3 l, float3 v, float ndl, float ndv, float r, float &don) {
+TS_D float oren_nayar_dr(float3 n, float3 l, float3 v, float ndl, float ndv, float r, float &don) {
   const float sigma = r * kPiF / 2.0f;
   const float s2 = sigma * sigma;
   const float A = 1.0f - s2 / (2.0f * (s2 + 0.33f));

@@ -115,12 +115,7 @@ TS_D Cx csqrt(Cx z) {  // main.py:887-896
   return {re, im};
 }
 // fresnel_spectral, main.py:925-966 (unpolarised, complex permittivities)
-#ifdef NI_F
-__device__ __noinline__
-#else
-TS_D
-#endif
-float fresnel(float cos_i, float ni, float ki, float nt, float kt) {
+TS_D float fresnel(float cos_i, float ni, float ki, float nt, float kt) {
   const float ang = acosf(fminf(fmaxf(cos_i, -1.f), 1.f));
   const Cx e_in = {ni * ni - ki * ki, 2.0f * ni * ki};
   const Cx e_tr = {nt * nt - kt * kt, 2.0f * nt * kt};
@@ -168,12 +163,7 @@ TS_D void oren_nayar_terms(float rough, float &A, float &B) {
   A = 1.0f - s2 / (2.0f * (s2 + 0.33f));
   B = 0.45f * s2 / (s2 + 0.09f);
 }
-#ifdef NI_ON
-__device__ __noinline__
-#else
-TS_D
-#endif
-float oren_nayar_angular(float3 n, float3 l, float3 v, float ndl, float ndv, float A, float B) {
+TS_D float oren_nayar_angular(float3 n, float3 l, float3 v, float ndl, float ndv, float A, float B) {
   const float th_i = acosf(ndl), th_o = acosf(ndv);
   const float al = fmaxf(th_i, th_o), be = fminf(th_i, th_o);
   float cphi = 0.f;

@@ -11,7 +11,6 @@ namespace ts {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kSMs = 148;
 constexpr int kTied = -2;               // tri_orig of a ray that k_trace_batch_ties decides
 
 inline int grid_for(size_t n) {

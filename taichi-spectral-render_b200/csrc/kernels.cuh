@@ -7,6 +7,8 @@
 
 namespace ts {
 
+constexpr int kSMs = 148;  // of a B200: what the kernels' grids and the lines between them are made for
+
 // Film layout: [band][row j][column i] FP64, band-major so that one warp of
 // neighbouring pixels depositing into the same band writes 256 contiguous bytes.
 struct Film {
@@ -29,8 +31,8 @@ constexpr int kTogetherTris = 32768;
 // Passes of few paths, by what runs them: a group of lanes per ray up to kFewPaths
 // (the trace stages, trace_way()), the path kernel in place of the stages up to
 // kPassPaths, or kFewPaths where a medium scatters (pass_in_one_kernel()).
-constexpr int kFewPaths = 148 * 768;
-constexpr int kPassPaths = 148 * 1536;
+constexpr int kFewPaths = kSMs * 768;
+constexpr int kPassPaths = kSMs * 1536;
 
 // npass consecutive sample passes (cast_rays) from pass / band, band wrapping
 // mod B (npass <= B): persistent megakernel with per-lane path regeneration.

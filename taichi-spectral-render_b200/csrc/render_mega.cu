@@ -19,8 +19,10 @@ namespace {
 // work[0..7] = paths, path vertices, traversals, node visits, triangle tests,
 // surface hits resolved, film deposits, (unused).
 // kMinBlocks: resident blocks of 128 threads per SM the compiler must allow
-// (5: 96 registers, no spills; 8: 64 registers with local-memory spills --
-// more warps to hide the node-fetch latency, faster on large frames).
+// (5: 96 registers; four children spill nothing, the layouts that hand ties to
+// trace_plain(), two and eight children, 25 to 90 B, quantized nodes 10 to 210 B.
+// 8: 64 registers with 250 B to 1.2 KB of spills -- more warps to hide the node-fetch
+// latency, faster on large frames).
 // kTogether: the block's warps take each vertex together (mega_vertex).
 template <int W, bool kCount, int kMinBlocks = 5, bool kTogether = false>
 __global__ void __launch_bounds__(128, kMinBlocks) k_render_mega(const __grid_constant__ DevScene s, const __grid_constant__ DevConfig c, uint32_t pass0, int npass, int band0,
@@ -34,7 +36,7 @@ __global__ void __launch_bounds__(128, kMinBlocks) k_render_mega(const __grid_co
   // Few paths: fewer lanes of each warp rather than fewer warps, whose lanes'
   // branches run one after the other.  us per pass, full warps / so: box 32^2
   // 513 / 193, 64^2 506 / 316; terrain 64^2 391 / 241; volume 32^2 3141 / 1081.
-  const int warps = (int)min((int64_t)gridDim.x * (blockDim.x >> 5), (int64_t)148 * kMinBlocks * 4);  // what the device holds
+  const int warps = (int)min((int64_t)gridDim.x * (blockDim.x >> 5), (int64_t)kSMs * kMinBlocks * 4);  // what the device holds
   bool exhausted = lane >= max(1, (total - 1) / warps + 1);
   MegaLane L;
   L.pix = -1;
@@ -80,8 +82,11 @@ void launch_w(const DevScene &s, const DevConfig &c, uint32_t pass0, int npass, 
   // Together where shading, not the length of single traversals, takes the time:
   // small trees and enough paths.  us per pass apart / together: box (2,062
   // triangles) 64^2 306 / 316, 128^2 565 / 468, 192^2 737 / 584, 512^2 1570 / 1217,
-  // volume (20,014) 128^2 3373 / 2640, 192^2 4183 / 3535, bundles of 25 at 256^2
-  // 63 / 63 ms; terrain (647,258) 256^2 568 / 594, 512^2 762 / 829.
+  // volume (20,014) 128^2 3373 / 2640, 192^2 4183 / 3535.  By the size of the tree,
+  // 256^2, 512^2 and a bundle of 25 at 256^2: terrain of 33,000 triangles 421 / 409, 630 /
+  // 586, 2923 / 2493; 65,000 451 / 459, 658 / 635, 3058 / 2678; 130,000 482 / 504, 715 /
+  // 696, 3253 / 2941; 647,258 570 / 590, 814 / 883, 3584 / 3559; volume of 60,000 5151 /
+  // 4881, 12081 / 12092, 63878 / 57318; 200,000 5437 / 5381, 12806 / 13360, 67290 / 63059.
   const bool together = s.num_tris <= kTogetherTris && (int64_t)c.W * c.H * npass >= 16384;
   // Unless the caller chose, 64 registers where there are paths for the 8 blocks of
   // an SM that they allow, several for each lane; with fewer paths the spills cost

@@ -44,8 +44,10 @@ static_assert(kCntTotal <= 8192, "WaveBuffers::counts");
 // serialisation: a stage's blocks come up while the one before drains, and every
 // thread waits for that one's end before it reads or writes anything.  Every
 // block of a stage waits, also one without work, so a stage's end implies the
-// ends of all before it.  A 64^2 pass of 18 launches takes 500 us without, 474 us so;
-// 25 passes at 256^2 19.4 and 18.5 ms.
+// ends of all before it.  us without / so: an allocation-free tile of 64^2 pixels in
+// 17 to 65 stages, box 380 / 351, terrain (647k triangles) 333 / 269, volume 2334 /
+// 2236, of 256^2 546 / 515, 581 / 532, 4365 / 4237; a pass of 1024^2 pixels 2567 / 2568,
+// 2226 / 2139, 19632 / 19581.
 __device__ __forceinline__ void stage_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -73,7 +75,6 @@ void launch_stage(void (*kernel)(Params...), int grid, int block, size_t smem, c
 // then costs a launch and no atomics (11 us before, 2,368 blocks asking in turn).
 // trace_lanes asks for all of its items: it has many, and the code for the first
 // ones cost it 10 %.
-constexpr int kSMs = 148;
 constexpr int kStageThreads = 1024;  // resident threads per SM: trace_lanes, k_shade_loop (64 registers)
 constexpr int kWideThreads = 512;    // trace_groups, k_shade (128 registers)
 
@@ -486,9 +487,9 @@ __global__ void __launch_bounds__(128) k_trace_ties(const __grid_constant__ DevS
 // 1579, 1024^2 - / 2541 / 2541, 1600^2 - / 5315 / 4940; volume 256^2 4311 / 4834 /
 // 6896, 640^2 - / 10340 / 11113, 1024^2 - / 21135 / 20269; terrain (2.6M) 640^2 - /
 // 1475 / 2198, 1024^2 - / 2297 / 3109, 1600^2 - / 3954 / 4682.
-constexpr int kGroupSlots = 148 * 384;
-constexpr int kPacedSlots = 148 * 1536, kPacedSlotsLargeTree = 148 * 7168;   // of the loop
-constexpr int kPacedPaths = 148 * 4096, kPacedPathsLargeTree = 148 * 16384;  // of a pass
+constexpr int kGroupSlots = kSMs * 384;
+constexpr int kPacedSlots = kSMs * 1536, kPacedSlotsLargeTree = kSMs * 7168;   // of the loop
+constexpr int kPacedPaths = kSMs * 4096, kPacedPathsLargeTree = kSMs * 16384;  // of a pass
 
 template <bool kLoop>
 inline Way trace_way(const DevScene &s, int paths) {
@@ -908,7 +909,7 @@ cudaError_t launch_wave_chunk(const DevScene &s, const DevConfig &c, uint32_t pa
     e = cudaMemsetAsync(w.key_hist, 0, 2 * kMaxKeys * sizeof(int), st);
     if (e != cudaSuccess) return e;
   }
-  const int sort_grid = grid < 4 * 148 ? grid : 4 * 148;
+  const int sort_grid = grid < 4 * kSMs ? grid : 4 * kSMs;
   for (int d = 0; d < c.max_depth; ++d) {
     const int ext_sorted = (sort_keys & 2) ? 1 : 0;
     const int sh_sorted = (sort_keys & 4) && d > 0 ? 1 : 0;
