@@ -38,6 +38,17 @@ BYTES_MAT_VERTEX = 8 * 32  # material lookups per path vertex (8 x two float4)
 BYTES_DEPOSIT = 16   # FP64 read-modify-write of a film cell
 
 
+# paths that select a wavefront launch's kernels (render_wave.cu, kernels.cuh): the loop's slots and a pass's
+# pixels with a group of lanes per ray, and the largest pass that is one launch of the path kernel
+LOOP_GROUP_SLOTS, FEW_PATHS, PASS_PATHS = 148 * 384, 148 * 768, 148 * 1536
+
+
+def tie_kernel(info, lanes):
+    """A trace stage with a ray per lane is followed by the kernel that decides ties where the layout is
+    walked as four-child nodes."""
+    return lanes and info["node_width"] in (2, 8) and not info["node_quantized"]
+
+
 def parse():
     p = argparse.ArgumentParser()
     p.add_argument("--gpus", type=int, default=1)
@@ -507,8 +518,9 @@ def adjoint_leg():
     pm, pe = r.param_count()
     adj = torch.rand((B, c.height, c.width), dtype=torch.float64, device="cuda")
     g = torch.zeros(pm + pe, dtype=torch.float64, device="cuda")
+    n = 2 * B
     r.cast_rays_bundle(0, B, pass_idx=0)
-    r.adjoint_passes(0, B, 0, adj, g)
+    r.adjoint_passes(0, n, 0, adj, g)  # the timed size: its scratch is allocated here
     r.cast_rays(0, pass_idx=0)
 
     def timed(fn, n):
@@ -520,7 +532,6 @@ def adjoint_leg():
         torch.cuda.synchronize()
         return a.elapsed_time(b) / n
 
-    n = 2 * B
     f1 = timed(lambda: [r.cast_rays(p % B, pass_idx=1000 + p) for p in range(n)], n)
     fb = timed(lambda: [r.cast_rays_bundle(0, B, pass_idx=1000 + i * B) for i in range(2)], n)
     ab = timed(lambda: r.adjoint_passes(0, n, 1000, adj, g), n)  # both replays
@@ -899,11 +910,9 @@ def bench_ours(args):
                 for b in range(B):
                     r.cast_rays(b, pass_idx=timed_first + k * B + b)
                     iters.append(r.wave_loop_iterations())
-        # a loop launch: the init kernel, then trace + shade + control per iteration, and where the
-        # layout is walked as four-child nodes by a ray per lane, the kernel that decides ties
-        ties = info["node_width"] in (2, 8) and not info["node_quantized"] and min(
-            r.config.queue_capacity, (B if use_bundles else 1) * npix) > 227328
-        gpu_launches = sum(1 + (4 if ties else 3) * it for it in iters)
+        # a loop launch: the init kernel, then trace + shade + control per iteration, and the tie kernel
+        slots = min(r.config.queue_capacity or npix, (B if use_bundles else 1) * npix)
+        gpu_launches = sum(1 + (4 if tie_kernel(info, slots > LOOP_GROUP_SLOTS) else 3) * it for it in iters)
         launches = ("one regenerating wavefront loop per %s (init kernel, then a CUDA-graph while-loop of trace, "
                     "shade, control; %.1f iterations per launch)" % ("step (25-pass bundle)" if use_bundles
                                                                      else "pass", sum(iters) / len(iters)))
@@ -911,11 +920,14 @@ def bench_ours(args):
         gpu_launches = args.steps * (1 if use_bundles else B)
         launches = "one megakernel launch per " + ("step (25-pass bundle)" if use_bundles else "pass")
     else:
-        if npix <= 227328 and not r.config.sort_keys:
+        mat_f, mat_i = r.compiled.mat_f32, r.compiled.mat_i32
+        media = bool(((mat_i[:, 0] != 0) & (mat_f[:, 3] > 0)).any())
+        if npix <= (FEW_PATHS if media else PASS_PATHS) and not r.config.sort_keys:
             gpu_launches = args.steps * B
             launches = "one path-kernel launch per pass"
         else:
-            gpu_launches = args.steps * B * (2 + 2 * cfg.max_path_length)
+            ties = cfg.max_path_length + 1 if tie_kernel(info, npix > FEW_PATHS) else 0
+            gpu_launches = args.steps * B * (2 + 2 * cfg.max_path_length + ties)
             launches = "depth-synchronous wavefront: generate, then trace + shade per depth, per pass"
     torch.cuda.synchronize()
 
