@@ -302,12 +302,14 @@ cudaError_t launch_resolve_xyz(Film f, const float *cmf, double scale, float *xy
   return cudaGetLastError();
 }
 bool resolve_rgb_by_frame(const Film &f, int iw, int ih) {
-  // An image of at least the frame's pixels repeats them: each is resolved and
-  // tone-mapped once, then copied.  1024^2 frame, 1600^2 image: 135 us when every
-  // image pixel read the film and took its own powers, 59 us so; in one kernel, whose
-  // blocks kept the colours under a tile of the image in shared memory, 112 us.
-  // Small images are shorter than the second launch.
-  return (int64_t)iw * ih >= (int64_t)f.W * f.H && (int64_t)iw * ih > (1 << 18);
+  // An image of more pixels than the frame repeats them: each is resolved and
+  // tone-mapped once, then copied.  us, block average aside, every image pixel by
+  // itself / by the frame: 1024^2 to 1600^2 111 / 86, 512^2 to 1024^2 44 / 28, 784x134
+  // to 1568x268 28 / 26; but at the frame's size 1024^2 62 / 78, 700^2 31 / 46, and small
+  // images are shorter than the second launch: 256^2 to 512^2 23 / 24.  In one kernel,
+  // whose blocks kept the colours under a tile of the image in shared memory, 1600^2
+  // took 138.
+  return 2 * (int64_t)iw * ih >= 3 * (int64_t)f.W * f.H && (int64_t)iw * ih > (1 << 18);
 }
 cudaError_t launch_resolve_rgb(Film f, const float *cmf, double scale, float *frame_rgb, ColorMatrix M, float exposure,
                                float gamma, int iw, int ih, float *rgb, cudaStream_t st) {

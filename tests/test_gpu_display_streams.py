@@ -13,7 +13,8 @@ def bits(image):
     return image.view(torch.int32)
 
 
-@pytest.mark.parametrize("frame,image", [((700, 500), (1400, 1000)), ((700, 500), (300, 1300)), ((300, 260), (300, 260))])
+@pytest.mark.parametrize("frame,image", [((700, 500), (1400, 1000)), ((700, 500), (300, 1800)), ((700, 500), (700, 500)),
+                                         ((300, 260), (300, 260))])
 def test_exposures_on_two_streams(frame, image):
     s, c, ex = configs.box_scene(width=frame[0], height=frame[1], sphere_slices=8, sphere_stacks=9)
     c.image_width, c.image_height = image
