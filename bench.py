@@ -38,9 +38,15 @@ BYTES_MAT_VERTEX = 8 * 32  # material lookups per path vertex (8 x two float4)
 BYTES_DEPOSIT = 16   # FP64 read-modify-write of a film cell
 
 
-# paths that select a wavefront launch's kernels (render_wave.cu, kernels.cuh): the loop's slots and a pass's
-# pixels with a group of lanes per ray, and the largest pass that is one launch of the path kernel
+# paths that select a wavefront launch's kernels (render_wave.cu, kernels.cuh): those with a group of lanes per
+# ray, slots of a loop that fills them again or all paths of a launch, and the largest pass that is one launch
+# of the path kernel
 LOOP_GROUP_SLOTS, FEW_PATHS, PASS_PATHS = 148 * 384, 148 * 768, 148 * 1536
+
+
+def few_paths(info):
+    """Most paths of a launch with a group of lanes per ray."""
+    return PASS_PATHS if info["node_width"] == 2 and info["num_tris"] > 32768 else FEW_PATHS
 
 
 def tie_kernel(info, lanes):
@@ -911,8 +917,10 @@ def bench_ours(args):
                     r.cast_rays(b, pass_idx=timed_first + k * B + b)
                     iters.append(r.wave_loop_iterations())
         # a loop launch: the init kernel, then trace + shade + control per iteration, and the tie kernel
-        slots = min(r.config.queue_capacity or npix, (B if use_bundles else 1) * npix)
-        gpu_launches = sum(1 + (4 if tie_kernel(info, slots > LOOP_GROUP_SLOTS) else 3) * it for it in iters)
+        paths = (B if use_bundles else 1) * npix
+        slots = min(r.config.queue_capacity or npix, paths)
+        ties = tie_kernel(info, slots > (LOOP_GROUP_SLOTS if slots < paths else few_paths(info)))
+        gpu_launches = sum(1 + (4 if ties else 3) * it for it in iters)
         launches = ("one regenerating wavefront loop per %s (init kernel, then a CUDA-graph while-loop of trace, "
                     "shade, control; %.1f iterations per launch)" % ("step (25-pass bundle)" if use_bundles
                                                                      else "pass", sum(iters) / len(iters)))
@@ -926,7 +934,7 @@ def bench_ours(args):
             gpu_launches = args.steps * B
             launches = "one path-kernel launch per pass"
         else:
-            ties = cfg.max_path_length + 1 if tie_kernel(info, npix > FEW_PATHS) else 0
+            ties = cfg.max_path_length + 1 if tie_kernel(info, npix > few_paths(info)) else 0
             gpu_launches = args.steps * B * (2 + 2 * cfg.max_path_length + ties)
             launches = "depth-synchronous wavefront: generate, then trace + shade per depth, per pass"
     torch.cuda.synchronize()

@@ -981,6 +981,7 @@ struct ts_batch {
   size_t wave_bytes = 0;
   ts::BatchLoopGraph *loop = nullptr;
   int loop_cap = 0, loop_limit = 0;
+  bool loop_refills = false;  // a step of all scenes has more paths than loop_cap slots
   bool together = true;  // every scene is small enough for mega_vertex's warps together
   std::string err;
 };
@@ -1102,6 +1103,7 @@ ts_status ts_batch_create(const ts_batch_config *cfg, ts_ctx *const *ctxs, int32
     // every slot starts a new item at least once per max_depth iterations while items are left
     const int64_t bound = ((total + cap - 1) / cap + 2) * (int64_t)(depth + 1) + 4;
     b->loop_cap = (int)cap;
+    b->loop_refills = total > cap;
     b->loop_limit = (int)std::min<int64_t>(bound, INT32_MAX);
     e = alloc_wave_buffers(b->wave, b->wave_allocs, b->wave_bytes, b->loop_cap, true);
   }
@@ -1163,7 +1165,7 @@ ts_status ts_batch_step(ts_batch *b, void *stream) {
     TS_BCUDA(b, ts::launch_batch_loop_step(b->d_slots, b->n, b->d_hdr, b->d_active, b->d_err, b->wave, b->width,
                                            b->num_sms * 8, ts::kMaxBlock, b->loop_cap,
                                            b->loop_limit, acc_blocks, as_stream(stream), &b->loop,
-                                           b->cfg.use_graph != 0),
+                                           b->cfg.use_graph != 0, b->loop_refills),
              "ts_batch_step");
     return TS_OK;
   }

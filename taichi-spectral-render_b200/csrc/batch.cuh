@@ -50,11 +50,13 @@ cudaError_t launch_batch_finish(BatchSlot *slots, int n, int acc_blocks, cudaStr
 // of every active slot (render_wave.cu): prepare, loop init, the while-loop of
 // trace -> shade -> control, block averages, pass advance.  With use_graph
 // the whole step is one CUDA graph (built at the first step, replayed after);
-// limit bounds the loop's iterations (kErrIterationCap past it).
+// limit bounds the loop's iterations (kErrIterationCap past it); refills: a step of
+// all scenes has more paths than slots.
 struct BatchLoopGraph;
 cudaError_t launch_batch_loop_step(BatchSlot *slots, int n, BatchHeader *h, const int *active, uint32_t *err,
                                    const WaveBuffers &w, int width, int grid, int block, int capacity,
-                                   int limit, int acc_blocks, cudaStream_t st, BatchLoopGraph **graph, bool use_graph);
+                                   int limit, int acc_blocks, cudaStream_t st, BatchLoopGraph **graph, bool use_graph,
+                                   bool refills);
 void free_batch_loop(BatchLoopGraph *g);
 // room for the largest batch's slot table in the batch's render kernel
 cudaError_t batch_set_smem_limit(int width, int occupancy, bool together);

@@ -28,9 +28,10 @@ struct Film {
 // largest scene whose vertices a block's warps take together (mega_path.cuh)
 constexpr int kTogetherTris = 32768;
 
-// Passes of few paths, by what runs them: a group of lanes per ray up to kFewPaths
-// (the trace stages, trace_way()), the path kernel in place of the stages up to
-// kPassPaths, or kFewPaths where a medium scatters (pass_in_one_kernel()).
+// Passes of few paths, by what runs them: a group of lanes per ray up to kFewPaths, or
+// kPassPaths with two children and a large tree (the trace stages, trace_way()); the
+// path kernel in place of the stages up to kPassPaths, or kFewPaths where a medium
+// scatters (pass_in_one_kernel()).
 constexpr int kFewPaths = kSMs * 768;
 constexpr int kPassPaths = kSMs * 1536;
 

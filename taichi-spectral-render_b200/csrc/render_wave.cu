@@ -471,12 +471,13 @@ __global__ void __launch_bounds__(128) k_trace_ties(const __grid_constant__ DevS
   if (eb) atomicOr(err, eb);
 }
 
-// The way by the paths under way (slots of the loop, pixels of a pass) and the tree.
+// The way by the paths under way (slots of the loop, pixels of a pass), whether slots
+// are filled again as paths end, and the tree.
 // A group of lanes makes a ray's step a third as long and costs twice the
 // instructions, so it wins while the schedulers are mostly empty; stepping together
-// saves a quarter of the instructions and wins once they are full.  A pass has its
-// last stages to run with few paths, and a large tree waits longer for its loads:
-// both move the lines up.
+// saves a quarter of the instructions and wins once they are full.  A pass, or a loop
+// that starts with all of its paths, has its last stages to run with few, and a large
+// tree waits longer for its loads: both move the lines up.
 // Loop of one frame's slots, 25 passes, ms, groups / own pace / together: box 192^2
 // 10.5 / 10.6 / 11.8, 256^2 13.2 / 12.3 / 13.1, 384^2 19.8 / 14.9 / 15.3, 448^2 26.1 /
 // 18.0 / 17.9, 512^2 32.6 / 20.6 / 20.1; volume 192^2 75 / 85 / 99, 256^2 101 / 103 /
@@ -487,16 +488,21 @@ __global__ void __launch_bounds__(128) k_trace_ties(const __grid_constant__ DevS
 // 1579, 1024^2 - / 2541 / 2541, 1600^2 - / 5315 / 4940; volume 256^2 4311 / 4834 /
 // 6896, 640^2 - / 10340 / 11113, 1024^2 - / 21135 / 20269; terrain (2.6M) 640^2 - /
 // 1475 / 2198, 1024^2 - / 2297 / 3109, 1600^2 - / 3954 / 4682.
+// All 25 passes of 140^2 pixels at once (490,000 paths), own pace / together: box 1598 /
+// 1638, volume 11764 / 11558; with quantized eight-child nodes volume 16570 / 15390, of
+// 128^2 (409,600) 14794 / 14280.  A sorted pass of the terrain (647k) at 448^2, groups / own
+// pace: two children, whose ties have a launch of their own then, 1214 / 1262, four
+// 1202 / 1111.
 constexpr int kGroupSlots = kSMs * 384;
-constexpr int kPacedSlots = kSMs * 1536, kPacedSlotsLargeTree = kSMs * 7168;   // of the loop
-constexpr int kPacedPaths = kSMs * 4096, kPacedPathsLargeTree = kSMs * 16384;  // of a pass
+constexpr int kPacedSlots = kSMs * 1536, kPacedSlotsLargeTree = kSMs * 7168;   // filled again
+constexpr int kPacedPaths = kSMs * 2560, kPacedPathsLargeTree = kSMs * 16384;  // not
 
-template <bool kLoop>
-inline Way trace_way(const DevScene &s, int paths) {
+inline Way trace_way(const DevScene &s, int paths, bool refills) {
   const bool records = s.node_width != 5 && s.node_width != 9;  // a quantized node's children have no record per lane
-  if (records && paths <= (kLoop ? kGroupSlots : kFewPaths)) return Way::kGroups;
   const bool large = s.num_tris > kTogetherTris;
-  const int paced = kLoop ? (large ? kPacedSlotsLargeTree : kPacedSlots) : (large ? kPacedPathsLargeTree : kPacedPaths);
+  const int grouped = refills ? kGroupSlots : large && s.node_width == 2 ? kPassPaths : kFewPaths;
+  if (records && paths <= grouped) return Way::kGroups;
+  const int paced = refills ? (large ? kPacedSlotsLargeTree : kPacedSlots) : (large ? kPacedPathsLargeTree : kPacedPaths);
   return paths <= paced ? Way::kOwnPace : Way::kTogether;
 }
 
@@ -510,8 +516,8 @@ void trace_launch(void (*kernel)(Params...), int grid, int block, size_t smem, c
 template <int W, bool kLoop>
 void launch_trace_w(const DevScene &s, const DevConfig &c, int depth, Film f, const WaveBuffers &w, uint32_t *err,
                     int grid, int block, cudaStream_t st, int ext_sorted, int shadow_sorted, WaveLoop *L,
-                    int paths) {
-  const Way way = trace_way<kLoop>(s, paths);
+                    int paths, bool refills) {
+  const Way way = trace_way(s, paths, refills);
   if constexpr (W != 5 && W != 9) {
     if (way == Way::kGroups) {
       const size_t smem = (size_t)(block / kGroupLanes) * kGroupStack * sizeof(int2);
@@ -530,17 +536,18 @@ void launch_trace_w(const DevScene &s, const DevConfig &c, int depth, Film f, co
     trace_launch<kLoop>(k_trace_ties<W, kLoop>, kSMs, 128, (size_t)0, st, s, c, depth, f, w, err, L);
 }
 
-// paths: path slots in use, the most extension rays (and shadow queries) the stage can have
+// paths: path slots in use, the most extension rays (and shadow queries) the stage can
+// have; refills: ended paths' slots take other paths
 template <bool kLoop = false>
 void launch_trace(const DevScene &s, const DevConfig &c, int depth, Film f, const WaveBuffers &w, uint32_t *err,
                   int grid, int block, cudaStream_t st, int paths, int ext_sorted = 0,
-                  int shadow_sorted = 0, WaveLoop *L = nullptr) {
+                  int shadow_sorted = 0, WaveLoop *L = nullptr, bool refills = false) {
   const auto go = s.node_width == 9   ? launch_trace_w<9, kLoop>
                   : s.node_width == 5 ? launch_trace_w<5, kLoop>
                   : s.node_width == 8 ? launch_trace_w<8, kLoop>
                   : s.node_width == 4 ? launch_trace_w<4, kLoop>
                                       : launch_trace_w<2, kLoop>;
-  go(s, c, depth, f, w, err, grid, block, st, ext_sorted, shadow_sorted, L, paths);
+  go(s, c, depth, f, w, err, grid, block, st, ext_sorted, shadow_sorted, L, paths, refills);
 }
 
 // ---- queue sorting ------------------------------------------------------
@@ -953,7 +960,7 @@ void free_wave_loop(WaveLoopGraph *g) {
 namespace {
 
 cudaError_t build_wave_loop(WaveLoopGraph::Loop &G, cudaStream_t &capture, const DevScene &s, const DevConfig &c, Film f,
-                            const WaveBuffers &w, uint32_t *err, int grid, int block, int paths) {
+                            const WaveBuffers &w, uint32_t *err, int grid, int block, int paths, bool refills) {
   if (G.exec) cudaGraphExecDestroy(G.exec);
   if (G.graph) cudaGraphDestroy(G.graph);
   G.exec = nullptr;
@@ -974,7 +981,7 @@ cudaError_t build_wave_loop(WaveLoopGraph::Loop &G, cudaStream_t &capture, const
   if ((e = cudaStreamBeginCaptureToGraph(capture, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
       cudaSuccess)
     return e;
-  launch_trace<true>(s, c, 0, f, w, err, grid, block, capture, paths, 0, 0, w.loop);
+  launch_trace<true>(s, c, 0, f, w, err, grid, block, capture, paths, 0, 0, w.loop, refills);
   k_shade_loop<<<resident_grid(grid, block, kStageThreads), block, 0, capture>>>(s, c, f, w, w.loop, err);
   k_loop_control<<<1, 32, 0, capture>>>(w.loop, h, 1, err);
   const cudaError_t le = cudaGetLastError();
@@ -1029,7 +1036,7 @@ cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pas
     const int init_grid = (int)((n0 + 255) / 256 < 4096 ? (n0 + 255) / 256 : 4096);
     k_loop_init<<<init_grid, 256, 0, st>>>(s, c, w, w.loop, pass0, band0, npass, n0, limit, shared);
     for (int it = 0; it < limit; ++it) {
-      launch_trace<true>(s, c, 0, f, w, err, grid, block, st, n0, 0, 0, w.loop);
+      launch_trace<true>(s, c, 0, f, w, err, grid, block, st, n0, 0, 0, w.loop, total > n0);
       k_shade_loop<<<resident_grid(grid, block, kStageThreads), block, 0, st>>>(s, c, f, w, w.loop, err);
       k_loop_control<<<1, 32, 0, st>>>(w.loop, 0, 0, err);
       int go = 0;
@@ -1041,10 +1048,10 @@ cudaError_t launch_wave_loop(const DevScene &s, const DevConfig &c, uint32_t pas
     return cudaGetLastError();
   }
   if (!*graph) *graph = new WaveLoopGraph;
-  WaveLoopGraph::Loop &G = (*graph)->loop[(int)trace_way<true>(s, n0)];
+  WaveLoopGraph::Loop &G = (*graph)->loop[(int)trace_way(s, n0, total > n0)];
   if (!G.exec || G.key.size() != sizeof k || memcmp(G.key.data(), kb, sizeof k) != 0) {
     G.key.clear();
-    const cudaError_t e = build_wave_loop(G, (*graph)->capture, s, c, f, w, err, grid, block, n0);
+    const cudaError_t e = build_wave_loop(G, (*graph)->capture, s, c, f, w, err, grid, block, n0, total > n0);
     if (e != cudaSuccess) return e;
     G.key.assign(kb, kb + sizeof k);
   }
@@ -1220,9 +1227,11 @@ void free_batch_loop(BatchLoopGraph *g) {
 
 namespace {
 
+// the lines of trace_way() between lanes at their own pace and together, without its groups
 template <int W>
-void launch_trace_bloop_w(const BatchSlot *slots, const WaveBuffers &w, uint32_t *err, int grid, int block, cudaStream_t st) {
-  if (w.capacity <= kPacedSlots)
+void launch_trace_bloop_w(const BatchSlot *slots, const WaveBuffers &w, uint32_t *err, int grid, int block, cudaStream_t st,
+                          bool refills) {
+  if (w.capacity <= (refills ? kPacedSlots : kPacedPaths))
     k_trace_bloop<W, false><<<resident_grid(grid, block, kStageThreads), block, 0, st>>>(slots, w, err, w.loop);
   else
     k_trace_bloop<W, true><<<grid, block, 0, st>>>(slots, w, err, w.loop);
@@ -1230,19 +1239,19 @@ void launch_trace_bloop_w(const BatchSlot *slots, const WaveBuffers &w, uint32_t
 }
 
 cudaError_t launch_trace_bloop(const BatchSlot *slots, const WaveBuffers &w, uint32_t *err, int width, int grid,
-                               int block, cudaStream_t st) {
+                               int block, cudaStream_t st, bool refills) {
   const auto go = width == 9   ? launch_trace_bloop_w<9>
                   : width == 5 ? launch_trace_bloop_w<5>
                   : width == 8 ? launch_trace_bloop_w<8>
                   : width == 4 ? launch_trace_bloop_w<4>
                                : launch_trace_bloop_w<2>;
-  go(slots, w, err, grid, block, st);
+  go(slots, w, err, grid, block, st, refills);
   return cudaGetLastError();
 }
 
 // the loop body: one iteration (trace, shade, control)
-cudaError_t bloop_body(BatchSlot *slots, int n, const WaveBuffers &w, uint32_t *err, int width, int grid, int block, cudaGraphConditionalHandle h, int in_graph, cudaStream_t st) {
-  cudaError_t e = launch_trace_bloop(slots, w, err, width, grid, block, st);
+cudaError_t bloop_body(BatchSlot *slots, int n, const WaveBuffers &w, uint32_t *err, int width, int grid, int block, cudaGraphConditionalHandle h, int in_graph, cudaStream_t st, bool refills) {
+  cudaError_t e = launch_trace_bloop(slots, w, err, width, grid, block, st, refills);
   if (e != cudaSuccess) return e;
   k_shade_bloop<<<resident_grid(grid, block, kStageThreads), block, 0, st>>>(slots, n, w, w.loop, err);
   k_loop_control<<<1, 32, 0, st>>>(w.loop, h, in_graph, err);
@@ -1261,7 +1270,7 @@ cudaError_t bloop_head(BatchSlot *slots, int n, BatchHeader *h, const int *activ
 // the whole step as one graph: head -> while(loop body) -> finish
 cudaError_t build_bloop_graph(BatchLoopGraph &G, BatchSlot *slots, int n, BatchHeader *h, const int *active,
                               uint32_t *err, const WaveBuffers &w, int width, int grid, int block,
-                              int capacity, int limit, int acc_blocks) {
+                              int capacity, int limit, int acc_blocks, bool refills) {
   cudaError_t e;
   if (!G.capture && (e = cudaStreamCreateWithFlags(&G.capture, cudaStreamNonBlocking)) != cudaSuccess) return e;
   if ((e = cudaGraphCreate(&G.graph, 0)) != cudaSuccess) return e;
@@ -1293,7 +1302,7 @@ cudaError_t build_bloop_graph(BatchLoopGraph &G, BatchSlot *slots, int n, BatchH
   if ((e = cudaStreamBeginCaptureToGraph(G.capture, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                          cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
     return e;
-  le = bloop_body(slots, n, w, err, width, grid, block, cond, 1, G.capture);
+  le = bloop_body(slots, n, w, err, width, grid, block, cond, 1, G.capture, refills);
   cudaGraph_t body = nullptr;
   e = cudaStreamEndCapture(G.capture, &body);
   if (le != cudaSuccess) return le;
@@ -1314,7 +1323,7 @@ cudaError_t build_bloop_graph(BatchLoopGraph &G, BatchSlot *slots, int n, BatchH
 cudaError_t launch_batch_loop_step(BatchSlot *slots, int n, BatchHeader *h, const int *active, uint32_t *err,
                                    const WaveBuffers &w, int width, int grid, int block, int capacity,
                                    int limit, int acc_blocks, cudaStream_t st, BatchLoopGraph **graph,
-                                   bool use_graph) {
+                                   bool use_graph, bool refills) {
   if (capacity < 1 || capacity > w.capacity || !w.view || !w.sq_view || !w.tag || !w.loop || limit < 1)
     return cudaErrorInvalidValue;
   if (!use_graph) {
@@ -1327,7 +1336,7 @@ cudaError_t launch_batch_loop_step(BatchSlot *slots, int n, BatchHeader *h, cons
       if (e == cudaSuccess) e = cudaStreamSynchronize(st);
       if (e != cudaSuccess) return e;
       if (!go) break;
-      e = bloop_body(slots, n, w, err, width, grid, block, 0, 0, st);
+      e = bloop_body(slots, n, w, err, width, grid, block, 0, 0, st, refills);
       if (e != cudaSuccess) return e;
     }
     return launch_batch_finish(slots, n, acc_blocks, st);
@@ -1336,7 +1345,7 @@ cudaError_t launch_batch_loop_step(BatchSlot *slots, int n, BatchHeader *h, cons
   BatchLoopGraph &G = **graph;
   if (!G.exec) {
     const cudaError_t e =
-        build_bloop_graph(G, slots, n, h, active, err, w, width, grid, block, capacity, limit, acc_blocks);
+        build_bloop_graph(G, slots, n, h, active, err, w, width, grid, block, capacity, limit, acc_blocks, refills);
     if (e != cudaSuccess) {
       if (G.graph) cudaGraphDestroy(G.graph);
       G.graph = nullptr;

@@ -19,10 +19,13 @@ def renderer(scene, cfg, ex, width, quantize=False, **settings):
                        bvh_params={"width": width, "quantize": quantize})
 
 
-def film(r, passes):
+def film(r, passes, bundle=False):
     r.clear_pixel_space()
-    for p in range(passes):
-        r.cast_rays(p, pass_idx=p)
+    if bundle:  # of more passes than path slots: they are filled again
+        r.cast_rays_bundle(0, passes, pass_idx=0)
+    else:
+        for p in range(passes):
+            r.cast_rays(p, pass_idx=p)
     assert r.check_device() == 0
     return r.block_film.clone()
 
@@ -34,9 +37,9 @@ def doubled(scene):
 
 
 # FP64 film sums in another order: equal to a few last bits.  Paths on either side of what selects the way: 56,832 and
-# 227,328 slots of the loop, 113,664 and 606,208 pixels of a pass
+# 227,328 slots that are filled again, 113,664 and 378,880 paths of a pass
 @pytest.mark.parametrize("width,height", [(1, 1), (33, 3), (296, 192), (297, 192), (592, 192), (593, 192), (592, 384),
-                                          (592, 385), (1024, 592), (1024, 593)])
+                                          (592, 385), (640, 592), (640, 593)])
 @pytest.mark.parametrize("node_width,quantize", LAYOUTS)
 def test_stages_and_loop_give_the_megakernel_film(width, height, node_width, quantize):
     s, c, ex = configs.volume_scene(width=width, height=height, depth=6, medium_slices=20, medium_stacks=21)
@@ -48,24 +51,27 @@ def test_stages_and_loop_give_the_megakernel_film(width, height, node_width, qua
             assert torch.allclose(a, film(r, 2), rtol=1e-12, atol=0), settings
             if "queue_capacity" in settings:
                 assert r.wave_loop_iterations() > 0
+                assert torch.allclose(a, film(r, 2, bundle=True), rtol=1e-12, atol=0), settings
 
 
-# a tree of more than 32,768 triangles: 1,060,864 slots of the loop, and passes of any size here at their own pace
-@pytest.mark.parametrize("width,height", [(592, 385), (1024, 1036), (1024, 1037)])
+# a tree of more than 32,768 triangles: 1,060,864 slots that are filled again; passes at their own pace, above 227,328
+# pixels with two children
+@pytest.mark.parametrize("width,height", [(592, 384), (592, 385), (1024, 1036), (1024, 1037)])
 @pytest.mark.parametrize("node_width,quantize", LAYOUTS[:2] + LAYOUTS[4:])
 def test_large_tree(width, height, node_width, quantize):
     s, c, ex = configs.terrain_scene(width=width, height=height, depth=3, grid=140, sphere_slices=20, sphere_stacks=21)
     with renderer(s, c, ex, node_width, quantize, kernel="mega") as r:
         assert r.scene_info()["num_tris"] > 32768
-        a = film(r, 1)
+        a = film(r, 2)
         assert float(a.sum()) > 0
         for settings in ({"sort_keys": 1}, {"queue_capacity": width * height}):
             r.set_launch_config(**{"kernel": "wavefront", "sort_keys": 0, "queue_capacity": 0, **settings})
-            assert torch.allclose(a, film(r, 1), rtol=1e-12, atol=0), settings
+            bundle = "queue_capacity" in settings
+            assert torch.allclose(a, film(r, 2, bundle), rtol=1e-12, atol=0), settings
 
 
-# 1,600 paths: groups, which decide their ties at once; 240,000: in the loop together, in a pass at their own pace, whose
-# ties go to lists; 60,000: own pace in the loop
+# 1,600 paths: groups, which decide their ties at once; 60,000 and 240,000: slots that are filled again at their own pace
+# and together, a pass in groups and at its own pace, whose ties go to lists
 @pytest.mark.parametrize("width,height", [(40, 40), (300, 200), (600, 400)])
 @pytest.mark.parametrize("node_width", [2, 4, 8])
 def test_ties_in_stages_and_loop(width, height, node_width):
@@ -76,20 +82,24 @@ def test_ties_in_stages_and_loop(width, height, node_width):
         for settings in ({"sort_keys": 1}, {"sort_keys": 7}, {}, {"queue_capacity": width * height}):
             r.set_launch_config(**{"kernel": "wavefront", "sort_keys": 0, "queue_capacity": 0, **settings})
             assert torch.allclose(a, film(r, 2), rtol=1e-12, atol=0), settings
+            if "queue_capacity" in settings:
+                assert torch.allclose(a, film(r, 2, bundle=True), rtol=1e-12, atol=0), settings
 
 
-# 62,000 slots: own pace; 240,250: together
-@pytest.mark.parametrize("width", [40, 155])
+# all paths of a step in their slots, 62,000 and 372,000 (own pace), 620,000 (together); 230,000 slots filled again
+# (together)
+@pytest.mark.parametrize("width,slots", [(40, 0), (240, 0), (400, 0), (310, 230000)])
 @pytest.mark.parametrize("use_graph", [True, False])
 @pytest.mark.parametrize("node_width", [2, 4, 8])
-def test_ties_in_a_wavefront_batch(node_width, use_graph, width):
+def test_ties_in_a_wavefront_batch(node_width, use_graph, width, slots):
     rs = []
     for k in range(2):
         s, c, ex = configs.box_scene(seed=k, width=width, height=31, depth=5, sphere_slices=12, sphere_stacks=13)
         rs.append(renderer(doubled(s), c, ex, node_width, kernel="mega"))
     films = []
     for kernel in ("mega", "wavefront"):
-        with sbatch.Batch(rs, kernel=kernel, use_graph=use_graph) as b:
+        with sbatch.Batch(rs, kernel=kernel, use_graph=use_graph,
+                          queue_capacity=slots if kernel == "wavefront" else 0) as b:
             b.reset(0)
             b.step()
             assert b.check() == 0
